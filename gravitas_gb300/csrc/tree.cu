@@ -1345,47 +1345,96 @@ __global__ __launch_bounds__(kThreads) void k_kick_drift(int64_t n, double h, do
 
 constexpr int kDirThreads = 128;
 
-__global__ __launch_bounds__(kDirThreads) void k_direct_fp64(int64_t n, const double *__restrict__ px,
-                                                             const double *__restrict__ py, const double *__restrict__ pz,
-                                                             const double *__restrict__ mass,
-                                                             const uint8_t *__restrict__ kind, double eps2, int dm_off,
-                                                             const int64_t *__restrict__ targets, int64_t ntargets,
-                                                             double *ax, double *ay, double *az) {
-    __shared__ double s_x[kDirThreads], s_y[kDirThreads], s_z[kDirThreads], s_m[kDirThreads];
-    __shared__ uint8_t s_skip[kDirThreads];
-    int64_t q = int64_t(blockIdx.x) * kDirThreads + threadIdx.x;
-    bool valid = q < ntargets;
-    int64_t i = valid ? (targets ? targets[q] : q) : 0;
-    double xi = px[i], yi = py[i], zi = pz[i];
-    double fax = 0, fay = 0, faz = 0;
-    for (int64_t j0 = 0; j0 < n; j0 += kDirThreads) {
-        int64_t j = j0 + threadIdx.x;
-        if (j < n) {
-            uint8_t kd = kind ? kind[j] : 0;
-            s_x[threadIdx.x] = px[j];
-            s_y[threadIdx.x] = py[j];
-            s_z[threadIdx.x] = pz[j];
-            s_m[threadIdx.x] = mass[j];
-            s_skip[threadIdx.x] = kd == GBH_BLACK_HOLE || (dm_off && kd == GBH_DARK_MATTER);
-        }
-        __syncthreads();
-        int64_t cnt = n - j0 < kDirThreads ? n - j0 : kDirThreads;
-        for (int t = 0; t < cnt; ++t) {
-            if (j0 + t == i || s_skip[t]) continue;
-            double dx = s_x[t] - xi, dy = s_y[t] - yi, dz = s_z[t] - zi;
-            double re2 = dx * dx + dy * dy + dz * dz + eps2;
-            double f = s_m[t] / (re2 * sqrt(re2));
-            fax += f * dx;
-            fay += f * dy;
-            faz += f * dz;
+// A sum of FP64 pair terms in the reference's order (ascending j) is a serial chain of adds, but
+// the terms themselves are independent. A block takes T targets: its compute warps form the terms
+// of T targets x J sources in shared memory (a thread keeps its source in registers and takes the
+// targets in turn) while the add warps, one lane per target and axis, add the previous tile's
+// terms in order, so every sum keeps its bits. One barrier a tile (two buffers). Skipped pairs
+// leave a term of +0: the sums start at +0 and never become -0, so adding it changes nothing.
+//
+// The kernel is bound by the FP64 pipe (about 33 operations a pair, most of them the division and
+// the square root), which needs every SM busy; one thread a target filled 32 of 152 SMs with
+// 4,096 targets. T is chosen so that the blocks fill whole waves of two a SM: J = 64 sources a
+// tile with up to 32 targets, or J = 256 with up to 8 (few targets: all compute threads still have
+// a source). 4,096 targets of 131,072 bodies: 159 ms with a thread a target, 35.1 ms so (5.0e11 FP64
+// operations/s of the 6.3e11 the pipe issues).
+constexpr int kDirCompute = 256;  // compute threads; the add warps follow them
+template <int kJ>
+struct DirTile {
+    static constexpr int kT = 2048 / kJ;                           // most targets of a block
+    static constexpr int kStride = kJ + 1;                         // padded row: the add lanes hit all banks
+    static constexpr int kRows = 3 * kT;
+    static constexpr int kAdd = (kRows + 31) / 32 * 32;            // add threads
+    static constexpr size_t kBytes = sizeof(double) * 2 * kRows * kStride;
+};
+
+template <int kJ>
+__global__ __launch_bounds__(kDirCompute + DirTile<kJ>::kAdd) void k_direct_fp64(
+    int64_t n, const double *__restrict__ px, const double *__restrict__ py, const double *__restrict__ pz,
+    const double *__restrict__ mass, const uint8_t *__restrict__ kind, double eps2, int dm_off,
+    const int64_t *__restrict__ targets, int64_t ntargets, int T, double *ax, double *ay, double *az) {
+    using Tile = DirTile<kJ>;
+    extern __shared__ double s_term[];  // [2][target][axis][kStride]
+    __shared__ double s_x[Tile::kT], s_y[Tile::kT], s_z[Tile::kT];
+    __shared__ int64_t s_i[Tile::kT];
+    const int tid = threadIdx.x;
+    const int64_t q0 = int64_t(blockIdx.x) * T;
+    const int nt = ntargets - q0 < T ? int(ntargets - q0) : T;
+    if (tid < nt) {
+        const int64_t i = targets ? targets[q0 + tid] : q0 + tid;
+        s_i[tid] = i;
+        s_x[tid] = px[i];
+        s_y[tid] = py[i];
+        s_z[tid] = pz[i];
+    }
+    __syncthreads();
+    const int64_t ntiles = (n + kJ - 1) / kJ;
+    const bool adder = tid >= kDirCompute;
+    const int a = tid - kDirCompute;  // add lane: target a / 3, axis a % 3
+    const int jj = tid % kJ, g = tid / kJ;
+    double x = 0, y = 0, z = 0, m = 0, sum = 0;
+    bool skip = true;
+    auto load = [&](int64_t tile) {
+        const int64_t j = tile * kJ + jj;
+        skip = j >= n;
+        if (skip) return;
+        const uint8_t kd = kind ? kind[j] : 0;
+        skip = kd == GBH_BLACK_HOLE || (dm_off && kd == GBH_DARK_MATTER);
+        x = px[j];
+        y = py[j];
+        z = pz[j];
+        m = mass[j];
+    };
+    if (!adder) load(0);
+    // tile t is formed while tile t - 1 is added
+    for (int64_t t = 0; t <= ntiles; ++t) {
+        if (!adder && t < ntiles) {
+            const double xj = x, yj = y, zj = z, mj = m;
+            const bool sk = skip;
+            const int64_t j = t * kJ + jj;
+            if (t + 1 < ntiles) load(t + 1);  // in flight during this tile's arithmetic
+            double *row = s_term + size_t(t & 1) * Tile::kRows * Tile::kStride + jj;
+            for (int k = g; k < nt; k += kDirCompute / kJ) {
+                const double dx = xj - s_x[k], dy = yj - s_y[k], dz = zj - s_z[k];
+                const double re2 = dx * dx + dy * dy + dz * dz + eps2;
+                const double f = mj / (re2 * sqrt(re2));
+                const bool off = sk || j == s_i[k];
+                row[(3 * k) * Tile::kStride] = off ? 0.0 : f * dx;
+                row[(3 * k + 1) * Tile::kStride] = off ? 0.0 : f * dy;
+                row[(3 * k + 2) * Tile::kStride] = off ? 0.0 : f * dz;
+            }
+        } else if (adder && t > 0 && a < 3 * nt) {
+            const double *row = s_term + (size_t((t - 1) & 1) * Tile::kRows + a) * Tile::kStride;
+#pragma unroll 16
+            for (int k = 0; k < kJ; ++k) sum += row[k];
         }
         __syncthreads();
     }
-    if (!valid) return;
-    bool hole = kind && kind[i] == GBH_BLACK_HOLE;
-    ax[q] = hole ? 0 : fax;
-    ay[q] = hole ? 0 : fay;
-    az[q] = hole ? 0 : faz;
+    if (!adder || a >= 3 * nt) return;
+    const int64_t i = s_i[a / 3];
+    if (kind && kind[i] == GBH_BLACK_HOLE) sum = 0;
+    double *out = a % 3 == 0 ? ax : a % 3 == 1 ? ay : az;
+    out[q0 + a / 3] = sum;
 }
 
 // ---------------------------------------------------------------- potential (potential.go:16-81)
@@ -2129,14 +2178,31 @@ cudaError_t kick_drift(const Launch &L, int64_t n, double h, double dt, double c
     return cudaSuccess;
 }
 
+template <int kJ>
+static cudaError_t launch_direct(const Launch &L, int64_t n, const double *px, const double *py, const double *pz,
+                                 const double *mass, const uint8_t *kind, double eps2, int dm_off,
+                                 const int64_t *targets, int64_t ntargets, int T, double *ax, double *ay, double *az) {
+    using Tile = DirTile<kJ>;
+    // set on every call: the attribute belongs to the current device
+    cudaError_t e = cudaFuncSetAttribute(k_direct_fp64<kJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Tile::kBytes));
+    if (e != cudaSuccess) return e;
+    k_direct_fp64<kJ><<<blocks_for(ntargets, T), kDirCompute + Tile::kAdd, Tile::kBytes, L.stream>>>(
+        n, px, py, pz, mass, kind, eps2, dm_off, targets, ntargets, T, ax, ay, az);
+    GBH_LAUNCH_CHECK();
+    return cudaSuccess;
+}
+
 cudaError_t direct_fp64(const Launch &L, int64_t n, const double *px, const double *py, const double *pz,
                         const double *mass, const uint8_t *kind, double eps2, int dm_off, const int64_t *targets,
                         int64_t ntargets, double *ax, double *ay, double *az) {
     if (ntargets == 0 || n == 0) return cudaSuccess;
-    k_direct_fp64<<<blocks_for(ntargets, kDirThreads), kDirThreads, 0, L.stream>>>(n, px, py, pz, mass, kind, eps2,
-                                                                                  dm_off, targets, ntargets, ax, ay, az);
-    GBH_LAUNCH_CHECK();
-    return cudaSuccess;
+    // two blocks a SM are resident: as few targets a block as fill whole waves of them
+    const int64_t wave = 2 * int64_t(L.num_sms > 0 ? L.num_sms : 152);
+    const int64_t waves = (ntargets + wave * DirTile<64>::kT - 1) / (wave * DirTile<64>::kT);
+    const int T = int((ntargets + waves * wave - 1) / (waves * wave));
+    if (T <= DirTile<256>::kT)
+        return launch_direct<256>(L, n, px, py, pz, mass, kind, eps2, dm_off, targets, ntargets, T, ax, ay, az);
+    return launch_direct<64>(L, n, px, py, pz, mass, kind, eps2, dm_off, targets, ntargets, T, ax, ay, az);
 }
 
 // Potential from the mixed walk's psi (sorted order): the block sums of m_k psi_k minus each

@@ -1,0 +1,38 @@
+"""FP64 pair sums whose terms are formed in parallel and added in order: bit identical to the
+oracle's serial loops at the edges of their tiles."""
+import numpy as np
+import pytest
+
+from gravitas_gb300 import abi, ics
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+P = abi.ptr
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = abi.Context(0)
+    yield c
+    c.close()
+
+
+def disk(n, seed=3):
+    """n bodies: the test disk with its two holes, some dark matter, two bodies at one place."""
+    s = ics.test_disk(max(n, 3) - 2, seed=seed)
+    s["kind"][1:n - 1:7] = O.DARK_MATTER
+    s["px"][n // 2], s["py"][n // 2], s["pz"][n // 2] = s["px"][1], s["py"][1], s["pz"][1]
+    return {k: np.ascontiguousarray(v[:n]) for k, v in s.items()}
+
+
+@pytest.mark.parametrize("n,ntargets", [(1, 1), (2, 2), (63, 5), (64, 64), (65, 1), (255, 9), (257, 33), (3001, 304),
+                                        (3001, 2433), (5000, 5000)])
+def test_direct_sum_bit_identical(ctx, n, ntargets):
+    s = disk(n)
+    tg = np.sort(np.random.default_rng(n).choice(n, ntargets, replace=False)).astype(np.int64)
+    for dm_off in (False, True):
+        got = np.full((3, ntargets), 7.0)
+        ctx.call("gbh_direct_accelerations", abi.make_params(0, 0.03, 0, False, dm_off, "fp64"), n, P(s["px"]),
+                 P(s["py"]), P(s["pz"]), P(s["mass"]), P(s["kind"]), P(tg), ntargets, *[P(g) for g in got])
+        want = O.direct(s["px"], s["py"], s["pz"], s["mass"], s["kind"], eps=0.03, dm_off=dm_off, targets=tg)
+        assert np.array_equal(got.T, want)
