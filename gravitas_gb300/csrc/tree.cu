@@ -1343,8 +1343,6 @@ __global__ __launch_bounds__(kThreads) void k_kick_drift(int64_t n, double h, do
 
 // ---------------------------------------------------------------- direct sum (direct.go:18-48)
 
-constexpr int kDirThreads = 128;
-
 // A sum of FP64 pair terms in the reference's order (ascending j) is a serial chain of adds, but
 // the terms themselves are independent. A block takes T targets: its compute warps form the terms
 // of T targets x J sources in shared memory (a thread keeps its source in registers and takes the
@@ -1458,50 +1456,93 @@ __device__ __forceinline__ double pair_potential(double mi, double mj, double r2
 // pair model's potential in ascending j, kinds and liveness as the reference reads them (all
 // bodies). The rows are then added in ascending i (the reference adds its ParallelFor chunks
 // in completion order, so only round-off may differ).
-__global__ __launch_bounds__(kDirThreads) void k_pot_exact_rows(int64_t n, const double *__restrict__ px,
-                                                                const double *__restrict__ py,
-                                                                const double *__restrict__ pz,
-                                                                const double *__restrict__ mass,
-                                                                const uint8_t *__restrict__ kind, double eps2, double c,
-                                                                int dm_off, double *rows) {
-    __shared__ double s_x[kDirThreads], s_y[kDirThreads], s_z[kDirThreads], s_m[kDirThreads];
-    __shared__ uint8_t s_k[kDirThreads];
-    const int64_t i0 = int64_t(blockIdx.x) * kDirThreads;
-    const int64_t i = i0 + threadIdx.x;
-    const bool act = i < n;
-    const uint8_t ki = act && kind ? kind[i] : 0;
-    const double xi = act ? px[i] : 0, yi = act ? py[i] : 0, zi = act ? pz[i] : 0, mi = act ? mass[i] : 0;
-    const double smi = dm_off && ki == GBH_DARK_MATTER ? 0.0 : mi;
-    double part = 0;
-    for (int64_t j0 = i0 + 1; j0 < n; j0 += kDirThreads) {
-        int64_t j = j0 + threadIdx.x;
-        if (j < n) {
-            s_x[threadIdx.x] = px[j];
-            s_y[threadIdx.x] = py[j];
-            s_z[threadIdx.x] = pz[j];
-            s_m[threadIdx.x] = mass[j];
-            s_k[threadIdx.x] = kind ? kind[j] : 0;
-        }
-        __syncthreads();
-        int cnt = n - j0 < kDirThreads ? int(n - j0) : kDirThreads;
-        for (int t = 0; t < cnt; ++t) {
-            if (j0 + t <= i) continue;
-            double dx = s_x[t] - xi, dy = s_y[t] - yi, dz = s_z[t] - zi;
-            uint8_t kj = s_k[t];
-            double rs = pair_rs(ki, mi, kj, s_m[t], c);
-            double smj = dm_off && kj == GBH_DARK_MATTER ? 0.0 : s_m[t];
-            part += pair_potential(smi, smj, dx * dx + dy * dy + dz * dz, eps2, rs);
+//
+// As in k_direct_fp64, the compute threads form a tile's terms and one add lane a row adds them in
+// order. Bound by the FP64 pipe (about 28 operations a pair). A block takes T rows, few enough
+// that the blocks fill every SM several times over (the rows shorten, so the longest blocks are
+// launched first and the short ones fill the end). 30,000 bodies: 44.8 ms with one thread a row
+// and one thread adding the rows from global memory, 28.3 ms so.
+constexpr int kPotRows = 32, kPotJ = 64;
+constexpr int kPotStride = kPotJ + 1;
+__global__ __launch_bounds__(kDirCompute + 32) void k_pot_exact_rows(int64_t n, const double *__restrict__ px,
+                                                                     const double *__restrict__ py,
+                                                                     const double *__restrict__ pz,
+                                                                     const double *__restrict__ mass,
+                                                                     const uint8_t *__restrict__ kind, double eps2,
+                                                                     double c, int dm_off, int T, double *rows) {
+    __shared__ double s_term[2][kPotRows][kPotStride];
+    __shared__ double s_x[kPotRows], s_y[kPotRows], s_z[kPotRows], s_m[kPotRows];
+    __shared__ uint8_t s_k[kPotRows];
+    const int tid = threadIdx.x;
+    const int64_t i0 = int64_t(blockIdx.x) * T;
+    const int nt = n - i0 < T ? int(n - i0) : T;
+    if (tid < nt) {
+        s_x[tid] = px[i0 + tid];
+        s_y[tid] = py[i0 + tid];
+        s_z[tid] = pz[i0 + tid];
+        s_m[tid] = mass[i0 + tid];
+        s_k[tid] = kind ? kind[i0 + tid] : 0;
+    }
+    __syncthreads();
+    const int64_t ntiles = (n - i0 + kPotJ - 1) / kPotJ;
+    const bool adder = tid >= kDirCompute;
+    const int a = tid - kDirCompute;
+    const int jj = tid % kPotJ, g = tid / kPotJ;
+    double x = 0, y = 0, z = 0, m = 0, sum = 0;
+    uint8_t kd = 0;
+    auto load = [&](int64_t tile) {
+        const int64_t j = i0 + tile * kPotJ + jj;
+        if (j >= n) return;
+        kd = kind ? kind[j] : 0;
+        x = px[j];
+        y = py[j];
+        z = pz[j];
+        m = mass[j];
+    };
+    if (!adder) load(0);
+    for (int64_t t = 0; t <= ntiles; ++t) {
+        if (!adder && t < ntiles) {
+            const double xj = x, yj = y, zj = z, mj = m;
+            const uint8_t kj = kd;
+            const int64_t j = i0 + t * kPotJ + jj;
+            if (t + 1 < ntiles) load(t + 1);
+            const double smj = dm_off && kj == GBH_DARK_MATTER ? 0.0 : mj;
+            for (int k = g; k < nt; k += kDirCompute / kPotJ) {
+                const double dx = xj - s_x[k], dy = yj - s_y[k], dz = zj - s_z[k];
+                const uint8_t ki = s_k[k];
+                const double mi = s_m[k];
+                const double rs = pair_rs(ki, mi, kj, mj, c);
+                const double smi = dm_off && ki == GBH_DARK_MATTER ? 0.0 : mi;
+                const double v = pair_potential(smi, smj, dx * dx + dy * dy + dz * dz, eps2, rs);
+                s_term[t & 1][k][jj] = j < n && j > i0 + k ? v : 0.0;
+            }
+        } else if (adder && t > 0 && a < nt) {
+            const double *row = s_term[(t - 1) & 1][a];
+#pragma unroll 16
+            for (int k = 0; k < kPotJ; ++k) sum += row[k];
         }
         __syncthreads();
     }
-    if (act) rows[i] = part;
+    if (adder && a < nt) rows[i0 + a] = sum;
 }
 
-__global__ void k_pot_exact_final(int64_t n, const double *__restrict__ rows, double *out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// The rows added in ascending i by one thread, from tiles that the block stages in shared memory.
+constexpr int kPotFinal = 2048;
+__global__ __launch_bounds__(kThreads) void k_pot_exact_final(int64_t n, const double *__restrict__ rows, double *out) {
+    __shared__ double s[2][kPotFinal];
     double sum = 0;
-    for (int64_t i = 0; i < n; ++i) sum += rows[i];
-    *out = sum;
+    const int64_t ntiles = (n + kPotFinal - 1) / kPotFinal;
+    for (int64_t t = 0; t <= ntiles; ++t) {
+        if (t < ntiles && threadIdx.x >= 32)
+            for (int k = threadIdx.x - 32; k < kPotFinal; k += kThreads - 32)
+                s[t & 1][k] = t * kPotFinal + k < n ? rows[t * kPotFinal + k] : 0.0;  // + 0: no change
+        if (t > 0 && threadIdx.x == 0) {
+#pragma unroll 16
+            for (int k = 0; k < kPotFinal; ++k) sum += s[(t - 1) & 1][k];
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *out = sum;
 }
 
 // holePotential, potential.go:84-96.
@@ -2264,10 +2305,13 @@ __global__ void k_potential_final_state(int64_t nparts, const double *part, int6
 cudaError_t potential_exact_fp64(const Launch &L, int64_t n, const double *px, const double *py, const double *pz,
                                  const double *mass, const uint8_t *kind, double eps2, double c, int dm_off,
                                  double *rows, double *u_dev) {
-    k_pot_exact_rows<<<blocks_for(n, kDirThreads), kDirThreads, 0, L.stream>>>(n, px, py, pz, mass, kind, eps2, c,
-                                                                               dm_off, rows);
+    // about four blocks a SM or more
+    const int64_t per = n / (4 * int64_t(L.num_sms > 0 ? L.num_sms : 152));
+    const int T = int(per < 1 ? 1 : per > kPotRows ? kPotRows : per);
+    k_pot_exact_rows<<<blocks_for(n, T), kDirCompute + 32, 0, L.stream>>>(n, px, py, pz, mass, kind, eps2, c, dm_off, T,
+                                                                          rows);
     GBH_LAUNCH_CHECK();
-    k_pot_exact_final<<<1, 32, 0, L.stream>>>(n, rows, u_dev);
+    k_pot_exact_final<<<1, kThreads, 0, L.stream>>>(n, rows, u_dev);
     GBH_LAUNCH_CHECK();
     return cudaSuccess;
 }
@@ -2457,11 +2501,23 @@ __global__ __launch_bounds__(kThreads) void k_diag_partial(int64_t n, const doub
     }
 }
 
-__global__ void k_diag_final(int nparts, const double *__restrict__ part, double *out) {
-    if (threadIdx.x >= kDiagSums) return;
+// Each sum's block parts in block order: staged in shared memory by the whole block, added by one
+// lane a sum (1,024 parts: 11 threads reading them from global memory took 40 us).
+__global__ __launch_bounds__(kThreads) void k_diag_final(int nparts, const double *__restrict__ part, double *out) {
+    constexpr int kTile = 128;  // parts a tile
+    __shared__ double s[kTile * kDiagSums];
     double v = 0;
-    for (int b = 0; b < nparts; ++b) v += part[b * kDiagSums + threadIdx.x];
-    out[threadIdx.x] = v;
+    for (int b0 = 0; b0 < nparts; b0 += kTile) {
+        const int cnt = nparts - b0 < kTile ? nparts - b0 : kTile;
+        for (int k = threadIdx.x; k < cnt * kDiagSums; k += kThreads) s[k] = part[b0 * kDiagSums + k];
+        __syncthreads();
+        if (threadIdx.x < kDiagSums) {
+#pragma unroll 8
+            for (int b = 0; b < cnt; ++b) v += s[b * kDiagSums + threadIdx.x];
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x < kDiagSums) out[threadIdx.x] = v;
 }
 
 }  // namespace
@@ -2475,7 +2531,7 @@ cudaError_t diagnostics(const Launch &L, int64_t n, const double *px, const doub
     if (nb > unsigned(kFlagBlocksMax)) nb = kFlagBlocksMax;
     k_diag_partial<<<nb, kThreads, 0, L.stream>>>(n, px, py, pz, vx, vy, vz, mass, kind, c, dm_off, part);
     GBH_LAUNCH_CHECK();
-    k_diag_final<<<1, 32, 0, L.stream>>>(int(nb), part, out);
+    k_diag_final<<<1, kThreads, 0, L.stream>>>(int(nb), part, out);
     GBH_LAUNCH_CHECK();
     return cudaSuccess;
 }

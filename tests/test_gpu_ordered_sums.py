@@ -36,3 +36,18 @@ def test_direct_sum_bit_identical(ctx, n, ntargets):
                  P(s["py"]), P(s["pz"]), P(s["mass"]), P(s["kind"]), P(tg), ntargets, *[P(g) for g in got])
         want = O.direct(s["px"], s["py"], s["pz"], s["mass"], s["kind"], eps=0.03, dm_off=dm_off, targets=tg)
         assert np.array_equal(got.T, want)
+
+
+def upload(ctx, s):
+    ctx.call("gbh_state_upload", len(s["px"]), *[P(s[k]) for k in ("px", "py", "pz", "vx", "vy", "vz")], None, None, None,
+             P(s["mass"]), P(s["kind"]), P(s["alive"]))
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 63, 64, 65, 607, 2047, 2049, 4097])
+def test_exact_potential_bit_identical(ctx, n):
+    s = disk(n)
+    upload(ctx, s)
+    for dm_off, c in ((False, 0.0), (True, 4.0)):
+        d = ctx.diagnostics(abi.make_params(0.5, 0.03, 8, False, dm_off, "mixed"), c)
+        assert d["quality"] == 2
+        assert d["potential"] == O.potential_exact(s["px"], s["py"], s["pz"], s["mass"], s["kind"], 0.03, c, dm_off)
