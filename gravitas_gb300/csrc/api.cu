@@ -523,20 +523,17 @@ int run_split_steps(gbh_ctx *ctx, const gbh_params *p, double dt, int64_t nsteps
             while (double(k) * tau_min < 20.0 * dt && k < 256) k *= 2;
         ctx->last_substeps = k;
         CK(gbh::split_outer(L, sb, n, px, py, pz, ctx->mass, kind, dm, eps2, c));
-        CK(gbh::split_kick_outer(L, sb, n, h, vx, vy, vz, ctx->ax, ctx->ay, ctx->az));
+        CK(gbh::split_kick_outer(L, sb, n, h, true, dt, c, kind, px, py, pz, vx, vy, vz, ctx->ax, ctx->ay, ctx->az));
         const double hs = dt / double(k);
-        CK(gbh::split_fast(L, sb, n, nnear, px, py, pz, ctx->mass, kind, dm, eps2, c));
+        CK(gbh::split_fast(L, sb, n, nnear, false, 0.0, px, py, pz, vx, vy, vz, ctx->mass, kind, dm, eps2, c));
         for (int64_t q = 0; q < k; ++q) {
-            CK(gbh::split_fast_update(L, sb, n, nnear, false, 0.5 * hs, c, px, py, pz, vx, vy, vz));
-            CK(gbh::split_fast_update(L, sb, n, nnear, true, hs, c, px, py, pz, vx, vy, vz));
-            CK(gbh::split_fast(L, sb, n, nnear, px, py, pz, ctx->mass, kind, dm, eps2, c));
-            CK(gbh::split_fast_update(L, sb, n, nnear, false, 0.5 * hs, c, px, py, pz, vx, vy, vz));
+            CK(gbh::split_fast_open(L, sb, n, nnear, 0.5 * hs, hs, c, px, py, pz, vx, vy, vz));
+            CK(gbh::split_fast(L, sb, n, nnear, true, 0.5 * hs, px, py, pz, vx, vy, vz, ctx->mass, kind, dm, eps2, c));
         }
-        CK(gbh::split_drift_far(L, sb, n, dt, c, kind, px, py, pz, vx, vy, vz));
         int rc = slow();  // advanceGas without gas (blockstep.go:129-135)
         if (rc) return rc;
         CK(gbh::split_outer(L, sb, n, px, py, pz, ctx->mass, kind, dm, eps2, c));
-        CK(gbh::split_kick_outer(L, sb, n, h, vx, vy, vz, ctx->ax, ctx->ay, ctx->az));
+        CK(gbh::split_kick_outer(L, sb, n, h, false, 0.0, c, kind, px, py, pz, vx, vy, vz, ctx->ax, ctx->ay, ctx->az));
     }
     return GBH_OK;
 }

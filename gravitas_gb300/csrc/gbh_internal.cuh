@@ -310,16 +310,18 @@ cudaError_t split_classify(const Launch &L, SplitBufs &s, int64_t n, const doubl
 // far = hole pulls of the far stars and the far stars' pulls on the holes.
 cudaError_t split_outer(const Launch &L, SplitBufs &s, int64_t n, const double *px, const double *py,
                         const double *pz, const double *mass, const uint8_t *kind, int dm_off, double eps2, double c);
-cudaError_t split_kick_outer(const Launch &L, SplitBufs &s, int64_t n, double h, double *vx, double *vy, double *vz,
-                             const double *ax, const double *ay, const double *az);
-// fast = hole pulls of the near stars, and the holes' pulls from the other holes and the near stars.
-cudaError_t split_fast(const Launch &L, SplitBufs &s, int64_t n, int32_t nnear, const double *px, const double *py,
-                       const double *pz, const double *mass, const uint8_t *kind, int dm_off, double eps2, double c);
-// Near stars and holes: v += h fast (drift = false) or x += h v (drift = true).
-cudaError_t split_fast_update(const Launch &L, SplitBufs &s, int64_t n, int32_t nnear, bool drift, double h,
-                              double c, double *px, double *py, double *pz, double *vx, double *vy, double *vz);
-cudaError_t split_drift_far(const Launch &L, SplitBufs &s, int64_t n, double dt, double c, const uint8_t *kind,
-                            double *px, double *py, double *pz, const double *vx, const double *vy, const double *vz);
+// v += h (a + far) of every body; with drift the far bodies drift by dt right after their kick.
+cudaError_t split_kick_outer(const Launch &L, SplitBufs &s, int64_t n, double h, bool drift, double dt, double c,
+                             const uint8_t *kind, double *px, double *py, double *pz, double *vx, double *vy,
+                             double *vz, const double *ax, const double *ay, const double *az);
+// fast = hole pulls of the near stars, and the holes' pulls from the other holes and the near stars;
+// with kick then v += h fast of the near stars and holes (a substep's closing kick).
+cudaError_t split_fast(const Launch &L, SplitBufs &s, int64_t n, int32_t nnear, bool kick, double h, const double *px,
+                       const double *py, const double *pz, double *vx, double *vy, double *vz, const double *mass,
+                       const uint8_t *kind, int dm_off, double eps2, double c);
+// A substep's opening kick and drift of the near stars and holes: v += h fast, x += dt v (/ gamma).
+cudaError_t split_fast_open(const Launch &L, SplitBufs &s, int64_t n, int32_t nnear, double h, double dt, double c,
+                            double *px, double *py, double *pz, double *vx, double *vy, double *vz);
 
 // ---- adjoint.cu (gradient of the KDK leapfrog with the softened direct-sum force) ----
 // Scratch of the tree adjoint (walk_lists.cu): node-moment and source-star accumulators, each

@@ -128,166 +128,215 @@ __global__ void k_near_list(int64_t n, const uint8_t *__restrict__ near8, const 
     if (i == n - 1) out[1] = scan[i] + near8[i];
 }
 
-// outerHoleForces, far bodies (split.go:83-96): far stars feel every hole; near stars and holes
-// get 0 here (the holes' sums come from k_far_holes_*).
-__global__ void k_far_bodies(int64_t n, const double *__restrict__ px, const double *__restrict__ py,
-                             const double *__restrict__ pz, const double *__restrict__ mass,
-                             const uint8_t *__restrict__ kind, const uint8_t *__restrict__ near8,
-                             const int32_t *__restrict__ holes, int32_t nh, double eps2, double c, double *fx,
-                             double *fy, double *fz) {
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double x = 0, y = 0, z = 0;
-    if (kind[i] != GBH_BLACK_HOLE && !near8[i]) hole_pull(i, holes, nh, px, py, pz, mass, kind, eps2, c, x, y, z);
-    fx[i] = x;
-    fy[i] = y;
-    fz[i] = z;
-}
-
-// outerHoleForces, holes (split.go:97-116): partial sums of each hole's pull from the far stars
-// of one 256-body chunk, sequential in index order.
-__global__ void k_far_holes_part(int64_t n, const double *__restrict__ px, const double *__restrict__ py,
-                                 const double *__restrict__ pz, const double *__restrict__ mass,
-                                 const uint8_t *__restrict__ kind, const uint8_t *__restrict__ near8, int dm_off,
-                                 const int32_t *__restrict__ holes, int32_t nh, double eps2, double c,
-                                 double *part) {
-    __shared__ double sx[kHoleChunk], sy[kHoleChunk], sz[kHoleChunk], sm[kHoleChunk];
-    __shared__ uint8_t skip[kHoleChunk];
-    const int64_t c0 = int64_t(blockIdx.x) * kHoleChunk;
-    const int cnt = n - c0 < kHoleChunk ? int(n - c0) : kHoleChunk;
-    for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
-        int64_t i = c0 + q;
-        sx[q] = px[i];
-        sy[q] = py[i];
-        sz[q] = pz[i];
-        sm[q] = source_mass(i, mass, kind, dm_off);
-        skip[q] = kind[i] == GBH_BLACK_HOLE || near8[i];
+// outerHoleForces (split.go:83-116) of one 256-body chunk. Each body: far stars feel every hole;
+// near stars and holes get 0 here (the holes' sums are added by k_kick_outer). Each hole: the
+// chunk's far stars pull on it, summed in index order.
+//
+// A hole's sum is a serial chain of FP64 adds (72 cycles each), but its terms are independent:
+// every thread forms its own body's terms for up to kHoleBatch holes in shared memory (+0 for a
+// skipped body: the sums start at +0 and never become -0, so it changes nothing), and one lane per
+// hole and axis adds them in order. 20,000 bodies and 2 holes: 290 us with one thread a hole
+// running through the chunk's square roots and divisions, 24 us so (with the far bodies' own pulls).
+constexpr int kHoleBatch = 7;  // 43 KB of terms
+constexpr int kTermStride = kHoleChunk + 1;
+__global__ __launch_bounds__(kHoleChunk) void k_far_part(int64_t n, const double *__restrict__ px,
+                                                         const double *__restrict__ py, const double *__restrict__ pz,
+                                                         const double *__restrict__ mass,
+                                                         const uint8_t *__restrict__ kind,
+                                                         const uint8_t *__restrict__ near8, int dm_off,
+                                                         const int32_t *__restrict__ holes, int32_t nh, double eps2,
+                                                         double c, double *fx, double *fy, double *fz, double *part) {
+    __shared__ double s_term[3 * kHoleBatch][kTermStride];
+    const int64_t i = int64_t(blockIdx.x) * kHoleChunk + threadIdx.x;
+    const bool far = i < n && kind[i] != GBH_BLACK_HOLE && !near8[i];
+    double x = 0, y = 0, z = 0, sm = 0;
+    if (far) {
+        hole_pull(i, holes, nh, px, py, pz, mass, kind, eps2, c, x, y, z);
+        sm = source_mass(i, mass, kind, dm_off);
     }
-    __syncthreads();
-    for (int32_t k = threadIdx.x; k < nh; k += blockDim.x) {
-        int32_t h = holes[k];
-        double x = px[h], y = py[h], z = pz[h];
-        const double rs = schwarzschild(mass[h], c);
-        double ax = 0, ay = 0, az = 0;
-        for (int q = 0; q < cnt; ++q) {
-            if (skip[q]) continue;
-            double dx = sx[q] - x, dy = sy[q] - y, dz = sz[q] - z;
-            double f = pair_force(sm[q], dx * dx + dy * dy + dz * dz, eps2, rs);
-            ax += f * dx;
-            ay += f * dy;
-            az += f * dz;
+    if (i < n) {
+        fx[i] = x;
+        fy[i] = y;
+        fz[i] = z;
+    }
+    if (far) {
+        x = px[i];
+        y = py[i];
+        z = pz[i];
+    }
+    for (int32_t k0 = 0; k0 < nh; k0 += kHoleBatch) {
+        const int cnt = nh - k0 < kHoleBatch ? nh - k0 : kHoleBatch;
+        for (int k = 0; k < cnt; ++k) {
+            double tx = 0, ty = 0, tz = 0;
+            if (far) {
+                const int32_t h = holes[k0 + k];
+                const double dx = x - px[h], dy = y - py[h], dz = z - pz[h];
+                const double f = pair_force(sm, dx * dx + dy * dy + dz * dz, eps2, schwarzschild(mass[h], c));
+                tx = f * dx;
+                ty = f * dy;
+                tz = f * dz;
+            }
+            s_term[3 * k][threadIdx.x] = tx;
+            s_term[3 * k + 1][threadIdx.x] = ty;
+            s_term[3 * k + 2][threadIdx.x] = tz;
         }
-        double *p = part + (int64_t(blockIdx.x) * nh + k) * 3;
-        p[0] = ax;
-        p[1] = ay;
-        p[2] = az;
+        __syncthreads();
+        if (threadIdx.x < 3 * cnt) {
+            double a = 0;
+#pragma unroll 16
+            for (int q = 0; q < kHoleChunk; ++q) a += s_term[threadIdx.x][q];
+            part[(int64_t(blockIdx.x) * nh + k0) * 3 + threadIdx.x] = a;
+        }
+        __syncthreads();
     }
 }
 
-// Each hole's far-star pull: the chunk partials added in chunk order to 0.
-__global__ void k_far_holes_final(int64_t nchunks, const int32_t *__restrict__ holes, int32_t nh,
-                                  const double *__restrict__ part, double *fx, double *fy, double *fz) {
-    int32_t k = int32_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k >= nh) return;
-    double ax = 0, ay = 0, az = 0;
-    for (int64_t c = 0; c < nchunks; ++c) {
-        const double *p = part + (c * nh + k) * 3;
-        ax += p[0];
-        ay += p[1];
-        az += p[2];
+// kickOuter (split.go:206-213): every body, v += h (a + far), and with `drift` the drift by dt of
+// the far bodies (driftFar, split.go:236-250, no gas: neither a hole nor near) right after their
+// kick: the substeps between the two read and move only near stars and holes. The last nh blocks
+// take a hole each: its chunk partials added in chunk order to 0, then its kick.
+__global__ __launch_bounds__(kEw) void k_kick_outer(int64_t n, double h, bool drift, double dt, double c,
+                                                    const uint8_t *__restrict__ kind,
+                                                    const uint8_t *__restrict__ near8, double *px, double *py,
+                                                    double *pz, double *vx, double *vy, double *vz,
+                                                    const double *__restrict__ ax, const double *__restrict__ ay,
+                                                    const double *__restrict__ az, const double *__restrict__ fx,
+                                                    const double *__restrict__ fy, const double *__restrict__ fz,
+                                                    const int32_t *__restrict__ holes, int32_t nh, int64_t nchunks,
+                                                    const double *__restrict__ part) {
+    const int64_t nb = int64_t(gridDim.x) - nh;
+    if (int64_t(blockIdx.x) >= nb) {
+        __shared__ double s[3][kEw + 1];
+        const int32_t k = int32_t(blockIdx.x - nb);
+        double a = 0;
+        for (int64_t c0 = 0; c0 < nchunks; c0 += kEw) {
+            const int64_t q = c0 + threadIdx.x;
+            for (int e = 0; e < 3; ++e) s[e][threadIdx.x] = q < nchunks ? part[(q * nh + k) * 3 + e] : 0.0;
+            __syncthreads();
+            const int cnt = nchunks - c0 < kEw ? int(nchunks - c0) : kEw;
+            if (threadIdx.x < 3) {
+#pragma unroll 8
+                for (int t = 0; t < cnt; ++t) a += s[threadIdx.x][t];
+            }
+            __syncthreads();
+        }
+        if (threadIdx.x < 3) {
+            const int32_t i = holes[k];
+            double *v = threadIdx.x == 0 ? vx : threadIdx.x == 1 ? vy : vz;
+            const double *ac = threadIdx.x == 0 ? ax : threadIdx.x == 1 ? ay : az;
+            v[i] = v[i] + h * (ac[i] + a);
+        }
+        return;
     }
-    int32_t h = holes[k];
-    fx[h] = ax;
-    fy[h] = ay;
-    fz[h] = az;
-}
-
-// kickOuter (split.go:206-213): every body, v += h (a + far).
-__global__ void k_kick_outer(int64_t n, double h, double *vx, double *vy, double *vz, const double *__restrict__ ax,
-                             const double *__restrict__ ay, const double *__restrict__ az,
-                             const double *__restrict__ fx, const double *__restrict__ fy,
-                             const double *__restrict__ fz) {
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    vx[i] = vx[i] + h * (ax[i] + fx[i]);
-    vy[i] = vy[i] + h * (ay[i] + fy[i]);
-    vz[i] = vz[i] + h * (az[i] + fz[i]);
-}
-
-// fastForces, near stars (split.go:142-147): the pull of every hole.
-__global__ void k_fast_near(int32_t nnear, const int32_t *__restrict__ near, const double *__restrict__ px,
-                            const double *__restrict__ py, const double *__restrict__ pz,
-                            const double *__restrict__ mass, const uint8_t *__restrict__ kind,
-                            const int32_t *__restrict__ holes, int32_t nh, double eps2, double c, double *fx,
-                            double *fy, double *fz) {
-    int32_t q = int32_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (q >= nnear) return;
-    int32_t i = near[q];
-    double x, y, z;
-    hole_pull(i, holes, nh, px, py, pz, mass, kind, eps2, c, x, y, z);
-    fx[i] = x;
-    fy[i] = y;
-    fz[i] = z;
-}
-
-// fastForces, holes (split.go:148-158): the other holes, then the near stars in index order.
-__global__ void k_fast_holes(int32_t nnear, const int32_t *__restrict__ near, const double *__restrict__ px,
-                             const double *__restrict__ py, const double *__restrict__ pz,
-                             const double *__restrict__ mass, const uint8_t *__restrict__ kind, int dm_off,
-                             const int32_t *__restrict__ holes, int32_t nh, double eps2, double c, double *fx,
-                             double *fy, double *fz) {
-    int32_t k = int32_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k >= nh) return;
-    int32_t h = holes[k];
-    double x = px[h], y = py[h], z = pz[h];
-    const double rs = schwarzschild(mass[h], c);
-    double ax, ay, az;
-    hole_pull(h, holes, nh, px, py, pz, mass, kind, eps2, c, ax, ay, az);
-    for (int32_t q = 0; q < nnear; ++q) {
-        int32_t i = near[q];
-        double dx = px[i] - x, dy = py[i] - y, dz = pz[i] - z;
-        double f = pair_force(source_mass(i, mass, kind, dm_off), dx * dx + dy * dy + dz * dz, eps2, rs);
-        ax += f * dx;
-        ay += f * dy;
-        az += f * dz;
+    const bool hole = kind[i] == GBH_BLACK_HOLE;
+    if (hole)  // an alive hole is kicked by its own block; a dead one is not in the list (its far force is 0)
+        for (int32_t k = 0; k < nh; ++k)
+            if (holes[k] == i) return;
+    const double u = vx[i] + h * (ax[i] + fx[i]), v = vy[i] + h * (ay[i] + fy[i]), w = vz[i] + h * (az[i] + fz[i]);
+    vx[i] = u;
+    vy[i] = v;
+    vz[i] = w;
+    if (drift && !hole && !near8[i]) {
+        const double f = drift_factor(dt, u, v, w, c);
+        px[i] = px[i] + f * u;
+        py[i] = py[i] + f * v;
+        pz[i] = pz[i] + f * w;
     }
-    fx[h] = ax;
-    fy[h] = ay;
-    fz[h] = az;
 }
 
-// kickFast (split.go:215-224) and driftIdx (split.go:226-234, c = 0) over the near stars, then
-// the holes: entry q < nnear is near[q], the rest are the holes.
-__global__ void k_fast_update(int32_t nnear, const int32_t *__restrict__ near, const int32_t *__restrict__ holes,
-                              int32_t nh, int drift, double h, double c, double *px, double *py, double *pz,
-                              double *vx, double *vy, double *vz, const double *__restrict__ fx,
-                              const double *__restrict__ fy, const double *__restrict__ fz) {
+// fastForces (split.go:142-158) and, with `kick`, the closing half kick h of a substep (kickFast,
+// split.go:215-224). Near stars: the pull of every hole, a thread each. Holes, a block each: the
+// pulls of the other holes, then of the near stars in index order; the compute threads form a
+// tile's terms and three lanes add the previous tile's in order, as k_far_part does. 400 near
+// stars: 500 us with a thread a hole, 21 us so.
+constexpr int kFastThreads = kEw + 32;  // the last warp adds
+__global__ __launch_bounds__(kFastThreads) void k_fast(int32_t nnear, const int32_t *__restrict__ near,
+                                                       const double *__restrict__ px, const double *__restrict__ py,
+                                                       const double *__restrict__ pz, const double *__restrict__ mass,
+                                                       const uint8_t *__restrict__ kind, int dm_off,
+                                                       const int32_t *__restrict__ holes, int32_t nh, double eps2,
+                                                       double c, bool kick, double h, double *vx, double *vy,
+                                                       double *vz, double *fx, double *fy, double *fz) {
+    if (int32_t(blockIdx.x) >= nh) {
+        const int32_t q = (int32_t(blockIdx.x) - nh) * kFastThreads + threadIdx.x;
+        if (q >= nnear) return;
+        const int32_t i = near[q];
+        double x, y, z;
+        hole_pull(i, holes, nh, px, py, pz, mass, kind, eps2, c, x, y, z);
+        fx[i] = x;
+        fy[i] = y;
+        fz[i] = z;
+        if (kick) {
+            vx[i] = vx[i] + h * x;
+            vy[i] = vy[i] + h * y;
+            vz[i] = vz[i] + h * z;
+        }
+        return;
+    }
+    __shared__ double s_term[2][3][kEw + 1];
+    const int tid = threadIdx.x;
+    const int32_t hole = holes[blockIdx.x];
+    const double x = px[hole], y = py[hole], z = pz[hole];
+    const double rs = schwarzschild(mass[hole], c);
+    const int32_t total = nh + nnear;
+    const int32_t ntiles = (total + kEw - 1) / kEw;
+    double sum = 0;
+    for (int32_t t = 0; t <= ntiles; ++t) {
+        if (tid < kEw && t < ntiles) {
+            const int32_t q = t * kEw + tid;
+            double tx = 0, ty = 0, tz = 0;
+            if (q < total) {
+                const int32_t i = q < nh ? holes[q] : near[q - nh];
+                if (i != hole) {
+                    const double dx = px[i] - x, dy = py[i] - y, dz = pz[i] - z;
+                    // hole pairs are Newtonian (PairRS) and always pull
+                    const double m = q < nh ? mass[i] : source_mass(i, mass, kind, dm_off);
+                    const double f = pair_force(m, dx * dx + dy * dy + dz * dz, eps2, q < nh ? 0.0 : rs);
+                    tx = f * dx;
+                    ty = f * dy;
+                    tz = f * dz;
+                }
+            }
+            s_term[t & 1][0][tid] = tx;
+            s_term[t & 1][1][tid] = ty;
+            s_term[t & 1][2][tid] = tz;
+        } else if (t > 0 && tid >= kEw && tid < kEw + 3) {
+            const int cnt = total - (t - 1) * kEw < kEw ? total - (t - 1) * kEw : kEw;
+#pragma unroll 8
+            for (int k = 0; k < cnt; ++k) sum += s_term[(t - 1) & 1][tid - kEw][k];
+        }
+        __syncthreads();
+    }
+    if (tid >= kEw && tid < kEw + 3) {
+        double *f = tid == kEw ? fx : tid == kEw + 1 ? fy : fz;
+        f[hole] = sum;
+        if (kick) {
+            double *v = tid == kEw ? vx : tid == kEw + 1 ? vy : vz;
+            v[hole] = v[hole] + h * sum;
+        }
+    }
+}
+
+// The opening half kick of a substep (kickFast, split.go:215-224) and its drift (driftIdx,
+// split.go:226-234) over the near stars, then the holes: entry q < nnear is near[q], the rest are
+// the holes.
+__global__ void k_fast_open(int32_t nnear, const int32_t *__restrict__ near, const int32_t *__restrict__ holes,
+                            int32_t nh, double h, double dt, double c, double *px, double *py, double *pz, double *vx,
+                            double *vy, double *vz, const double *__restrict__ fx, const double *__restrict__ fy,
+                            const double *__restrict__ fz) {
     int32_t q = int32_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (q >= nnear + nh) return;
     int32_t i = q < nnear ? near[q] : holes[q - nnear];
-    if (drift) {
-        const double f = drift_factor(h, vx[i], vy[i], vz[i], c);
-        px[i] = px[i] + f * vx[i];
-        py[i] = py[i] + f * vy[i];
-        pz[i] = pz[i] + f * vz[i];
-    } else {
-        vx[i] = vx[i] + h * fx[i];
-        vy[i] = vy[i] + h * fy[i];
-        vz[i] = vz[i] + h * fz[i];
-    }
-}
-
-// driftFar (split.go:236-250, no gas): every body that is neither a hole nor near.
-__global__ void k_drift_far(int64_t n, double dt, double c, const uint8_t *__restrict__ kind,
-                            const uint8_t *__restrict__ near8, double *px, double *py, double *pz,
-                            const double *__restrict__ vx, const double *__restrict__ vy,
-                            const double *__restrict__ vz) {
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n || kind[i] == GBH_BLACK_HOLE || near8[i]) return;
-    const double f = drift_factor(dt, vx[i], vy[i], vz[i], c);
-    px[i] = px[i] + f * vx[i];
-    py[i] = py[i] + f * vy[i];
-    pz[i] = pz[i] + f * vz[i];
+    const double u = vx[i] + h * fx[i], v = vy[i] + h * fy[i], w = vz[i] + h * fz[i];
+    vx[i] = u;
+    vy[i] = v;
+    vz[i] = w;
+    const double f = drift_factor(dt, u, v, w, c);
+    px[i] = px[i] + f * u;
+    py[i] = py[i] + f * v;
+    pz[i] = pz[i] + f * w;
 }
 
 }  // namespace
@@ -360,53 +409,37 @@ cudaError_t split_classify(const Launch &L, SplitBufs &s, int64_t n, const doubl
 
 cudaError_t split_outer(const Launch &L, SplitBufs &s, int64_t n, const double *px, const double *py,
                         const double *pz, const double *mass, const uint8_t *kind, int dm_off, double eps2, double c) {
-    double *fx = s.far, *fy = fx + n, *fz = fy + n;
-    k_far_bodies<<<ew_blocks(n), kEw, 0, L.stream>>>(n, px, py, pz, mass, kind, s.near8, s.holes, s.nholes, eps2, c,
-                                                     fx, fy, fz);
-    SPLIT_LAUNCH_CHECK();
-    int64_t nchunks = (n + kHoleChunk - 1) / kHoleChunk;
-    k_far_holes_part<<<unsigned(nchunks), 64, 0, L.stream>>>(n, px, py, pz, mass, kind, s.near8, dm_off, s.holes,
-                                                            s.nholes, eps2, c, s.part);
-    SPLIT_LAUNCH_CHECK();
-    k_far_holes_final<<<unsigned((s.nholes + 63) / 64), 64, 0, L.stream>>>(nchunks, s.holes, s.nholes, s.part, fx,
-                                                                          fy, fz);
+    k_far_part<<<unsigned((n + kHoleChunk - 1) / kHoleChunk), kHoleChunk, 0, L.stream>>>(
+        n, px, py, pz, mass, kind, s.near8, dm_off, s.holes, s.nholes, eps2, c, s.far, s.far + n, s.far + 2 * n, s.part);
     SPLIT_LAUNCH_CHECK();
     return cudaSuccess;
 }
 
-cudaError_t split_kick_outer(const Launch &L, SplitBufs &s, int64_t n, double h, double *vx, double *vy, double *vz,
-                             const double *ax, const double *ay, const double *az) {
-    k_kick_outer<<<ew_blocks(n), kEw, 0, L.stream>>>(n, h, vx, vy, vz, ax, ay, az, s.far, s.far + n, s.far + 2 * n);
+cudaError_t split_kick_outer(const Launch &L, SplitBufs &s, int64_t n, double h, bool drift, double dt, double c,
+                             const uint8_t *kind, double *px, double *py, double *pz, double *vx, double *vy,
+                             double *vz, const double *ax, const double *ay, const double *az) {
+    k_kick_outer<<<ew_blocks(n) + unsigned(s.nholes), kEw, 0, L.stream>>>(
+        n, h, drift, dt, c, kind, s.near8, px, py, pz, vx, vy, vz, ax, ay, az, s.far, s.far + n, s.far + 2 * n, s.holes,
+        s.nholes, (n + kHoleChunk - 1) / kHoleChunk, s.part);
     SPLIT_LAUNCH_CHECK();
     return cudaSuccess;
 }
 
-cudaError_t split_fast(const Launch &L, SplitBufs &s, int64_t n, int32_t nnear, const double *px, const double *py,
-                       const double *pz, const double *mass, const uint8_t *kind, int dm_off, double eps2, double c) {
-    double *fx = s.fast, *fy = fx + n, *fz = fy + n;
-    if (nnear > 0) {
-        k_fast_near<<<ew_blocks(nnear), kEw, 0, L.stream>>>(nnear, s.near, px, py, pz, mass, kind, s.holes, s.nholes,
-                                                            eps2, c, fx, fy, fz);
-        SPLIT_LAUNCH_CHECK();
-    }
-    k_fast_holes<<<unsigned((s.nholes + 31) / 32), 32, 0, L.stream>>>(nnear, s.near, px, py, pz, mass, kind, dm_off,
-                                                                      s.holes, s.nholes, eps2, c, fx, fy, fz);
+cudaError_t split_fast(const Launch &L, SplitBufs &s, int64_t n, int32_t nnear, bool kick, double h, const double *px,
+                       const double *py, const double *pz, double *vx, double *vy, double *vz, const double *mass,
+                       const uint8_t *kind, int dm_off, double eps2, double c) {
+    const unsigned nb = unsigned(s.nholes) + unsigned((nnear + kFastThreads - 1) / kFastThreads);
+    k_fast<<<nb, kFastThreads, 0, L.stream>>>(nnear, s.near, px, py, pz, mass, kind, dm_off, s.holes, s.nholes, eps2, c,
+                                              kick, h, vx, vy, vz, s.fast, s.fast + n, s.fast + 2 * n);
     SPLIT_LAUNCH_CHECK();
     return cudaSuccess;
 }
 
-cudaError_t split_fast_update(const Launch &L, SplitBufs &s, int64_t n, int32_t nnear, bool drift, double h,
-                              double c, double *px, double *py, double *pz, double *vx, double *vy, double *vz) {
-    k_fast_update<<<ew_blocks(int64_t(nnear) + s.nholes), kEw, 0, L.stream>>>(
-        nnear, s.near, s.holes, s.nholes, drift ? 1 : 0, h, c, px, py, pz, vx, vy, vz, s.fast, s.fast + n,
-        s.fast + 2 * n);
-    SPLIT_LAUNCH_CHECK();
-    return cudaSuccess;
-}
-
-cudaError_t split_drift_far(const Launch &L, SplitBufs &s, int64_t n, double dt, double c, const uint8_t *kind,
-                            double *px, double *py, double *pz, const double *vx, const double *vy, const double *vz) {
-    k_drift_far<<<ew_blocks(n), kEw, 0, L.stream>>>(n, dt, c, kind, s.near8, px, py, pz, vx, vy, vz);
+cudaError_t split_fast_open(const Launch &L, SplitBufs &s, int64_t n, int32_t nnear, double h, double dt, double c,
+                            double *px, double *py, double *pz, double *vx, double *vy, double *vz) {
+    k_fast_open<<<ew_blocks(int64_t(nnear) + s.nholes), kEw, 0, L.stream>>>(nnear, s.near, s.holes, s.nholes, h, dt, c,
+                                                                            px, py, pz, vx, vy, vz, s.fast, s.fast + n,
+                                                                            s.fast + 2 * n);
     SPLIT_LAUNCH_CHECK();
     return cudaSuccess;
 }

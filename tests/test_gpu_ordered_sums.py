@@ -51,3 +51,27 @@ def test_exact_potential_bit_identical(ctx, n):
         d = ctx.diagnostics(abi.make_params(0.5, 0.03, 8, False, dm_off, "mixed"), c)
         assert d["quality"] == 2
         assert d["potential"] == O.potential_exact(s["px"], s["py"], s["pz"], s["mass"], s["kind"], 0.03, c, dm_off)
+
+
+@pytest.mark.parametrize("n,nholes,scale", [(3, 1, 1.0), (255, 2, 1.0), (257, 8, 0.3), (600, 15, 0.3), (1200, 3, 0.1)])
+def test_hole_steps_bit_identical(ctx, n, nholes, scale):
+    """Hole counts at the edges of the batches, few to all stars near a hole (scale shrinks the disk),
+    a dead hole with an acceleration of its own."""
+    s = ics.test_disk(n, seed=5, holes=False)
+    for k in ("px", "py", "pz"):
+        s[k] *= scale
+    at = np.linspace(0, n - 1, nholes).astype(int)
+    s["kind"][at] = O.BLACK_HOLE
+    s["mass"][at] = 2.0 / nholes
+    dead = int(at[-1]) if nholes > 2 else -1
+    if dead >= 0:
+        s["alive"][dead] = 0
+        s["ax"][dead] = 0.25
+    f9 = ("px", "py", "pz", "vx", "vy", "vz", "ax", "ay", "az")
+    got = {k: s[k].copy() for k in (*f9, "mass", "kind", "alive")}
+    ref = {k: v.copy() for k, v in got.items()}
+    ctx.call("gbh_step_kdk", abi.make_params(0.5, 0.06, 8, False, False, "fp64"), 4e-3, 3, 1, n, *[P(got[k]) for k in f9],
+             P(s["mass"]), P(s["kind"]), P(s["alive"]))
+    O.split_kdk(ref, 4e-3, 0.06, 0.5, 8, 3, acc_valid=True)
+    for k in f9:
+        assert np.array_equal(got[k], ref[k]), k
