@@ -70,8 +70,10 @@ struct Layout {
 struct __align__(16) TravMem {
     uint32_t stack[kStackCap];   // sibling ranges: first | (count - 1) << 29
     int32_t lvl[kLevels];        // first stack slot of each depth
-    float4 rq[32];               // the nodes of a step that the box test keeps, pair-interleaved
-    int32_t owner[32];           // source staging: the lane whose leaf run starts at each slot
+    union {
+        float4 rq[32];           // the nodes of a step that the box test keeps, pair-interleaved
+        int32_t owner[32];       // source staging: (leaf's first star - its slot) at each run's first slot
+    };
 };
 
 struct __align__(16) WarpMem {
@@ -317,6 +319,16 @@ __device__ __forceinline__ GroupOut walk_group(TravMem &W, Sink &sink, int lane,
         __syncwarp();
         scount = 0;
     };
+    // Two stars of the group (the first and the last lane's last), for a first look at what the box
+    // keeps: a node that one of them opens needs no look at the others (the same decisions). Most
+    // nodes that a group opens are opened by either: 1M merger walk 3.85 -> 3.78 ms, 16k Plummer
+    // 0.128 -> 0.122. What the walk does not gain from, measured here: prefix sums of the range
+    // lengths by ballots (POPC runs at a quarter of the shuffles' rate), the next step's records by
+    // cp.async during the list evaluation (global loads are 6 % of its stalls, the buffer costs a
+    // block per SM), fewer registers for 11 (one star a lane) or 9 blocks (two) per SM.
+    const float2 smx = make_float2(-__shfl_sync(kFull, t[0].tx, 0), -__shfl_sync(kFull, t[kS - 1].tx, 31));
+    const float2 smy = make_float2(-__shfl_sync(kFull, t[0].ty, 0), -__shfl_sync(kFull, t[kS - 1].ty, 31));
+    const float2 smz = make_float2(-__shfl_sync(kFull, t[0].tz, 0), -__shfl_sync(kFull, t[kS - 1].tz, 31));
     while (sp > 0) {
         // ---- pop the sibling ranges of the deepest level, at most 32 nodes; lane j takes node j
         // of their concatenation (the range holding it is the last one starting at or before j)
@@ -352,6 +364,7 @@ __device__ __forceinline__ GroupOut walk_group(TravMem &W, Sink &sink, int lane,
         }
         float4 na = make_float4(0.f, 0.f, 0.f, 0.f), nb = na, nc = na, nd = na;
         float cx = 0.f, cy = 0.f, cz = 0.f, lim = 0.f;
+        bool keep = false;
         if (node >= 0 && !bad) {
             na = nodes[node].a;
             nb = nodes[node].b;
@@ -374,13 +387,17 @@ __device__ __forceinline__ GroupOut walk_group(TravMem &W, Sink &sink, int lane,
             const float qy = fmaxf(0.f, fmaxf(by0 - cy, cy - by1));
             const float qz = fmaxf(0.f, fmaxf(bz0 - cz, cz - bz1));
             acc = qx * qx + qy * qy + qz * qz >= lim;
+            const float2 ex = add2(f2(cx), smx), ey = add2(f2(cy), smy), ez = add2(f2(cz), smz);
+            const float2 d2 = fma2(ez, ez, fma2(ey, ey, mul2(ex, ex)));
+            keep = !acc && !(d2.x < lim || d2.y < lim);
         }
-        const unsigned mref = __ballot_sync(kFull, node >= 0 && !bad && !acc);
+        const unsigned mref = __ballot_sync(kFull, keep);
         if (mref) {
-            // the box keeps these nodes: each lane tests its own stars against two of them at once
-            // (packed FP32x2); stars beyond the group repeat the group's first star
+            // the box keeps these nodes and the two stars do not open them: each lane tests its own
+            // stars against two of them at once (packed FP32x2); stars beyond the group repeat the
+            // group's first star
             const int slot = __popc(mref & lt), nref = __popc(mref);
-            if ((mref >> lane) & 1u) {
+            if (keep) {
                 float *rq = reinterpret_cast<float *>(&W.rq[0]) + (slot >> 1) * 8 + (slot & 1);
                 rq[0] = cx;
                 rq[2] = cy;
@@ -412,7 +429,7 @@ __device__ __forceinline__ GroupOut walk_group(TravMem &W, Sink &sink, int lane,
                 near |= (__any_sync(kFull, ny) ? 1u : 0u) << (p + 1);
             }
             __syncwarp();
-            if ((mref >> lane) & 1u) acc = !((near >> slot) & 1u);
+            if (keep) acc = !((near >> slot) & 1u);
         }
         const uint32_t link = __float_as_uint(nb.w);
         const bool open_in = node >= 0 && !bad && !acc && !(na.w < 0.f);
@@ -501,14 +518,12 @@ __device__ __forceinline__ GroupOut walk_group(TravMem &W, Sink &sink, int lane,
                 // slot cs + j belongs to the last leaf whose (clipped) run starts at or before it
                 const bool mine = open_leaf && excl < cs + 32 && excl + lc > cs;
                 const int p0 = excl > cs ? excl - cs : 0;
-                if (mine) W.owner[p0] = lane;
+                if (mine) W.owner[p0] = lo - excl;
                 const unsigned st = __reduce_or_sync(kFull, mine ? 1u << p0 : 0u);
                 __syncwarp();
                 const int j = cs + lane;
-                const int ow = j < T ? W.owner[31 - __clz(st & upto)] : 0;
-                const int olo = __shfl_sync(kFull, lo, ow), oex = __shfl_sync(kFull, excl, ow);
                 if (j < T) {
-                    const int32_t star = olo + (j - oex);
+                    const int32_t star = W.owner[31 - __clz(st & upto)] + j;
                     const float4 h = st_hi[star], l = st_lo[star];
                     const int en = scount + lane;
                     constexpr int P = Lay::kSrcPair;
@@ -678,7 +693,7 @@ __device__ __forceinline__ void store_acc(const GroupStars<kS> &G, const Acc (&a
 // kSplit: work item i walks part i % nparts of group i / nparts (walk_group's split mode) and
 // writes its sums by sorted index to part_acc[part][axis][star]; k_split_combine adds the parts.
 template <bool kQuad, bool kSoft, int kS, bool kSplit = false>
-__global__ __launch_bounds__(kLwThreads) void k_walk_lists(const DevInfo *info, const LNode *__restrict__ nodes,
+__global__ __launch_bounds__(kLwThreads, kS == 2 ? 8 : 10) void k_walk_lists(const DevInfo *info, const LNode *__restrict__ nodes,
                                                            const float4 *__restrict__ st_hi,
                                                            const float4 *__restrict__ st_lo,
                                                            const int32_t *__restrict__ order, float eps, float eps2,
