@@ -422,8 +422,7 @@ cudaError_t tree_at(const Launch &L, AdjTape &t, const double *x, const double *
     b.list_depth = 0;
     b.lpt = true;
     b.split = true;  // few groups: the forward walk shares each among several warps (the same lists)
-    return tree_build(L, b, t.n, x, y, z, t.m, nullptr, nullptr, ax, ay, az, t.theta, t.leaf, 0, false, false,
-                      nullptr, nullptr);
+    return tree_build(L, b, t.n, x, y, z, t.m, nullptr, nullptr, ax, ay, az, t.theta, t.leaf, 0, false, false);
 }
 
 // Accelerations at (x, y, z): FP64 and the tree force straight into (ax, ay, az); FP32 pairs

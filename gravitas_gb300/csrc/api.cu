@@ -47,8 +47,9 @@ struct gbh_ctx {
     // forest: systems of the resident state (nsys == 1: a plain state)
     int32_t nsys = 1;
     int64_t sys_gen = 0;      // incremented whenever the systems change
-    uint16_t *sys_of = nullptr;
-    int64_t sys_of_cap = 0;
+    int4 *sys_tiles = nullptr;  // the systems' sort tiles
+    int64_t sys_tiles_cap = 0;
+    gbh::ForestTiles tiles;
     int64_t *sys_off = nullptr;
     int64_t sys_off_cap = 0;
     bool have_state = false, acc_valid = false;
@@ -329,7 +330,7 @@ int forces(gbh_ctx *ctx, const gbh_params *p, int64_t n, const double *px, const
         gbh::NvtxRange r("tree build");
         CK(gbh::tree_build(L, ctx->tb, n, px, py, pz, mass, kind, alive, ax, ay, az, theta, leaf,
                            p->dark_matter_off, p->walk == GBH_WALK_FP64, p->walk == GBH_WALK_PLAIN,
-                           forest ? ctx->sys_of : nullptr, forest ? ctx->sys_off : nullptr));
+                           forest ? &ctx->tiles : nullptr));
     }
     if (ctx->fault_link && !ctx->capturing) {
         ctx->fault_link = false;
@@ -809,7 +810,7 @@ void gbh_destroy(gbh_ctx *c) {
     gbh::split_free(c->split);
     free_state(c);
     void *ptrs[] = {c->part,  c->scalar,   c->holes, c->targets,  c->tout,   c->probe,
-                    c->scratch3, c->rung, c->end_tick, c->sys_of, c->sys_off};
+                    c->scratch3, c->rung, c->end_tick, c->sys_tiles, c->sys_off};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     for (auto &ev : c->ev)
@@ -1107,8 +1108,7 @@ int gbh_state_diagnostics(gbh_ctx *ctx, const gbh_params *p, double c, gbh_diagn
         sa = ctx->scratch3;
         ctx->tb.group = 64;
         CK(gbh::tree_build(L, ctx->tb, n, ctx->px, ctx->py, ctx->pz, ctx->mass, kind, alive, sa, sa + n, sa + 2 * n,
-                           theta, leaf, p->dark_matter_off, fp64, fp64, forest ? ctx->sys_of : nullptr,
-                           forest ? ctx->sys_off : nullptr));
+                           theta, leaf, p->dark_matter_off, fp64, fp64, forest ? &ctx->tiles : nullptr));
         if (fp64) {
             CK(gbh::potential_fp64(L, ctx->tb, n, ctx->px, ctx->py, ctx->pz, ctx->mass, kind, alive, ctx->holes,
                                    int32_t(holes.size()), p->softening * p->softening, c, p->dark_matter_off,
@@ -1156,14 +1156,22 @@ int gbh_forest_upload(gbh_ctx *ctx, int32_t nsys, const int64_t *offsets, const 
     const int64_t n = offsets[nsys];
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
     if ((rc = upload_state(ctx, n, px, py, pz, vx, vy, vz, ax, ay, az, mass, kind, alive))) return rc;
-    std::vector<uint16_t> sys(static_cast<size_t>(n));
-    for (int32_t q = 0; q < nsys; ++q)
-        for (int64_t i = offsets[q]; i < offsets[q + 1]; ++i) sys[size_t(i)] = uint16_t(q);
-    CK(grow(ctx->sys_of, ctx->sys_of_cap, n + 1));
+    std::vector<int4> tiles;
+    int64_t most = 0;
+    for (int32_t q = 0; q < nsys; ++q) {
+        const int32_t first = int32_t(tiles.size());
+        const int64_t cnt = (offsets[q + 1] - offsets[q] + gbh::kSortTile - 1) / gbh::kSortTile;
+        for (int64_t t = 0; t < cnt; ++t)
+            tiles.push_back(make_int4(int32_t(offsets[q] + t * gbh::kSortTile), q, first, int32_t(cnt)));
+        most = std::max(most, cnt);
+    }
+    CK(grow(ctx->sys_tiles, ctx->sys_tiles_cap, int64_t(tiles.size()) + 1));
     CK(grow(ctx->sys_off, ctx->sys_off_cap, int64_t(nsys) + 1));
-    if (n > 0) CK(cudaMemcpy(ctx->sys_of, sys.data(), sizeof(uint16_t) * size_t(n), cudaMemcpyHostToDevice));
+    if (!tiles.empty())
+        CK(cudaMemcpy(ctx->sys_tiles, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(ctx->sys_off, offsets, sizeof(int64_t) * size_t(nsys + 1), cudaMemcpyHostToDevice));
-    ctx->h2d += int64_t(sizeof(uint16_t) * size_t(n) + sizeof(int64_t) * size_t(nsys + 1));
+    ctx->h2d += int64_t(sizeof(int4) * tiles.size() + sizeof(int64_t) * size_t(nsys + 1));
+    ctx->tiles = gbh::ForestTiles{ctx->sys_tiles, int32_t(tiles.size()), most, ctx->sys_off};
     ctx->nsys = nsys;
     ++ctx->sys_gen;
     return finish(ctx, false);

@@ -24,8 +24,7 @@ constexpr int kNoCell = 22;               // "starts no cell": duplicate of the 
 // caller gets GBH_ERR_ARG); every other value names the kernel whose bound or check failed
 // (GBH_ERR_LIMIT).
 constexpr int kErrNonFinite = 20;
-// A one-sweep sort pass or a single-pass scan whose look-back wait ran past its bound.
-constexpr int kErrSortWait = 30;
+// A single-pass scan whose look-back wait ran past its bound.
 constexpr int kErrScanWait = 31;
 
 // Per-build scalars kept on the device, so a step needs no host round trip.
@@ -44,6 +43,7 @@ struct DevInfo {
     uint32_t ngroups;         // mixed-walk groups of a forest
     int32_t next_tick;        // block steps: the earliest step end over all bodies
     uint32_t next_count;      // block steps: the bodies whose step ends at next_tick
+    uint32_t bbox_done;       // blocks of k_bbox that have finished (wraps to 0 by itself)
     // FP32 views for the FP32 upsweep: min corner and side as hi + lo pairs, and the
     // opening base 2 * half_L / theta per level L
     float min_hi[3], min_lo[3];
@@ -101,21 +101,18 @@ struct TreeBufs {
     int32_t group = 64;     // stars per mixed-walk group (32: the list walk, or 64), set before tree_build
     int32_t list_depth = 0; // the list walk's node-list depth (0: kDefaultListDepth), set per call
     // compaction / bbox
-    uint32_t *flag = nullptr;     // star flags, then their exclusive scan
+    uint32_t *flag = nullptr;     // active flags of a block step's event, then their exclusive scan
     Pos4 *pos4 = nullptr;         // (x, y, z, m) of every star in state order, one 32-byte record
-    double *bbox_part = nullptr;  // per-block partial min/max (6 per block)
+    long long *bbox_part = nullptr;  // per-block parts of the bounding box
     // sort
     uint64_t *keys = nullptr, *keys_alt = nullptr;
     int32_t *order = nullptr, *order_alt = nullptr;
-    uint32_t *hist = nullptr;     // radix digit table
-    // one-sweep sort and single-pass scans: digit histograms, tile counters and look-back words
-    // (cleared at the start of every build)
-    uint32_t *os_state = nullptr;
-    int64_t os_words = 0;
-    // larger states: single-pass scans of the three-launch passes' digit tables (a counter and
-    // the look-back words of each pass), cleared at each build
-    uint32_t *hs_state = nullptr;
-    int64_t hs_words = 0;
+    int32_t *tile_len = nullptr;  // lengths of the sorted runs, by their first tile (two arrays of cap_tiles)
+    int64_t cap_tiles = 0;
+    // single-pass scans: tile counters and look-back words (cleared by the build's first kernel)
+    uint32_t *lb_state = nullptr;
+    int64_t lb_words = 0, lb_sort = 0;  // lb_sort: where the large sort's words start
+    uint32_t *hist = nullptr;           // digit table of the large sort's radix passes
     // sorted stars
     double *sx = nullptr, *sy = nullptr, *sz = nullptr, *sm = nullptr;
     float4 *st_hi = nullptr, *st_lo = nullptr;
@@ -169,6 +166,16 @@ struct TreeBufs {
     DevInfo *info = nullptr;
 };
 
+// Sort tiles of a forest: runs of at most kSortTile bodies that never straddle systems, as (first
+// body, system, the system's first tile, the system's tiles), in state order.
+constexpr int kSortTile = 1024;
+struct ForestTiles {
+    const int4 *tiles = nullptr;
+    int32_t ntiles = 0;
+    int64_t most = 0;                  // tiles of the largest system
+    const int64_t *sys_off = nullptr;  // first body of each system (nsys + 1 entries)
+};
+
 // Launch helper context: stream and launch counter.
 struct Launch {
     cudaStream_t stream;
@@ -182,13 +189,19 @@ void tree_free(TreeBufs &b);
 // Builds the tree of the alive non-hole bodies; zeroes alive holes' accelerations. exact:
 // FP64 moments bit identical to the reference (the FP64 walk); otherwise the FP32 upsweep of
 // moments.cu, which feeds the FP32 walks.
-// Forests: sys_of (state order, nsys > 1 only) is each body's system, sys_off (nsys + 1 entries,
-// state order) the first body of each system; bodies of a system are contiguous.
+// Forests (nsys > 1): the tiles of the systems' contiguous bodies.
 cudaError_t tree_build(const Launch &L, TreeBufs &b, int64_t n, const double *px, const double *py,
                        const double *pz, const double *mass, const uint8_t *kind,
                        const uint8_t *alive, double *ax, double *ay, double *az, double theta,
                        int leaf_size, int dm_off, bool exact, bool plain_records = true,
-                       const uint16_t *sys_of = nullptr, const int64_t *sys_off = nullptr);
+                       const ForestTiles *forest = nullptr);
+// ---- sort.cu (collect, keys and sort of tree_build; compiled without FMA contraction) ----
+cudaError_t sort_stars(const Launch &L, TreeBufs &b, int64_t n, const double *px, const double *py, const double *pz,
+                       const double *mass, const uint8_t *kind, const uint8_t *alive, double *ax, double *ay,
+                       double *az, double theta, int dm_off, bool exact, const ForestTiles *forest);
+size_t sort_part_bytes();              // of bbox_part
+int64_t sort_lb_words(int64_t n);      // look-back words of a sort of up to n bodies
+int64_t sort_hist_words(int64_t n);    // digit table words of the same
 // Block time steps (see tree.cu): tick-0 opening kicks and rungs, drift of all bodies, and the
 // closing/opening kicks of the bodies whose step ends at tick. DevInfo.next_tick receives the
 // earliest step end over all bodies.

@@ -5,9 +5,7 @@
 // kick/drift are bit identical to it.
 //
 // Pipeline of tree_build (one stream, no host round trip):
-//   k_flags_bbox -> scan -> k_bbox_final -> k_compact_keys          (collect + keys, build.go:11-31, 62-113)
-//   8 x (k_rs_hist -> scan -> k_rs_scatter)                         (stable LSD radix sort, morton.go:25-49)
-//   k_gather                                                        (sorted copies, build.go:34-41)
+//   sort_stars (sort.cu)                                            (collect, keys, sort, build.go:11-41, 62-113)
 //   k_chain_count -> scan -> k_chain_emit -> scan -> k_ref_index -> k_emit_nodes
 //                                                                   (node set and links of buildNode, build.go:134-172)
 //   k_upsweep                                                       (finish, build.go:176-217)
@@ -27,6 +25,7 @@
 #include <climits>
 
 #include "gbh_internal.cuh"
+#include "lookback.cuh"
 
 namespace gbh {
 
@@ -36,12 +35,6 @@ constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
 
-constexpr int kRsThreads = 256;
-constexpr int kRsItems = 8;
-constexpr int kRsTile = kRsThreads * kRsItems;
-constexpr int kRsWarps = kRsThreads / 32;
-constexpr int kRsBins = 256;
-
 constexpr int kThreads = 256;
 
 inline unsigned blocks_for(int64_t n, int threads) {
@@ -49,42 +42,7 @@ inline unsigned blocks_for(int64_t n, int threads) {
     return unsigned(b < 1 ? 1 : b);
 }
 
-// Records a device-side consistency failure (checked by the host after the call).
-__device__ __forceinline__ void dev_error(DevInfo *info, int where) {
-    atomicExch(&info->err, 1);
-    info->err_where = where;
-}
-
 // ---------------------------------------------------------------- exclusive scan (uint32)
-
-__device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
-    int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += t;
-    }
-    return v;
-}
-
-// Block-wide exclusive scan of one value per thread; returns the exclusive prefix and the total.
-__device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t *s_warp, uint32_t &total) {
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t incl = warp_incl_scan(v);
-    if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = lane < (kScanThreads / 32) ? s_warp[lane] : 0;
-        uint32_t wi = warp_incl_scan(w);
-        if (lane < (kScanThreads / 32)) s_warp[lane] = wi - w;
-        if (lane == (kScanThreads / 32) - 1) s_warp[kScanThreads / 32] = wi;
-    }
-    __syncthreads();
-    uint32_t r = s_warp[warp] + incl - v;
-    total = s_warp[kScanThreads / 32];
-    __syncthreads();
-    return r;
-}
 
 __device__ __forceinline__ int64_t dyn_len(int64_t n, const int64_t *ndyn) {
     if (ndyn) {
@@ -106,7 +64,7 @@ __global__ __launch_bounds__(kScanThreads) void k_scan_reduce(const uint32_t *__
             if (base + k < ne) v += in[base + k];
     }
     uint32_t total;
-    block_excl_scan(v, s_warp, total);
+    block_excl_scan<kScanThreads>(v, s_warp, total);
     if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
@@ -124,7 +82,7 @@ __global__ __launch_bounds__(kScanThreads) void k_scan_apply(const uint32_t *in,
         s += v[k];
     }
     uint32_t total;
-    uint32_t run = block_excl_scan(s, s_warp, total) + (sums ? sums[blockIdx.x] : 0);
+    uint32_t run = block_excl_scan<kScanThreads>(s, s_warp, total) + (sums ? sums[blockIdx.x] : 0);
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
         if (base + k < ne) out[base + k] = run;
@@ -188,26 +146,11 @@ cudaError_t scan_rec(const Launch &L, const uint32_t *in, uint32_t *out, int64_t
     return cudaGetLastError();
 }
 
-// Polls of a look-back wait (the one-sweep sort's and the single-pass scan's) before the block
-// gives up and records an error: far beyond any wait of a running predecessor.
-constexpr int kOsSpinLimit = 1 << 22;
+constexpr int kLbScans = 2;  // of a build: chain counts, child counts
+inline int64_t lb_tiles(int64_t n) { return (n + kScanTile - 1) / kScanTile; }
 
-// Look-back words are read and written whole (count and flag in one word); nothing else is
-// passed through them, so volatile (uncached, untorn) accesses suffice.
-__device__ __forceinline__ uint32_t ld_volatile(const uint32_t *p) { return *reinterpret_cast<const volatile uint32_t *>(p); }
-__device__ __forceinline__ void st_volatile(uint32_t *p, uint32_t v) { *reinterpret_cast<volatile uint32_t *>(p) = v; }
-__device__ __forceinline__ unsigned long long ld_volatile64(const unsigned long long *p) {
-    return *reinterpret_cast<const volatile unsigned long long *>(p);
-}
-__device__ __forceinline__ void st_volatile64(unsigned long long *p, unsigned long long v) {
-    *reinterpret_cast<volatile unsigned long long *>(p) = v;
-}
-
-// Single-pass exclusive scan with decoupled look-back (one launch; every scan of tree_build, in
-// place of a reduce, a scan of the tile sums and an apply): a block takes the next tile
-// from *ctr, publishes its sum, adds its predecessors' (their inclusive prefix, or their sums
-// back to one that has published a prefix) and publishes its own inclusive prefix. Waits are
-// bounded as in the one-sweep sort. status: one 64-bit word per tile (flag in the top 2 bits).
+// Single-pass exclusive scan with decoupled look-back (one launch, in place of a reduce, a scan of
+// the tile sums and an apply): a block takes the next tile from *ctr.
 __global__ __launch_bounds__(kScanThreads) void k_scan_lb(const uint32_t *in, uint32_t *out, int64_t n,
                                                           const int64_t *ndyn, uint32_t *ctr,
                                                           unsigned long long *status, DevInfo *info) {
@@ -228,51 +171,10 @@ __global__ __launch_bounds__(kScanThreads) void k_scan_lb(const uint32_t *in, ui
         sum += v[k];
     }
     uint32_t total;
-    uint32_t run = block_excl_scan(sum, s_warp, total);
+    uint32_t run = block_excl_scan<kScanThreads>(sum, s_warp, total);
     if (threadIdx.x < 32) {
-        // warp 0 publishes the tile's sum, then reads its predecessors' words 32 at a time (lane j
-        // the (j+1)-th tile back) and adds them down to the nearest published prefix
-        constexpr unsigned long long kAgg = 1ull << 62, kPre = 2ull << 62, kVal = (1ull << 62) - 1;
-        const int lane = threadIdx.x;
-        unsigned long long excl = 0;
-        if (tile == 0) {
-            if (lane == 0) st_volatile64(status, kPre | total);
-        } else {
-            if (lane == 0) st_volatile64(status + tile, kAgg | total);
-            int64_t t = int64_t(tile) - 1;
-            int spins = 0;
-            bool bad = false;
-            for (;;) {
-                const int64_t idx = t - lane;
-                unsigned long long w = idx >= 0 ? ld_volatile64(status + idx) : kPre;  // before tile 0: prefix 0
-                // every word up to the nearest prefix must be published; wait for the others
-                for (;;) {
-                    const unsigned pre = __ballot_sync(0xffffffffu, (w >> 62) == 2);
-                    const unsigned upto = pre ? (pre & (0u - pre)) * 2u - 1u : 0xffffffffu;  // lanes to the first prefix
-                    const unsigned wait = __ballot_sync(0xffffffffu, !(w >> 62)) & upto;
-                    if (!wait) break;
-                    if (++spins > kOsSpinLimit) {
-                        bad = true;
-                        break;
-                    }
-                    if ((wait >> lane) & 1u) w = ld_volatile64(status + idx);
-                }
-                if (bad) break;
-                const unsigned pre = __ballot_sync(0xffffffffu, (w >> 62) == 2);
-                const unsigned upto = pre ? (pre & (0u - pre)) * 2u - 1u : 0xffffffffu;
-                unsigned long long v = ((upto >> lane) & 1u) ? (w & kVal) : 0ull;
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                excl += v;
-                if (pre) break;
-                t -= 32;
-            }
-            if (lane == 0) {
-                if (bad) dev_error(info, kErrScanWait);
-                st_volatile64(status + tile, kPre | ((excl + total) & kVal));
-            }
-        }
-        if (lane == 0) s_prefix = excl;
+        const unsigned long long excl = look_back(status, tile, total, info);
+        if (threadIdx.x == 0) s_prefix = excl;
     }
     __syncthreads();
     run += uint32_t(s_prefix);
@@ -281,548 +183,6 @@ __global__ __launch_bounds__(kScanThreads) void k_scan_lb(const uint32_t *in, ui
         if (base + k < ne) out[base + k] = run;
         run += v[k];
     }
-}
-
-// ---------------------------------------------------------------- collect + bbox + keys
-
-__device__ __forceinline__ bool is_star(uint8_t alive, uint8_t kind) { return alive && kind != GBH_BLACK_HOLE; }
-
-// Order-preserving map of a double to a signed 64-bit integer (an involution): min and max of
-// the keys are the keys of the min and max, computed on the integer ALU instead of the slow
-// FP64 pipe. (-0 orders before +0; the coordinates are not NaN.)
-__device__ __forceinline__ long long ord_key(double v) {
-    long long b = __double_as_longlong(v);
-    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
-}
-__device__ __forceinline__ double ord_val(long long k) { return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll)); }
-
-// Per-block min/max of the 6 ordered keys into part[6 * blockIdx.x ...] (as raw 64-bit words).
-template <int kBlock>
-__device__ __forceinline__ void block_minmax(long long mn[3], long long mx[3], double *part) {
-    __shared__ long long s[6][kBlock / 32];
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        for (int o = 16; o > 0; o >>= 1) {
-            mn[c] = min(mn[c], __shfl_xor_sync(0xffffffffu, mn[c], o));
-            mx[c] = max(mx[c], __shfl_xor_sync(0xffffffffu, mx[c], o));
-        }
-        if (lane == 0) {
-            s[c][warp] = mn[c];
-            s[3 + c][warp] = mx[c];
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        bool isMin = threadIdx.x < 3;
-        long long v = s[threadIdx.x][0];
-        for (int w = 1; w < kBlock / 32; ++w) v = isMin ? min(v, s[threadIdx.x][w]) : max(v, s[threadIdx.x][w]);
-        part[blockIdx.x * 6 + threadIdx.x] = __longlong_as_double(v);
-    }
-}
-
-// Star flags, per-block bbox partials; alive holes get zero acceleration (bh.go:99-101).
-// A non-finite coordinate of a star makes the bbox non-finite by itself (NaN and infinities map to
-// keys beyond every finite one); a non-finite mass is folded in as the key of a NaN, so that
-// k_bbox_final can reject the input before keys are formed (collect, build.go:62-113, would
-// carry a NaN into the root cube and every key).
-__global__ __launch_bounds__(kThreads) void k_flags_bbox(int64_t n, const double *__restrict__ px,
-                                                         const double *__restrict__ py, const double *__restrict__ pz,
-                                                         const double *__restrict__ mass,
-                                                         const uint8_t *__restrict__ kind,
-                                                         const uint8_t *__restrict__ alive, uint32_t *__restrict__ flag,
-                                                         double *__restrict__ part, double *ax, double *ay, double *az,
-                                                         DevInfo *info, Pos4 *__restrict__ pos4) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {  // the build's first kernel clears the error record
-        info->err = 0;
-        info->err_where = 0;
-    }
-    long long mn[3] = {LLONG_MAX, LLONG_MAX, LLONG_MAX}, mx[3] = {LLONG_MIN, LLONG_MIN, LLONG_MIN};
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-        uint8_t al = alive ? alive[i] : 1, kd = kind ? kind[i] : 0;
-        bool st = is_star(al, kd);
-        flag[i] = st;
-        if (st) {
-            const double vx = px[i], vy = py[i], vz = pz[i], m = mass ? mass[i] : 0.0;
-            pos4[i] = Pos4{vx, vy, vz, m};  // one record for k_gather's reads through the sort order
-            long long x = ord_key(vx), y = ord_key(vy), z = ord_key(vz);
-            mn[0] = min(mn[0], x);
-            mx[0] = max(mx[0], mass && !isfinite(m) ? LLONG_MAX : x);
-            mn[1] = min(mn[1], y);
-            mx[1] = max(mx[1], y);
-            mn[2] = min(mn[2], z);
-            mx[2] = max(mx[2], z);
-        } else if (al && kd == GBH_BLACK_HOLE) {
-            ax[i] = 0;
-            ay[i] = 0;
-            az[i] = 0;
-        }
-    }
-    block_minmax<kThreads>(mn, mx, part);
-}
-
-// Root cube (build.go:19-21): side = max(max extent * (1+1e-9), 1e-12), scale = 2^21 / side.
-// One block reduces the per-block partials (min/max are exact, so the order does not matter).
-constexpr int kFinalThreads = 1024;
-__global__ __launch_bounds__(kFinalThreads) void k_bbox_final(int nparts, const double *__restrict__ part, int64_t n,
-                                                              const uint32_t *__restrict__ scan, const uint8_t *kind,
-                                                              const uint8_t *alive, double theta, DevInfo *info,
-                                                              SysGeo *geo) {
-    long long kmn[3] = {LLONG_MAX, LLONG_MAX, LLONG_MAX}, kmx[3] = {LLONG_MIN, LLONG_MIN, LLONG_MIN};
-    for (int b = threadIdx.x; b < nparts; b += blockDim.x)
-        for (int c = 0; c < 3; ++c) {
-            kmn[c] = min(kmn[c], __double_as_longlong(part[b * 6 + c]));
-            kmx[c] = max(kmx[c], __double_as_longlong(part[b * 6 + 3 + c]));
-        }
-    __shared__ long long s[6][kFinalThreads / 32];
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int c = 0; c < 3; ++c) {
-        for (int o = 16; o > 0; o >>= 1) {
-            kmn[c] = min(kmn[c], __shfl_xor_sync(0xffffffffu, kmn[c], o));
-            kmx[c] = max(kmx[c], __shfl_xor_sync(0xffffffffu, kmx[c], o));
-        }
-        if (lane == 0) {
-            s[c][warp] = kmn[c];
-            s[3 + c][warp] = kmx[c];
-        }
-    }
-    __syncthreads();
-    // warp 0 reduces the warps' values (lane w holds warp w's)
-    if (warp != 0) return;
-    static_assert(kFinalThreads / 32 == 32, "one value per lane");
-    double mn[3], mx[3];
-    for (int c = 0; c < 3; ++c) {
-        long long a = s[c][lane], b = s[3 + c][lane];
-        for (int o = 16; o > 0; o >>= 1) {
-            a = min(a, __shfl_xor_sync(0xffffffffu, a, o));
-            b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
-        }
-        mn[c] = ord_val(a);
-        mx[c] = ord_val(b);
-    }
-    double side = fmax(mx[0] - mn[0], fmax(mx[1] - mn[1], mx[2] - mn[2]));
-    side = fmax(side * (1 + 1e-9), 1e-12);
-    // opening bases 2 half_L / theta, half_L = side / 2^(L+1): halving is exact, so lane L forms its
-    // own level's half with one exact scaling instead of L successive halvings
-    if (lane <= kMaxLevel) {
-        const double half = ldexp(side, -(lane + 1));
-        info->crit_base[lane] = __double2float_rn(2 * half / theta);
-        if (geo) geo[0].crit_base[lane] = info->crit_base[lane];
-    }
-    if (lane != 0) return;
-    int64_t ns = 0;
-    if (n > 0) ns = int64_t(scan[n - 1]) + (is_star(alive ? alive[n - 1] : 1, kind ? kind[n - 1] : 0) ? 1 : 0);
-    info->minx = mn[0];
-    info->miny = mn[1];
-    info->minz = mn[2];
-    info->side = side;
-    info->scale = double(1 << kMortonBits) / side;
-    info->theta = theta;
-    info->nstars = ns;
-    info->nnodes = 0;
-    info->work = 0;
-    info->nleaves = 0;
-    if (ns > 0 && !(isfinite(mn[0]) && isfinite(mn[1]) && isfinite(mn[2]) && isfinite(mx[0]) && isfinite(mx[1]) &&
-                    isfinite(mx[2]))) {
-        info->err = 1;  // reported to the caller as GBH_ERR_ARG
-        info->err_where = kErrNonFinite;
-    }
-    for (int c = 0; c < 3; ++c) {
-        float h = __double2float_rn(mn[c]);
-        info->min_hi[c] = h;
-        info->min_lo[c] = __double2float_rn(mn[c] - double(h));
-    }
-    float sh = __double2float_rn(side);
-    info->side_hi = sh;
-    info->side_lo = __double2float_rn(side - double(sh));
-    if (geo) {  // the single system of a plain state
-        SysGeo &g = geo[0];
-        g.minx = info->minx;
-        g.miny = info->miny;
-        g.minz = info->minz;
-        g.side = side;
-        g.scale = info->scale;
-        for (int c = 0; c < 3; ++c) {
-            g.min_hi[c] = info->min_hi[c];
-            g.min_lo[c] = info->min_lo[c];
-        }
-        g.side_hi = info->side_hi;
-        g.side_lo = info->side_lo;
-        g.star_lo = 0;
-        g.star_hi = int32_t(ns);
-        g.root = 0;
-        g.group_lo = 0;
-        g.ngroups = int32_t((ns + 63) / 64);
-    }
-}
-
-// morton.go:7-15.
-__device__ __forceinline__ uint64_t spread(uint64_t v) {
-    v &= (uint64_t(1) << kMortonBits) - 1;
-    v = (v | v << 32) & 0x1f00000000ffffull;
-    v = (v | v << 16) & 0x1f0000ff0000ffull;
-    v = (v | v << 8) & 0x100f00f00f00f00full;
-    v = (v | v << 4) & 0x10c30c30c30c30c3ull;
-    v = (v | v << 2) & 0x1249249249249249ull;
-    return v;
-}
-
-// cell(), build.go:23-25: uint64(min(2^21-1, max(0, (v-lo)*scale))).
-__device__ __forceinline__ uint64_t cell(double v, double lo, double scale) {
-    double t = fmin(double((1 << kMortonBits) - 1), fmax(0.0, (v - lo) * scale));
-    return uint64_t(t);
-}
-
-// order[k] = i for the k-th star in state order; keys[k] = mortonKey(cells) (build.go:26-31).
-__global__ __launch_bounds__(kThreads) void k_compact_keys(int64_t n, const double *__restrict__ px,
-                                                           const double *__restrict__ py, const double *__restrict__ pz,
-                                                           const uint8_t *__restrict__ kind,
-                                                           const uint8_t *__restrict__ alive,
-                                                           const uint32_t *__restrict__ scan, const DevInfo *info,
-                                                           uint64_t *__restrict__ keys, int32_t *__restrict__ order) {
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (!is_star(alive ? alive[i] : 1, kind ? kind[i] : 0)) return;
-    double sc = info->scale;
-    uint64_t k = spread(cell(px[i], info->minx, sc)) << 2 | spread(cell(py[i], info->miny, sc)) << 1 |
-                 spread(cell(pz[i], info->minz, sc));
-    uint32_t pos = scan[i];
-    keys[pos] = k;
-    order[pos] = int32_t(i);
-}
-
-// ---------------------------------------------------------------- stable LSD radix sort
-
-// kSid: the digit is taken from the system id of the element's body (forest sorts by system
-// after the 8 key passes) instead of the key.
-template <bool kSid>
-__global__ __launch_bounds__(kRsThreads) void k_rs_hist(const uint64_t *__restrict__ keys, const int32_t *__restrict__ vals,
-                                                        const uint16_t *__restrict__ sys_of, const DevInfo *info,
-                                                        int shift, uint32_t ntiles, uint32_t *__restrict__ hist) {
-    __shared__ uint32_t h[kRsBins];
-    int64_t n = info->nstars;
-    h[threadIdx.x] = 0;
-    __syncthreads();
-    int64_t base = int64_t(blockIdx.x) * kRsTile;
-    if (base < n) {
-#pragma unroll
-        for (int it = 0; it < kRsItems; ++it) {
-            int64_t idx = base + it * kRsThreads + threadIdx.x;
-            if (idx < n) {
-                uint32_t d = kSid ? uint32_t(sys_of[vals[idx]] >> shift) : uint32_t(keys[idx] >> shift);
-                atomicAdd(&h[d & (kRsBins - 1)], 1u);
-            }
-        }
-    }
-    __syncthreads();
-    hist[size_t(threadIdx.x) * ntiles + blockIdx.x] = h[threadIdx.x];
-}
-
-// Stable scatter of one tile. Rank of a key = keys of the same digit earlier in the tile, in
-// the order (item round, warp, lane) used to load them; offs holds the digit-major exclusive
-// scan of the tile histograms, so equal digits keep their input order across tiles too.
-template <bool kSid>
-__global__ __launch_bounds__(kRsThreads) void k_rs_scatter(const uint64_t *__restrict__ kin,
-                                                           const int32_t *__restrict__ vin,
-                                                           uint64_t *__restrict__ kout, int32_t *__restrict__ vout,
-                                                           const uint16_t *__restrict__ sys_of, DevInfo *info, int shift,
-                                                           uint32_t ntiles, const uint32_t *__restrict__ offs) {
-    __shared__ uint32_t s_run[kRsBins];
-    __shared__ uint32_t s_goff[kRsBins];
-    __shared__ uint32_t s_w[2][kRsWarps][kRsBins];
-    int64_t n = info->nstars;
-    int64_t base = int64_t(blockIdx.x) * kRsTile;
-    if (base >= n) return;  // uniform over the block
-    int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    s_run[tid] = 0;
-    s_goff[tid] = offs[size_t(tid) * ntiles + blockIdx.x];
-#pragma unroll
-    for (int w = 0; w < kRsWarps; ++w) {
-        s_w[0][w][tid] = 0;
-        s_w[1][w][tid] = 0;
-    }
-    uint64_t k[kRsItems];
-    int32_t v[kRsItems];
-#pragma unroll
-    for (int it = 0; it < kRsItems; ++it) {
-        int64_t idx = base + it * kRsThreads + tid;
-        if (idx < n) {
-            k[it] = kin[idx];
-            v[it] = vin[idx];
-        }
-    }
-    __syncthreads();
-    const uint32_t lt = (1u << lane) - 1u;
-#pragma unroll
-    for (int it = 0; it < kRsItems; ++it) {
-        const int buf = it & 1;
-        int64_t idx = base + it * kRsThreads + tid;
-        bool valid = idx < n;
-        uint32_t d = 0u;
-        if (valid) d = (kSid ? uint32_t(sys_of[v[it]] >> shift) : uint32_t(k[it] >> shift)) & (kRsBins - 1);
-        uint32_t peers = __match_any_sync(0xffffffffu, valid ? d : uint32_t(kRsBins + lane));
-        uint32_t rank = __popc(peers & lt);
-        if (valid && rank == 0) s_w[buf][warp][d] = __popc(peers);
-        __syncthreads();
-        uint32_t run = s_run[tid];
-#pragma unroll
-        for (int w = 0; w < kRsWarps; ++w) {
-            uint32_t c = s_w[buf][w][tid];
-            s_w[buf][w][tid] = run;
-            run += c;
-            s_w[buf ^ 1][w][tid] = 0;  // readers of the other buffer finished before this round's first barrier
-        }
-        s_run[tid] = run;
-        __syncthreads();
-        if (valid) {
-            uint32_t pos = s_goff[d] + s_w[buf][warp][d] + rank;
-            if (pos < n) {
-                kout[pos] = k[it];
-                vout[pos] = v[it];
-            } else {
-                dev_error(info, 10);
-            }
-        }
-    }
-}
-
-// ---------------------------------------------------------------- one-sweep radix sort
-//
-// The same stable LSD sort in one launch per pass after a single histogram launch. k_os_hist
-// reads the keys once and counts every pass's digits (and, for a forest, the two system-id
-// digits); a pass block takes the next tile from a counter, ranks its keys exactly as
-// k_rs_scatter does, publishes its per-digit counts and then looks back over its predecessors'
-// published counts (decoupled look-back: a predecessor's word holds either its own count or its
-// inclusive prefix) to find where each of its digits starts. Tiles are taken in counter order, so
-// every tile a block waits for belongs to a block that is already running. Each wait is bounded:
-// past kOsSpinLimit polls the block records an error (reported as GBH_ERR_LIMIT), publishes what
-// it has so that its successors are not held, and its output is not used.
-
-constexpr int kOsPassesMax = 10;  // 8 key digits, then 2 system-id digits (forest)
-constexpr uint32_t kOsAgg = 1u << 30, kOsPre = 2u << 30, kOsCount = (1u << 30) - 1u;
-// States of up to kOsMaxN bodies (capacity) build with the one-sweep sort and single-pass scans;
-// larger ones with the three-launch passes. Measured on the merger (CUDA events, whole build,
-// one-sweep against three-launch): 16k bodies 0.29 / 0.36 ms, 64k 0.32 / 0.45, 131k 0.36 / 0.46,
-// 262k 0.41 / 0.50, 1M 0.72 / 0.69. With every tile of a large pass resident at once, each
-// tile's look-back walks back to the nearest published prefix while all of them are still
-// aggregates, a chain of L2 round trips that outgrows the launches it saves.
-constexpr int64_t kOsMaxN = int64_t(3) << 18;
-static_assert(kOsMaxN * 8 < int64_t(kOsCount), "one-sweep counts are 30-bit");
-constexpr int kOsHistBlocksPerSm = 2;
-constexpr int kOsWindow = 8;  // predecessors' look-back words read per round trip
-
-// Word offsets inside TreeBufs::os_state.
-constexpr int64_t kOsHistWords = int64_t(kOsPassesMax) * kRsBins;  // [pass][digit]
-constexpr int64_t kOsCtrWords = 32;                                 // tile counters: passes, then scans
-constexpr int kOsScanCtr = kOsPassesMax;                            // first scan counter
-constexpr int kOsScans = 3;                                         // flags, chain counts, child counts
-__host__ __device__ inline int64_t os_scan_tiles(int64_t n) { return (n + kScanTile - 1) / kScanTile; }
-// Keys a thread of a one-sweep pass ranks: the fewest of 4, 8, 12 that keep a state of `cap`
-// bodies within 96 tiles (measured: more tiles spread a small sort over more SMs, fewer tiles
-// shorten the look-back; against 8 keys a thread, 4 made the 16k build 6 % faster and 12 the
-// 262k build 4 % faster).
-inline int os_items(int64_t cap) { return cap <= 96 * 4 * kRsThreads ? 4 : cap <= 96 * 8 * kRsThreads ? 8 : 12; }
-inline int64_t os_sort_tiles(int64_t n, int items) {
-    const int64_t tile = int64_t(items) * kRsThreads;
-    return (n + tile - 1) / tile;
-}
-inline int64_t rs_sort_tiles(int64_t n) { return (n + kRsTile - 1) / kRsTile; }
-
-// Every pass's digit histogram in one read of the keys (warp-aggregated shared counters, then one
-// global add per non-zero bin and block).
-template <bool kSid>
-__global__ __launch_bounds__(kRsThreads) void k_os_hist(const uint64_t *__restrict__ keys,
-                                                        const int32_t *__restrict__ vals,
-                                                        const uint16_t *__restrict__ sys_of, const DevInfo *info,
-                                                        uint32_t *__restrict__ ghist) {
-    constexpr int kPasses = kSid ? kOsPassesMax : 8;
-    __shared__ uint32_t h[kPasses * kRsBins];
-    for (int i = threadIdx.x; i < kPasses * kRsBins; i += blockDim.x) h[i] = 0;
-    __syncthreads();
-    const int64_t n = info->nstars;
-    const int lane = threadIdx.x & 31;
-    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    // whole warps iterate together (the match below needs every lane)
-    for (int64_t i0 = int64_t(blockIdx.x) * blockDim.x + (threadIdx.x & ~31); i0 < n; i0 += stride) {
-        const int64_t i = i0 + lane;
-        const bool valid = i < n;
-        const uint64_t k = valid ? keys[i] : 0;
-        const uint32_t sd = kSid && valid ? uint32_t(sys_of[vals[i]]) : 0u;
-#pragma unroll
-        for (int p = 0; p < kPasses; ++p) {
-            const uint32_t d = p < 8 ? uint32_t(k >> (8 * p)) & 255u : (sd >> (8 * (p - 8))) & 255u;
-            const uint32_t peers = __match_any_sync(0xffffffffu, valid ? d : 256u + lane);
-            if (valid && (peers & ((1u << lane) - 1u)) == 0) atomicAdd(&h[p * kRsBins + d], __popc(peers));
-        }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < kPasses * kRsBins; i += blockDim.x)
-        if (h[i]) atomicAdd(&ghist[i], h[i]);
-}
-
-// Ranks a tile's keys by digit, stably, for the one-sweep pass. Warp w holds the tile's keys
-// [w, w + 1) x kItems x 32 (item it of lane l: position w kItems 32 + it 32 + l), so the
-// order (warp, item, lane) is the input order. Each warp counts its own keys per digit in
-// s_w[w][digit] (the lowest lane of each group of equal digits reads and advances the counter;
-// no block barrier inside the loop), so a key's rank among its warp's earlier keys of the same
-// digit is the counter before its group plus its place in the group. On return s_w holds the
-// warp counts (the caller turns them into offsets after a barrier). Measured against the
-// round-barrier ranking of k_rs_scatter: the one-sweep builds 2-4 % faster (16k-262k bodies);
-// in k_rs_scatter it made the 1M and 4M builds 3-5 % slower, so that kernel keeps its own.
-template <bool kSid, int kItems>
-__device__ __forceinline__ void rank_tile(const uint64_t *__restrict__ kin, const int32_t *__restrict__ vin,
-                                          const uint16_t *__restrict__ sys_of, int shift, int64_t base, int64_t n,
-                                          uint32_t (&s_w)[kRsWarps][kRsBins], uint64_t (&k)[kItems],
-                                          int32_t (&v)[kItems], uint32_t (&dig)[kItems], uint32_t (&rk)[kItems]) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-#pragma unroll
-    for (int w = 0; w < kRsWarps; ++w) s_w[w][tid] = 0;
-    const int64_t wbase = base + int64_t(warp) * (kItems * 32);
-#pragma unroll
-    for (int it = 0; it < kItems; ++it) {
-        const int64_t idx = wbase + it * 32 + lane;
-        if (idx < n) {
-            k[it] = kin[idx];
-            v[it] = vin[idx];
-        }
-    }
-    __syncthreads();  // counters cleared
-    const uint32_t lt = (1u << lane) - 1u;
-#pragma unroll
-    for (int it = 0; it < kItems; ++it) {
-        const bool valid = wbase + it * 32 + lane < n;
-        uint32_t d = 0u;
-        if (valid) d = (kSid ? uint32_t(sys_of[v[it]] >> shift) : uint32_t(k[it] >> shift)) & (kRsBins - 1);
-        const uint32_t peers = __match_any_sync(0xffffffffu, valid ? d : uint32_t(kRsBins + lane));
-        const int leader = __ffs(peers) - 1;
-        uint32_t old = 0;
-        if (valid && lane == leader) old = s_w[warp][d];
-        old = __shfl_sync(0xffffffffu, old, leader);
-        rk[it] = old + __popc(peers & lt);
-        dig[it] = d;
-        if (valid && lane == leader) s_w[warp][d] = old + __popc(peers);
-        __syncwarp();
-    }
-}
-
-// One stable pass over the tile the block takes. status: [tile][digit] words of this pass.
-template <bool kSid, int kItems>
-__global__ __launch_bounds__(kRsThreads) void k_os_pass(const uint64_t *__restrict__ kin,
-                                                        const int32_t *__restrict__ vin, uint64_t *__restrict__ kout,
-                                                        int32_t *__restrict__ vout, const uint16_t *__restrict__ sys_of,
-                                                        DevInfo *info, int shift, const uint32_t *__restrict__ ghist,
-                                                        uint32_t *ctr, uint32_t *status) {
-    __shared__ uint32_t s_goff[kRsBins];
-    __shared__ uint32_t s_w[kRsWarps][kRsBins];
-    __shared__ uint32_t s_warp[kScanThreads / 32 + 1];
-    __shared__ uint32_t s_tile;
-    static_assert(kRsThreads == kScanThreads && kRsThreads == kRsBins, "one thread per digit");
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) s_tile = atomicAdd(ctr, 1u);
-    // where each digit starts in the output: exclusive scan of the pass's histogram
-    uint32_t total;
-    const uint32_t gstart = block_excl_scan(ghist[tid], s_warp, total);  // its barriers publish s_tile too
-    const uint32_t tile = s_tile;
-    const int64_t n = info->nstars;
-    const int64_t base = int64_t(tile) * (kItems * kRsThreads);
-    if (base >= n) return;  // uniform over the block
-    uint64_t k[kItems];
-    int32_t v[kItems];
-    uint32_t dig[kItems], rk[kItems];
-    rank_tile<kSid, kItems>(kin, vin, sys_of, shift, base, n, s_w, k, v, dig, rk);
-    __syncthreads();
-    // digit tid: each warp's start inside the tile, and the tile's count
-    uint32_t run = 0;
-#pragma unroll
-    for (int w = 0; w < kRsWarps; ++w) {
-        const uint32_t c = s_w[w][tid];
-        s_w[w][tid] = run;
-        run += c;
-    }
-    // look-back for digit tid: this tile's count is run. Predecessors' words are read kOsWindow
-    // at a time (independent loads), then taken in order back to the first prefix.
-    const uint32_t agg = run;
-    uint32_t *mine = status + size_t(tile) * kRsBins + tid;
-    uint32_t excl = 0;
-    if (tile == 0) {
-        st_volatile(mine, kOsPre | agg);
-    } else {
-        st_volatile(mine, kOsAgg | agg);
-        int64_t t = int64_t(tile) - 1;
-        int spins = 0;
-        bool done = false, bad = false;
-        while (!done && !bad) {
-            uint32_t w[kOsWindow];
-#pragma unroll
-            for (int j = 0; j < kOsWindow; ++j)  // before tile 0: a prefix of 0
-                w[j] = t - j >= 0 ? ld_volatile(status + size_t(t - j) * kRsBins + tid) : kOsPre;
-#pragma unroll
-            for (int j = 0; j < kOsWindow; ++j) {
-                if (done || bad) continue;
-                while (!(w[j] >> 30)) {  // not published yet: wait for this word
-                    if (++spins > kOsSpinLimit) {
-                        bad = true;
-                        break;
-                    }
-                    w[j] = ld_volatile(status + size_t(t - j) * kRsBins + tid);
-                }
-                if (bad) continue;
-                excl += w[j] & kOsCount;
-                done = (w[j] >> 30) == (kOsPre >> 30);
-            }
-            t -= kOsWindow;
-        }
-        if (bad) dev_error(info, kErrSortWait);
-        st_volatile(mine, kOsPre | ((excl + agg) & kOsCount));
-    }
-    s_goff[tid] = gstart + excl;
-    __syncthreads();
-    const int64_t wbase = base + int64_t(warp) * (kItems * 32);
-#pragma unroll
-    for (int it = 0; it < kItems; ++it) {
-        if (wbase + it * 32 + lane < n) {
-            const uint32_t pos = s_goff[dig[it]] + s_w[warp][dig[it]] + rk[it];
-            if (pos < n) {
-                kout[pos] = k[it];
-                vout[pos] = v[it];
-            } else {
-                dev_error(info, 10);
-            }
-        }
-    }
-}
-
-// ---------------------------------------------------------------- sorted copies
-
-// build.go:34-41 with SourceMass (sim.go:93-98); FP32 hi/lo split for the walks. Each star's
-// position and mass come from its 32-byte record written by the collect kernel: one sector read
-// through the sort order instead of one sector per array.
-__global__ __launch_bounds__(kThreads) void k_gather(const DevInfo *info, const int32_t *__restrict__ order,
-                                                     const Pos4 *__restrict__ pos4,
-                                                     const uint8_t *__restrict__ kind, int dm_off, int fp64_copies,
-                                                     double *__restrict__ sx, double *__restrict__ sy,
-                                                     double *__restrict__ sz, double *__restrict__ sm,
-                                                     float4 *__restrict__ st_hi, float4 *__restrict__ st_lo,
-                                                     const uint16_t *__restrict__ sys_of,
-                                                     int32_t *__restrict__ sid_sorted) {
-    int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k >= info->nstars) return;
-    int32_t i = order[k];
-    if (sys_of) sid_sorted[k] = sys_of[i];
-    const Pos4 p = pos4[i];
-    const double x = p.x, y = p.y, z = p.z;
-    double m = p.m;
-    if (dm_off && kind && kind[i] == GBH_DARK_MATTER) m = 0;
-    if (fp64_copies) {  // read by the FP64 upsweep, walk and potential only
-        sx[k] = x;
-        sy[k] = y;
-        sz[k] = z;
-        sm[k] = m;
-    }
-    float hx = __double2float_rn(x), hy = __double2float_rn(y), hz = __double2float_rn(z);
-    st_hi[k] = make_float4(hx, hy, hz, __double2float_rn(m));
-    st_lo[k] = make_float4(__double2float_rn(x - double(hx)), __double2float_rn(y - double(hy)),
-                           __double2float_rn(z - double(hz)), 0.f);
 }
 
 // ---------------------------------------------------------------- node set (chains)
@@ -1688,178 +1048,23 @@ __global__ void k_potential_final(int64_t nparts, const double *part, const DevI
     if (threadIdx.x == 0) *u = -s[0] / 2;
 }
 
-constexpr int kFlagBlocksMax = 1024;
-
 }  // namespace
 
 // ---------------------------------------------------------------- forests (many systems)
 
 namespace {
 
-__global__ void k_sys_init(int32_t nsys, SysGeo *geo, DevInfo *info) {
-    int32_t s = int32_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (s == 0) {  // cleared before k_sys_final may report a non-finite system
-        info->err = 0;
-        info->err_where = 0;
-    }
-    if (s >= nsys) return;
-    for (int c = 0; c < 3; ++c) {
-        geo[s].kmin[c] = LLONG_MAX;
-        geo[s].kmax[c] = LLONG_MIN;
-    }
-}
-
-// Star flags, alive holes' accelerations zeroed, and each system's bbox (ordered keys, one
-// warp-wide atomic per quantity when the warp's stars share a system).
-__global__ __launch_bounds__(kThreads) void k_flags_sys(int64_t n, const double *__restrict__ px,
-                                                        const double *__restrict__ py, const double *__restrict__ pz,
-                                                        const double *__restrict__ mass,
-                                                        const uint8_t *__restrict__ kind,
-                                                        const uint8_t *__restrict__ alive,
-                                                        const uint16_t *__restrict__ sys_of, uint32_t *__restrict__ flag,
-                                                        SysGeo *geo, double *ax, double *ay, double *az,
-                                                        Pos4 *__restrict__ pos4) {
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    bool st = false;
-    int s = -1;
-    long long k[3] = {LLONG_MAX, LLONG_MAX, LLONG_MAX};
-    if (i < n) {
-        uint8_t al = alive ? alive[i] : 1, kd = kind ? kind[i] : 0;
-        st = is_star(al, kd);
-        flag[i] = st;
-        if (st) {
-            s = sys_of[i];
-            const double vx = px[i], vy = py[i], vz = pz[i], m = mass ? mass[i] : 0.0;
-            pos4[i] = Pos4{vx, vy, vz, m};
-            k[0] = mass && !isfinite(m) ? LLONG_MAX : ord_key(vx);  // as in k_flags_bbox
-            k[1] = ord_key(vy);
-            k[2] = ord_key(vz);
-        } else if (al && kd == GBH_BLACK_HOLE) {
-            ax[i] = 0;
-            ay[i] = 0;
-            az[i] = 0;
-        }
-    }
-    unsigned m = __match_any_sync(0xffffffffu, s);
-    int lane = threadIdx.x & 31;
-    bool uniform = m == 0xffffffffu;
-    if (uniform) {
-        if (s < 0) return;
-        long long mn[3] = {k[0], k[1], k[2]}, mx[3] = {k[0], k[1], k[2]};
-        for (int c = 0; c < 3; ++c)
-            for (int o = 16; o > 0; o >>= 1) {
-                mn[c] = min(mn[c], __shfl_xor_sync(0xffffffffu, mn[c], o));
-                mx[c] = max(mx[c], __shfl_xor_sync(0xffffffffu, mx[c], o));
-            }
-        if (lane == 0)
-            for (int c = 0; c < 3; ++c) {
-                atomicMin(&geo[s].kmin[c], mn[c]);
-                atomicMax(&geo[s].kmax[c], mx[c]);
-            }
-    } else if (s >= 0) {
-        for (int c = 0; c < 3; ++c) {
-            atomicMin(&geo[s].kmin[c], k[c]);
-            atomicMax(&geo[s].kmax[c], k[c]);
-        }
-    }
-}
-
-// Per system: root cube (build.go:19-21), FP32 views, opening bases, sorted star range.
-// Thread 0 also resets the per-build scalars.
-__global__ void k_sys_final(int32_t nsys, int64_t n, const int64_t *__restrict__ sys_off,
-                            const uint32_t *__restrict__ scan, const uint8_t *kind, const uint8_t *alive, double theta,
-                            SysGeo *geo, DevInfo *info) {
-    int32_t s = int32_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    int64_t total = n > 0 ? int64_t(scan[n - 1]) + (is_star(alive ? alive[n - 1] : 1, kind ? kind[n - 1] : 0) ? 1 : 0)
-                          : 0;
-    if (s == 0) {
-        info->theta = theta;
-        info->nstars = total;
-        info->nnodes = 0;
-        info->work = 0;
-        info->nleaves = 0;
-    }
-    if (s >= nsys) return;
-    SysGeo &g = geo[s];
-    double mn[3], mx[3];
-    for (int c = 0; c < 3; ++c) {
-        mn[c] = ord_val(g.kmin[c]);
-        mx[c] = ord_val(g.kmax[c]);
-    }
-
-    double side = fmax(mx[0] - mn[0], fmax(mx[1] - mn[1], mx[2] - mn[2]));
-    side = fmax(side * (1 + 1e-9), 1e-12);
-    g.minx = mn[0];
-    g.miny = mn[1];
-    g.minz = mn[2];
-    g.side = side;
-    g.scale = double(1 << kMortonBits) / side;
-    for (int c = 0; c < 3; ++c) {
-        float h = __double2float_rn(mn[c]);
-        g.min_hi[c] = h;
-        g.min_lo[c] = __double2float_rn(mn[c] - double(h));
-    }
-    float sh = __double2float_rn(side);
-    g.side_hi = sh;
-    g.side_lo = __double2float_rn(side - double(sh));
-    double half = side / 2;
-    for (int L = 0; L <= kMaxLevel; ++L, half = half / 2) g.crit_base[L] = __double2float_rn(2 * half / theta);
-    int64_t a = sys_off[s], b = sys_off[s + 1];
-    g.star_lo = int32_t(a < n ? int64_t(scan[a]) : total);
-    g.star_hi = int32_t(b < n ? int64_t(scan[b]) : total);
-    // an empty system keeps its initial keys (a NaN box); a system with stars must be finite
-    if (g.star_hi > g.star_lo && !(isfinite(mn[0]) && isfinite(mn[1]) && isfinite(mn[2]) && isfinite(mx[0]) &&
-                                   isfinite(mx[1]) && isfinite(mx[2])))
-        dev_error(info, kErrNonFinite);
-}
-
-// Each star's Morton key in its own system's cube (build.go:19-31).
-__global__ __launch_bounds__(kThreads) void k_compact_keys_sys(int64_t n, const double *__restrict__ px,
-                                                               const double *__restrict__ py,
-                                                               const double *__restrict__ pz,
-                                                               const uint8_t *__restrict__ kind,
-                                                               const uint8_t *__restrict__ alive,
-                                                               const uint16_t *__restrict__ sys_of,
-                                                               const uint32_t *__restrict__ scan,
-                                                               const SysGeo *__restrict__ geo,
-                                                               uint64_t *__restrict__ keys, int32_t *__restrict__ order) {
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (!is_star(alive ? alive[i] : 1, kind ? kind[i] : 0)) return;
-    const SysGeo &g = geo[sys_of[i]];
-    double sc = g.scale;
-    uint64_t k = spread(cell(px[i], g.minx, sc)) << 2 | spread(cell(py[i], g.miny, sc)) << 1 |
-                 spread(cell(pz[i], g.minz, sc));
-    uint32_t pos = scan[i];
-    keys[pos] = k;
-    order[pos] = int32_t(i);
-}
-
-// Roots (the pre-order index of a system's first star chain) and the gsize-star groups of the
-// mixed walk, which never straddle two systems.
-__global__ void k_sys_layout(int32_t nsys, int32_t gsize, const uint32_t *__restrict__ base, SysGeo *geo,
-                             DevInfo *info) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    int32_t groups = 0;
-    for (int32_t s = 0; s < nsys; ++s) {
-        SysGeo &g = geo[s];
-        int32_t cnt = g.star_hi - g.star_lo;
-        g.root = cnt > 0 ? int32_t(base[g.star_lo]) : -1;
-        g.group_lo = groups;
-        g.ngroups = (cnt + gsize - 1) / gsize;
-        groups += g.ngroups;
-    }
-    info->ngroups = uint32_t(groups);
-}
-
-__global__ void k_sys_groups(int32_t nsys, int32_t gsize, const SysGeo *__restrict__ geo, int4 *__restrict__ groups) {
-    int32_t s = int32_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (s >= nsys) return;
-    const SysGeo &g = geo[s];
-    for (int32_t q = 0; q < g.ngroups; ++q) {
-        int32_t start = g.star_lo + gsize * q;
-        int32_t cnt = g.star_hi - start < gsize ? g.star_hi - start : gsize;
-        groups[g.group_lo + q] = make_int4(start, cnt, g.root, 0);
+// Each system's root (the pre-order index of its first star's chain) and its entries of the
+// mixed walk's group table; a block a system.
+__global__ __launch_bounds__(128) void k_sys_groups(int32_t gsize, const uint32_t *__restrict__ base, SysGeo *geo,
+                                                    int4 *__restrict__ groups) {
+    SysGeo &g = geo[blockIdx.x];
+    const int32_t lo = g.star_lo, hi = g.star_hi, glo = g.group_lo, ng = g.ngroups;
+    const int32_t root = hi > lo ? int32_t(base[lo]) : -1;
+    if (threadIdx.x == 0) g.root = root;
+    for (int32_t q = threadIdx.x; q < ng; q += blockDim.x) {
+        const int32_t start = lo + gsize * q;
+        groups[glo + q] = make_int4(start, hi - start < gsize ? hi - start : gsize, root, 0);
     }
 }
 
@@ -1881,7 +1086,7 @@ static cudaError_t scan_dyn(const Launch &L, const uint32_t *in, uint32_t *out, 
 }
 
 void tree_free(TreeBufs &b) {
-    void *ptrs[] = {b.flag, b.pos4, b.bbox_part, b.keys, b.keys_alt, b.order, b.order_alt, b.hist, b.os_state, b.hs_state, b.sx, b.sy, b.sz, b.sm,
+    void *ptrs[] = {b.flag, b.pos4, b.bbox_part, b.keys, b.keys_alt, b.order, b.order_alt, b.lb_state, b.tile_len, b.hist, b.sx, b.sy, b.sz, b.sm,
                     b.st_hi, b.st_lo, b.st_off, b.chain_cnt, b.leaves, b.targets, b.geo, b.sid_sorted, b.groups, b.gcost, b.gperm, b.pre_parent, b.pre_info, b.pre_nchild, b.pre_mask, b.pre_ref, b.pre_star, b.nodes,
                     b.n_parent, b.n_info, b.n_arrive, b.pnodes, b.mnodes, b.mrange, b.lnode, b.walk_ctr, b.scan_tmp, b.info, b.part_acc};
     for (void *p : ptrs)
@@ -1908,10 +1113,7 @@ cudaError_t tree_alloc(TreeBufs &b, int64_t n, int leaf, int32_t nsys) {
     tree_free(b);
     b.generation = gen;
     cn = cn < 1 ? 1 : cn;
-    int64_t rs_tiles = (cn + kRsTile - 1) / kRsTile;
     int64_t scan_cap = scan_tmp_size(cnodes > cn * 1 ? cnodes : cn);
-    int64_t scan_cap2 = scan_tmp_size(rs_tiles * kRsBins);
-    if (scan_cap2 > scan_cap) scan_cap = scan_cap2;
     b.scan_tmp_cap = scan_cap;
     cudaError_t e = cudaSuccess;
 #define GBH_ALLOC(ptr, count)                                                     \
@@ -1920,12 +1122,11 @@ cudaError_t tree_alloc(TreeBufs &b, int64_t n, int leaf, int32_t nsys) {
     } while (0)
     GBH_ALLOC(b.flag, cn);
     GBH_ALLOC(b.pos4, cn);
-    GBH_ALLOC(b.bbox_part, kFlagBlocksMax * 6);
+    if (e == cudaSuccess) e = dev_alloc(&b.bbox_part, sort_part_bytes());
     GBH_ALLOC(b.keys, cn);
     GBH_ALLOC(b.keys_alt, cn);
     GBH_ALLOC(b.order, cn);
     GBH_ALLOC(b.order_alt, cn);
-    GBH_ALLOC(b.hist, rs_tiles * kRsBins);
     GBH_ALLOC(b.sx, cn);
     GBH_ALLOC(b.sy, cn);
     GBH_ALLOC(b.sz, cn);
@@ -1959,19 +1160,13 @@ cudaError_t tree_alloc(TreeBufs &b, int64_t n, int leaf, int32_t nsys) {
     GBH_ALLOC(b.lnode, cnodes);
     GBH_ALLOC(b.walk_ctr, 16);
     GBH_ALLOC(b.scan_tmp, scan_cap);
-    // single-pass scans of larger states: the digit tables of the three-launch passes (10 with a
-    // forest's system digits) and the build's three other scans, each 2 words of counter and the
-    // 64-bit look-back words of its tiles
-    const int64_t hs_words = kOsPassesMax * (2 + 2 * os_scan_tiles(rs_tiles * kRsBins)) +
-                             kOsScans * (2 + 2 * os_scan_tiles(cn > cnodes ? cn : cnodes));
-    GBH_ALLOC(b.hs_state, hs_words);
-    int64_t os_words = 0;
-    if (cn <= kOsMaxN) {  // node capacity stays below 2^30 too (at most 12 nodes a body)
-        const int64_t stiles = os_scan_tiles(cn > cnodes ? cn : cnodes);
-        os_words = kOsHistWords + kOsCtrWords + 2 * kOsScans * stiles +
-                   kOsPassesMax * os_sort_tiles(cn, os_items(cn)) * kRsBins;
-        GBH_ALLOC(b.os_state, os_words);
-    }
+    // single-pass scans: the chain counts' and the child counts', and the large sort's
+    b.lb_sort = kLbScans * lb_words_of(lb_tiles(cn > cnodes ? cn : cnodes));
+    const int64_t lb_words = b.lb_sort + sort_lb_words(cn);
+    GBH_ALLOC(b.lb_state, lb_words);
+    const int64_t ctiles = cn / kSortTile + csys + 1;  // sort tiles never straddle systems
+    GBH_ALLOC(b.tile_len, 2 * ctiles);
+    GBH_ALLOC(b.hist, sort_hist_words(cn));
     GBH_ALLOC(b.info, 1);
 #undef GBH_ALLOC
     if (e != cudaSuccess) {
@@ -1980,8 +1175,8 @@ cudaError_t tree_alloc(TreeBufs &b, int64_t n, int leaf, int32_t nsys) {
     }
     b.cap_n = cn;
     b.cap_nodes = cnodes;
-    b.os_words = os_words;
-    b.hs_words = hs_words;
+    b.lb_words = lb_words;
+    b.cap_tiles = ctiles;
     b.cap_sys = csys;
     b.cap_groups = cgroups;
     b.nsys = nsys;
@@ -1998,182 +1193,36 @@ cudaError_t tree_alloc(TreeBufs &b, int64_t n, int leaf, int32_t nsys) {
         if (e_ != cudaSuccess) return e_;          \
     } while (0)
 
-// Word offset of the sort's look-back words in os_state (after the histograms, the counters and
-// the scans' 64-bit words).
-static int64_t os_scan_cap(const TreeBufs &b) { return os_scan_tiles(b.cap_n > b.cap_nodes ? b.cap_n : b.cap_nodes); }
-static int64_t os_sort_base(const TreeBufs &b) { return kOsHistWords + kOsCtrWords + 2 * kOsScans * os_scan_cap(b); }
-
-// Single-pass exclusive scan `which` (0 flags, 1 chain counts, 2 child counts) of a build.
+// Single-pass exclusive scan `which` (0 chain counts, 1 child counts) of a build.
 static cudaError_t scan_lb(const Launch &L, TreeBufs &b, int which, const uint32_t *in, uint32_t *out, int64_t n,
                            const int64_t *ndyn) {
-    const int64_t tiles = os_scan_tiles(n);
+    const int64_t tiles = lb_tiles(n);
     if (tiles < 1) return cudaSuccess;
-    uint32_t *ctr = b.os_state + kOsHistWords + kOsScanCtr + which;
-    unsigned long long *st =
-        reinterpret_cast<unsigned long long *>(b.os_state + kOsHistWords + kOsCtrWords) + which * os_scan_cap(b);
-    k_scan_lb<<<unsigned(tiles), kScanThreads, 0, L.stream>>>(in, out, n, ndyn, ctr, st, b.info);
-    ++*L.count;
-    return cudaGetLastError();
-}
-
-// Single-pass scans of larger states (hs_state), in place of the three-launch scans: pass p's
-// digit table (rs_tiles x 256 entries: at 1M bodies 81 tiles, a look-back of three round trips),
-// and scan `which` (0 flags, 1 chain counts, 2 child counts) of n entries.
-static cudaError_t scan_hs(const Launch &L, TreeBufs &b, uint32_t *base, const uint32_t *in, uint32_t *out, int64_t n,
-                           const int64_t *ndyn) {
-    const int64_t tiles = os_scan_tiles(n);
-    if (tiles < 1) return cudaSuccess;
+    uint32_t *base = b.lb_state + int64_t(which) * lb_words_of(lb_tiles(b.cap_n > b.cap_nodes ? b.cap_n : b.cap_nodes));
     k_scan_lb<<<unsigned(tiles), kScanThreads, 0, L.stream>>>(in, out, n, ndyn, base,
                                                               reinterpret_cast<unsigned long long *>(base + 2), b.info);
     ++*L.count;
     return cudaGetLastError();
 }
-static int64_t hs_pass_words(const TreeBufs &b) { return 2 + 2 * os_scan_tiles(rs_sort_tiles(b.cap_n) * kRsBins); }
-static cudaError_t scan_hist(const Launch &L, TreeBufs &b, int p, uint32_t ntiles) {
-    return scan_hs(L, b, b.hs_state + int64_t(p) * hs_pass_words(b), b.hist, b.hist, int64_t(ntiles) * kRsBins,
-                   nullptr);
-}
-static cudaError_t scan_big(const Launch &L, TreeBufs &b, int which, const uint32_t *in, uint32_t *out, int64_t n,
-                            const int64_t *ndyn) {
-    const int64_t stiles = os_scan_tiles(b.cap_n > b.cap_nodes ? b.cap_n : b.cap_nodes);
-    uint32_t *base = b.hs_state + kOsPassesMax * hs_pass_words(b) + int64_t(which) * (2 + 2 * stiles);
-    return scan_hs(L, b, base, in, out, n, ndyn);
-}
 
 cudaError_t tree_build(const Launch &L, TreeBufs &b, int64_t n, const double *px, const double *py, const double *pz,
                        const double *mass, const uint8_t *kind, const uint8_t *alive, double *ax, double *ay,
                        double *az, double theta, int leaf, int dm_off, bool exact, bool plain_records,
-                       const uint16_t *sys_of, const int64_t *sys_off) {
+                       const ForestTiles *forest_tiles) {
     cudaStream_t s = L.stream;
     const int64_t cap = b.cap_n;
     const bool forest = b.nsys > 1;
-    if (forest && (!sys_of || !sys_off)) return cudaErrorInvalidValue;
-    cudaError_t e;
-    // one-sweep sort and single-pass scans (capacity up to kOsMaxN bodies): histograms, tile
-    // counters and the look-back words of the passes this tree build runs start at zero
-    const bool os = b.os_state != nullptr;
-    // a forest then sorts stably by system id, one pass per byte: up to 256 systems the high
-    // byte is 0 everywhere, and that pass (a stable pass over equal digits) is left out
-    const int sid_passes = forest ? (b.nsys > 256 ? 2 : 1) : 0;
-    const int npass = 8 + sid_passes;
-    // the passes ping-pong between the two buffers and end in keys / order: with an odd count
-    // the keys are formed in the other pair
-    uint64_t *const keys0 = (npass & 1) ? b.keys_alt : b.keys;
-    int32_t *const order0 = (npass & 1) ? b.order_alt : b.order;
-    const int os_k = os_items(cap);  // keys a thread of a one-sweep pass ranks
-    const int64_t os_tiles = os_sort_tiles(cap, os_k);
-    if (os) {
-        const int64_t words = os_sort_base(b) + int64_t(npass) * os_tiles * kRsBins;
-        if ((e = cudaMemsetAsync(b.os_state, 0, sizeof(uint32_t) * size_t(words), s)) != cudaSuccess) return e;
-    } else if ((e = cudaMemsetAsync(b.hs_state, 0, sizeof(uint32_t) * size_t(b.hs_words), s)) != cudaSuccess) {
-        return e;
-    }
-    if (!forest) {
-        // collect + bbox (build.go:62-113)
-        unsigned fb = blocks_for(n, kThreads);
-        if (fb > unsigned(kFlagBlocksMax)) fb = kFlagBlocksMax;
-        k_flags_bbox<<<fb, kThreads, 0, s>>>(n, px, py, pz, mass, kind, alive, b.flag, b.bbox_part, ax, ay, az,
-                                             b.info, b.pos4);
-        GBH_LAUNCH_CHECK();
-        e = os ? scan_lb(L, b, 0, b.flag, b.flag, n, nullptr) : scan_big(L, b, 0, b.flag, b.flag, n, nullptr);
-        if (e != cudaSuccess) return e;
-        k_bbox_final<<<1, kFinalThreads, 0, s>>>(int(fb), b.bbox_part, n, b.flag, kind, alive, theta, b.info, b.geo);
-        GBH_LAUNCH_CHECK();
-        k_compact_keys<<<blocks_for(n, kThreads), kThreads, 0, s>>>(n, px, py, pz, kind, alive, b.flag, b.info, keys0,
-                                                                    order0);
-        GBH_LAUNCH_CHECK();
-    } else {
-        // collect per system: each system gets its own root cube and keys (build.go:11-31)
-        const unsigned sb = blocks_for(b.nsys, 128);
-        k_sys_init<<<sb, 128, 0, s>>>(b.nsys, b.geo, b.info);
-        GBH_LAUNCH_CHECK();
-        k_flags_sys<<<blocks_for(n, kThreads), kThreads, 0, s>>>(n, px, py, pz, mass, kind, alive, sys_of, b.flag,
-                                                                 b.geo, ax, ay, az, b.pos4);
-        GBH_LAUNCH_CHECK();
-        e = os ? scan_lb(L, b, 0, b.flag, b.flag, n, nullptr) : scan_big(L, b, 0, b.flag, b.flag, n, nullptr);
-        if (e != cudaSuccess) return e;
-        k_sys_final<<<sb, 128, 0, s>>>(b.nsys, n, sys_off, b.flag, kind, alive, theta, b.geo, b.info);
-        GBH_LAUNCH_CHECK();
-        k_compact_keys_sys<<<blocks_for(n, kThreads), kThreads, 0, s>>>(n, px, py, pz, kind, alive, sys_of, b.flag,
-                                                                        b.geo, keys0, order0);
-        GBH_LAUNCH_CHECK();
-    }
-    // radix sort (morton.go:25-49): 8 stable passes, ping-pong, result back in keys/order
-    const uint32_t ntiles = uint32_t((cap + kRsTile - 1) / kRsTile);
-    uint64_t *kin = keys0, *kout = keys0 == b.keys ? b.keys_alt : b.keys;
-    int32_t *vin = order0, *vout = order0 == b.order ? b.order_alt : b.order;
-    if (os) {
-        // forest: then stably by system, (system, key) order, each system's stars contiguous
-        uint32_t *ghist = b.os_state, *ctr = b.os_state + kOsHistWords;
-        unsigned hb = unsigned(L.num_sms > 0 ? L.num_sms : 152) * kOsHistBlocksPerSm;
-        if (int64_t(hb) * kRsThreads > cap) hb = blocks_for(cap, kRsThreads);
-        if (forest) k_os_hist<true><<<hb, kRsThreads, 0, s>>>(kin, vin, sys_of, b.info, ghist);
-        else k_os_hist<false><<<hb, kRsThreads, 0, s>>>(kin, vin, nullptr, b.info, ghist);
-        GBH_LAUNCH_CHECK();
-        for (int p = 0; p < npass; ++p) {
-            uint32_t *st = b.os_state + os_sort_base(b) + int64_t(p) * os_tiles * kRsBins;
-            const uint16_t *so = p < 8 ? nullptr : sys_of;
-            const int shift = p < 8 ? 8 * p : 8 * (p - 8);
-            const unsigned g = unsigned(os_tiles);
-            const uint32_t *gh = ghist + p * kRsBins;
-            if (p < 8) {
-                if (os_k == 4) k_os_pass<false, 4><<<g, kRsThreads, 0, s>>>(kin, vin, kout, vout, so, b.info, shift, gh, ctr + p, st);
-                else if (os_k == 8) k_os_pass<false, 8><<<g, kRsThreads, 0, s>>>(kin, vin, kout, vout, so, b.info, shift, gh, ctr + p, st);
-                else k_os_pass<false, 12><<<g, kRsThreads, 0, s>>>(kin, vin, kout, vout, so, b.info, shift, gh, ctr + p, st);
-            } else {
-                if (os_k == 4) k_os_pass<true, 4><<<g, kRsThreads, 0, s>>>(kin, vin, kout, vout, so, b.info, shift, gh, ctr + p, st);
-                else if (os_k == 8) k_os_pass<true, 8><<<g, kRsThreads, 0, s>>>(kin, vin, kout, vout, so, b.info, shift, gh, ctr + p, st);
-                else k_os_pass<true, 12><<<g, kRsThreads, 0, s>>>(kin, vin, kout, vout, so, b.info, shift, gh, ctr + p, st);
-            }
-            GBH_LAUNCH_CHECK();
-            uint64_t *tk = kin;
-            kin = kout;
-            kout = tk;
-            int32_t *tv = vin;
-            vin = vout;
-            vout = tv;
-        }
-    }
-    for (int shift = 0; shift < 64 && !os; shift += 8) {
-        k_rs_hist<false><<<ntiles, kRsThreads, 0, s>>>(kin, vin, nullptr, b.info, shift, ntiles, b.hist);
-        GBH_LAUNCH_CHECK();
-        if ((e = scan_hist(L, b, shift / 8, ntiles)) != cudaSuccess) return e;
-        k_rs_scatter<false><<<ntiles, kRsThreads, 0, s>>>(kin, vin, kout, vout, nullptr, b.info, shift, ntiles, b.hist);
-        GBH_LAUNCH_CHECK();
-        uint64_t *tk = kin;
-        kin = kout;
-        kout = tk;
-        int32_t *tv = vin;
-        vin = vout;
-        vout = tv;
-    }
-    if (forest && !os) {  // then stably by system: (system, key) order, each system's stars contiguous
-        for (int shift = 0; shift < 8 * sid_passes; shift += 8) {
-            k_rs_hist<true><<<ntiles, kRsThreads, 0, s>>>(kin, vin, sys_of, b.info, shift, ntiles, b.hist);
-            GBH_LAUNCH_CHECK();
-            if ((e = scan_hist(L, b, 8 + shift / 8, ntiles)) != cudaSuccess) return e;
-            k_rs_scatter<true><<<ntiles, kRsThreads, 0, s>>>(kin, vin, kout, vout, sys_of, b.info, shift, ntiles,
-                                                             b.hist);
-            GBH_LAUNCH_CHECK();
-            uint64_t *tk = kin;
-            kin = kout;
-            kout = tk;
-            int32_t *tv = vin;
-            vin = vout;
-            vout = tv;
-        }
-    }
-    // sorted copies (build.go:34-41)
+    if (forest && !forest_tiles) return cudaErrorInvalidValue;
+    cudaError_t e = sort_stars(L, b, n, px, py, pz, mass, kind, alive, ax, ay, az, theta, dm_off, exact,
+                               forest ? forest_tiles : nullptr);
+    if (e != cudaSuccess) return e;
     const unsigned nb = blocks_for(cap, kThreads);
-    k_gather<<<nb, kThreads, 0, s>>>(b.info, b.order, b.pos4, kind, dm_off, exact ? 1 : 0, b.sx, b.sy, b.sz,
-                                     b.sm, b.st_hi, b.st_lo, forest ? sys_of : nullptr, b.sid_sorted);
-    GBH_LAUNCH_CHECK();
     // node set
     uint32_t *cnt = b.chain_cnt, *base = b.chain_cnt + cap;
     const int32_t *sid = forest ? b.sid_sorted : nullptr;
     k_chain_count<<<nb, kThreads, 0, s>>>(b.keys, b.info, sid, b.geo, leaf, cnt);
     GBH_LAUNCH_CHECK();
-    e = os ? scan_lb(L, b, 1, cnt, base, cap, &b.info->nstars) : scan_big(L, b, 1, cnt, base, cap, &b.info->nstars);
+    e = scan_lb(L, b, 0, cnt, base, cap, &b.info->nstars);
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync(b.pre_mask, 0, sizeof(uint32_t) * size_t(b.cap_nodes), s);
     if (e == cudaSuccess) e = cudaMemsetAsync(b.pre_nchild, 0, sizeof(uint32_t) * size_t(b.cap_nodes), s);
@@ -2181,8 +1230,7 @@ cudaError_t tree_build(const Launch &L, TreeBufs &b, int64_t n, const double *px
     k_chain_emit<<<nb, kThreads, 0, s>>>(b.keys, b.info, cnt, base, b.pre_parent, b.pre_info, b.pre_nchild, b.pre_mask,
                                          b.pre_star, b.leaves, sid, b.geo);
     GBH_LAUNCH_CHECK();
-    e = os ? scan_lb(L, b, 2, b.pre_nchild, b.pre_nchild, b.cap_nodes, &b.info->nnodes)
-           : scan_big(L, b, 2, b.pre_nchild, b.pre_nchild, b.cap_nodes, &b.info->nnodes);
+    e = scan_lb(L, b, 1, b.pre_nchild, b.pre_nchild, b.cap_nodes, &b.info->nnodes);
     if (e != cudaSuccess) return e;
     const unsigned nbn = node_blocks(b.cap_nodes);
     k_ref_index<<<nbn, kThreads, 0, s>>>(b.info, base, b.pre_star, b.pre_parent, b.pre_info, b.pre_mask, b.pre_nchild,
@@ -2193,9 +1241,7 @@ cudaError_t tree_build(const Launch &L, TreeBufs &b, int64_t n, const double *px
                                           b.geo, b.cap_nodes);
     GBH_LAUNCH_CHECK();
     if (forest) {
-        k_sys_layout<<<1, 32, 0, s>>>(b.nsys, b.group == 32 ? 32 : 64, base, b.geo, b.info);
-        GBH_LAUNCH_CHECK();
-        k_sys_groups<<<blocks_for(b.nsys, 128), 128, 0, s>>>(b.nsys, b.group == 32 ? 32 : 64, b.geo, b.groups);
+        k_sys_groups<<<unsigned(b.nsys), 128, 0, s>>>(b.group == 32 ? 32 : 64, base, b.geo, b.groups);
         GBH_LAUNCH_CHECK();
     }
     b.moments_exact = exact;
@@ -2390,111 +1436,11 @@ cudaError_t potential_fp64(const Launch &L, const TreeBufs &b, int64_t n, const 
 
 namespace gbh {
 
-// ---------------------------------------------------------------- Morton order into caller-owned scratch
-
-namespace {
-inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
-
-// Star flags and per-block bbox partials, as k_flags_bbox but writing no accelerations.
-__global__ __launch_bounds__(kThreads) void k_flags_bbox_noacc(int64_t n, const double *__restrict__ px,
-                                                               const double *__restrict__ py,
-                                                               const double *__restrict__ pz,
-                                                               const uint8_t *__restrict__ kind,
-                                                               const uint8_t *__restrict__ alive,
-                                                               uint32_t *__restrict__ flag, double *__restrict__ part) {
-    long long mn[3] = {LLONG_MAX, LLONG_MAX, LLONG_MAX}, mx[3] = {LLONG_MIN, LLONG_MIN, LLONG_MIN};
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-        bool st = is_star(alive ? alive[i] : 1, kind ? kind[i] : 0);
-        flag[i] = st;
-        if (st) {
-            long long x = ord_key(px[i]), y = ord_key(py[i]), z = ord_key(pz[i]);
-            mn[0] = min(mn[0], x);
-            mx[0] = max(mx[0], x);
-            mn[1] = min(mn[1], y);
-            mx[1] = max(mx[1], y);
-            mn[2] = min(mn[2], z);
-            mx[2] = max(mx[2], z);
-        }
-    }
-    block_minmax<kThreads>(mn, mx, part);
-}
-}  // namespace
-
-size_t morton_sort_scratch_bytes(int64_t nmax) {
-    int64_t tiles = (nmax + kRsTile - 1) / kRsTile;
-    size_t b = align256(sizeof(DevInfo));
-    b += align256(sizeof(double) * kFlagBlocksMax * 6);
-    b += align256(sizeof(uint32_t) * size_t(nmax));
-    b += align256(sizeof(uint64_t) * size_t(nmax));
-    b += align256(sizeof(int32_t) * size_t(nmax));
-    b += align256(sizeof(uint32_t) * size_t(tiles) * kRsBins);
-    b += align256(sizeof(uint32_t) * size_t(scan_tmp_size(nmax > tiles * kRsBins ? nmax : tiles * kRsBins)));
-    return b;
-}
-
-// The collect, key and stable-sort stages of tree_build (the same kernels), with every
-// temporary carved out of one caller-provided device block instead of TreeBufs.
-cudaError_t morton_sort(const Launch &L, int64_t n, const double *px, const double *py, const double *pz,
-                        const uint8_t *kind, const uint8_t *alive, uint64_t *keys, int32_t *order, void *scratch,
-                        size_t scratch_bytes, DevInfo **info_out) {
-    if (morton_sort_scratch_bytes(n) > scratch_bytes) return cudaErrorInvalidValue;
-    char *p = static_cast<char *>(scratch);
-    DevInfo *info = reinterpret_cast<DevInfo *>(p);
-    p += align256(sizeof(DevInfo));
-    double *bbox_part = reinterpret_cast<double *>(p);
-    p += align256(sizeof(double) * kFlagBlocksMax * 6);
-    uint32_t *flag = reinterpret_cast<uint32_t *>(p);
-    p += align256(sizeof(uint32_t) * size_t(n));
-    uint64_t *keys_alt = reinterpret_cast<uint64_t *>(p);
-    p += align256(sizeof(uint64_t) * size_t(n));
-    int32_t *order_alt = reinterpret_cast<int32_t *>(p);
-    p += align256(sizeof(int32_t) * size_t(n));
-    const uint32_t ntiles = uint32_t((n + kRsTile - 1) / kRsTile);
-    uint32_t *hist = reinterpret_cast<uint32_t *>(p);
-    p += align256(sizeof(uint32_t) * size_t(ntiles) * kRsBins);
-    uint32_t *tmp = reinterpret_cast<uint32_t *>(p);
-    int64_t tmp_cap = int64_t((static_cast<char *>(scratch) + scratch_bytes - p) / sizeof(uint32_t));
-    *info_out = info;
-    cudaStream_t s = L.stream;
-    cudaError_t e = cudaMemsetAsync(info, 0, sizeof(DevInfo), s);
-    if (e != cudaSuccess || n == 0) return e;
-    unsigned fb = blocks_for(n, kThreads);
-    if (fb > unsigned(kFlagBlocksMax)) fb = kFlagBlocksMax;
-    k_flags_bbox_noacc<<<fb, kThreads, 0, s>>>(n, px, py, pz, kind, alive, flag, bbox_part);
-    GBH_LAUNCH_CHECK();
-    if ((e = scan_u32(L, flag, flag, n, tmp, tmp_cap)) != cudaSuccess) return e;
-    k_bbox_final<<<1, kFinalThreads, 0, s>>>(int(fb), bbox_part, n, flag, kind, alive, 0.9, info, nullptr);
-    GBH_LAUNCH_CHECK();
-    k_compact_keys<<<blocks_for(n, kThreads), kThreads, 0, s>>>(n, px, py, pz, kind, alive, flag, info, keys, order);
-    GBH_LAUNCH_CHECK();
-    uint64_t *kin = keys, *kout = keys_alt;
-    int32_t *vin = order, *vout = order_alt;
-    for (int shift = 0; shift < 64; shift += 8) {
-        k_rs_hist<false><<<ntiles ? ntiles : 1, kRsThreads, 0, s>>>(kin, vin, nullptr, info, shift, ntiles ? ntiles : 1,
-                                                                    hist);
-        GBH_LAUNCH_CHECK();
-        if ((e = scan_u32(L, hist, hist, int64_t(ntiles ? ntiles : 1) * kRsBins, tmp, tmp_cap)) != cudaSuccess) return e;
-        k_rs_scatter<false><<<ntiles ? ntiles : 1, kRsThreads, 0, s>>>(kin, vin, kout, vout, nullptr, info, shift,
-                                                                        ntiles ? ntiles : 1, hist);
-        GBH_LAUNCH_CHECK();
-        uint64_t *tk = kin;
-        kin = kout;
-        kout = tk;
-        int32_t *tv = vin;
-        vin = vout;
-        vout = tv;
-    }
-    return cudaSuccess;  // eight passes: the result is back in keys/order
-}
-
-}  // namespace gbh
-
-namespace gbh {
-
 // ---------------------------------------------------------------- diagnostics (diag.go:31-135)
 
 namespace {
 
+constexpr int kDiagBlocksMax = 1024;
 constexpr int kDiagSums = 11;  // kinetic, p(3), L(3), m x (3), m
 
 // Per-block sums over bodies i (all bodies, as Momentum/AngularMomentum/CenterOfMass iterate
@@ -2559,13 +1505,13 @@ __global__ __launch_bounds__(kThreads) void k_diag_final(int nparts, const doubl
 
 }  // namespace
 
-int diag_parts() { return kFlagBlocksMax; }
+int diag_parts() { return kDiagBlocksMax; }
 
 cudaError_t diagnostics(const Launch &L, int64_t n, const double *px, const double *py, const double *pz,
                         const double *vx, const double *vy, const double *vz, const double *mass, const uint8_t *kind,
                         double c, int dm_off, double *part, double *out) {
     unsigned nb = blocks_for(n, kThreads);
-    if (nb > unsigned(kFlagBlocksMax)) nb = kFlagBlocksMax;
+    if (nb > unsigned(kDiagBlocksMax)) nb = kDiagBlocksMax;
     k_diag_partial<<<nb, kThreads, 0, L.stream>>>(n, px, py, pz, vx, vy, vz, mass, kind, c, dm_off, part);
     GBH_LAUNCH_CHECK();
     k_diag_final<<<1, kThreads, 0, L.stream>>>(int(nb), part, out);
