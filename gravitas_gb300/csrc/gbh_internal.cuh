@@ -118,13 +118,13 @@ struct TreeBufs {
     float4 *st_hi = nullptr, *st_lo = nullptr;
     float4 *st_off = nullptr;  // FP32 offset of each star from its leaf's centre of mass, and its mass
     // chain topology, indexed by sorted position
-    uint32_t *chain_cnt = nullptr;  // nodes starting at each position, then the scan
+    uint32_t *chain_base = nullptr;  // pre-order index of the first node starting at each position
     // pre-order node arrays (index p)
     int32_t *pre_parent = nullptr;
     uint32_t *pre_info = nullptr;   // level | octant << 8
     uint32_t *pre_mask = nullptr;   // occupied child octants (bit per octant)
-    uint32_t *pre_nchild = nullptr; // child count, then its exclusive scan
-    int32_t *pre_ref = nullptr;     // reference index of pre-order node p
+    uint32_t *child_base = nullptr; // children of the nodes before p
+    int32_t *pre_hi = nullptr;      // end of the node's star range
     int32_t *pre_star = nullptr;    // sorted position whose chain holds pre-order node p
     // reference-layout node arrays (index r)
     gbh_node *nodes = nullptr;
@@ -136,7 +136,7 @@ struct TreeBufs {
     int2 *mrange = nullptr;
     LNode *lnode = nullptr;         // list-walk records
     uint32_t *walk_ctr = nullptr;   // list walk: next group to take (persistent warps)
-    int32_t *leaves = nullptr;      // sorted position of every leaf's first star
+    int32_t *leaves = nullptr;      // the leaves' node indices
     int32_t *targets = nullptr;     // sorted positions of the stars a restricted walk evaluates
     // forest: systems, their geometry, the system of every sorted star, mixed-walk groups
     int32_t nsys = 1;

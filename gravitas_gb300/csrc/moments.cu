@@ -179,9 +179,6 @@ __device__ __forceinline__ void grp_sum_quad(FMom &q) {
 // together with the next node's fields and parent, loaded one level ahead).
 __global__ __launch_bounds__(kThreads) void k_upsweep_fast(const uint64_t *__restrict__ keys, const DevInfo *info,
                                                            const int32_t *__restrict__ leaves,
-                                                           const uint32_t *__restrict__ cnt,
-                                                           const uint32_t *__restrict__ base,
-                                                           const int32_t *__restrict__ pre_ref,
                                                            const float4 *__restrict__ st_hi,
                                                            const float4 *__restrict__ st_lo,
                                                            float4 *__restrict__ st_off, const gbh_node *nodes,
@@ -201,22 +198,16 @@ __global__ __launch_bounds__(kThreads) void k_upsweep_fast(const uint64_t *__res
         int32_t r = 0, P = -1, GP = -1;
         UpNode u, pu;
         if (act) {
-            const int32_t i = leaves[t];
-            if (i < 0 || i >= ns || cnt[i] == 0) {
+            r = leaves[t];
+            if (r < 0 || r >= nn) {
                 act = false;
-                if (leader) set_err(err_info, 23);
+                if (leader) set_err(err_info, 20);
             } else {
-                r = pre_ref[base[i] + cnt[i] - 1];  // the last node of a chain is a leaf
-                if (r < 0 || r >= nn) {
+                u = up_node(nodes, n_info, r);
+                P = n_parent[r];
+                if (u.lo < 0 || u.hi > ns || u.lo >= u.hi) {
                     act = false;
-                    if (leader) set_err(err_info, 20);
-                } else {
-                    u = up_node(nodes, n_info, r);
-                    P = n_parent[r];
-                    if (u.lo < 0 || u.hi > ns || u.lo >= u.hi) {
-                        act = false;
-                        if (leader) set_err(err_info, 21);
-                    }
+                    if (leader) set_err(err_info, 21);
                 }
             }
         }
@@ -394,12 +385,11 @@ __global__ __launch_bounds__(kThreads) void k_export_fast(const DevInfo *info, c
 }  // namespace
 
 cudaError_t upsweep_fast(const Launch &L, TreeBufs &b, bool plain_records) {
-    const uint32_t *cnt = b.chain_cnt, *base = b.chain_cnt + b.cap_n;
     // a group of 8 lanes per leaf (at most one leaf per node), grid-stride beyond 4096 blocks
     int64_t nb = (b.cap_nodes + kThreads / kGroup - 1) / (kThreads / kGroup);
     nb = nb < 1 ? 1 : nb > 4096 ? 4096 : nb;
     k_upsweep_fast<<<unsigned(nb), kThreads, 0, L.stream>>>(
-        b.keys, b.info, b.leaves, cnt, base, b.pre_ref, b.st_hi, b.st_lo, b.st_off, b.nodes, b.n_parent, b.n_info,
+        b.keys, b.info, b.leaves, b.st_hi, b.st_lo, b.st_off, b.nodes, b.n_parent, b.n_info,
         b.n_arrive,
         b.pnodes, b.mnodes, b.mrange, b.lnode, plain_records, b.nsys > 1 ? b.sid_sorted : nullptr, b.geo, b.info);
     ++*L.count;

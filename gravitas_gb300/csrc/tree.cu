@@ -6,8 +6,7 @@
 //
 // Pipeline of tree_build (one stream, no host round trip):
 //   sort_stars (sort.cu)                                            (collect, keys, sort, build.go:11-41, 62-113)
-//   k_chain_count -> scan -> k_chain_emit -> scan -> k_ref_index -> k_emit_nodes
-//                                                                   (node set and links of buildNode, build.go:134-172)
+//   k_chains -> k_topology -> k_child_scan -> k_emit_nodes          (node set and links of buildNode, build.go:134-172)
 //   k_upsweep                                                       (finish, build.go:176-217)
 //
 // Node set without recursion. A cell at level L is the set of sorted stars whose keys share
@@ -146,45 +145,6 @@ cudaError_t scan_rec(const Launch &L, const uint32_t *in, uint32_t *out, int64_t
     return cudaGetLastError();
 }
 
-constexpr int kLbScans = 2;  // of a build: chain counts, child counts
-inline int64_t lb_tiles(int64_t n) { return (n + kScanTile - 1) / kScanTile; }
-
-// Single-pass exclusive scan with decoupled look-back (one launch, in place of a reduce, a scan of
-// the tile sums and an apply): a block takes the next tile from *ctr.
-__global__ __launch_bounds__(kScanThreads) void k_scan_lb(const uint32_t *in, uint32_t *out, int64_t n,
-                                                          const int64_t *ndyn, uint32_t *ctr,
-                                                          unsigned long long *status, DevInfo *info) {
-    __shared__ uint32_t s_warp[kScanThreads / 32 + 1];
-    __shared__ uint32_t s_tile;
-    __shared__ unsigned long long s_prefix;
-    if (threadIdx.x == 0) s_tile = atomicAdd(ctr, 1u);
-    __syncthreads();
-    const uint32_t tile = s_tile;
-    const int64_t ne = dyn_len(n, ndyn);
-    if (int64_t(tile) * kScanTile >= ne) return;  // uniform
-    const int64_t base = int64_t(tile) * kScanTile + int64_t(threadIdx.x) * kScanItems;
-    uint32_t v[kScanItems];
-    uint32_t sum = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        v[k] = base + k < ne ? in[base + k] : 0;
-        sum += v[k];
-    }
-    uint32_t total;
-    uint32_t run = block_excl_scan<kScanThreads>(sum, s_warp, total);
-    if (threadIdx.x < 32) {
-        const unsigned long long excl = look_back(status, tile, total, info);
-        if (threadIdx.x == 0) s_prefix = excl;
-    }
-    __syncthreads();
-    run += uint32_t(s_prefix);
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        if (base + k < ne) out[base + k] = run;
-        run += v[k];
-    }
-}
-
 // ---------------------------------------------------------------- node set (chains)
 
 // Sorted star range [lo, hi) of the system that sorted position i belongs to (the whole array
@@ -257,88 +217,94 @@ __device__ int64_t cell_start(const uint64_t *__restrict__ keys, int64_t lo_boun
     return lo;
 }
 
-// Number of nodes that start at sorted position i.
-__global__ __launch_bounds__(kThreads) void k_chain_count(const uint64_t *__restrict__ keys, const DevInfo *info,
-                                                          const int32_t *__restrict__ sid_sorted,
-                                                          const SysGeo *__restrict__ geo, int leaf,
-                                                          uint32_t *__restrict__ cnt) {
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    int64_t n = info->nstars;
-    if (i >= n) return;
-    const SysRange R = sys_range(sid_sorted, geo, i, n);
-    int L0 = start_level(keys, i, R.lo);
-    uint32_t c = 0;
-    if (L0 <= kMaxLevel) {
-        // A level-L cell starting at i holds more than leaf stars exactly when the star leaf
-        // positions on is still inside it (cells are contiguous runs of the sorted keys).
-        const uint64_t ki = keys[i];
-        const bool ahead = i + leaf < R.hi;
-        const uint64_t ka = ahead ? keys[i + leaf] : 0;
-        bool exists = true;
-        if (i > R.lo) {  // the parent cell (level L0-1) contains i-1 and i; it splits iff it holds > leaf stars
-            int Lp = L0 - 1;
-            exists = (ahead && prefix(ka, Lp) == prefix(ki, Lp)) ||
-                     cell_end(keys, R.hi, i, Lp) - cell_start(keys, R.lo, i, Lp) > leaf;
-        }
-        if (exists) {
-            for (int L = L0;; ++L) {
-                ++c;
-                if (!(ahead && prefix(ka, L) == prefix(ki, L) && L < kMaxLevel)) break;
+// Nodes that start at sorted position i of the system [lo, hi) (0 when none), from level L0 on.
+__device__ __forceinline__ uint32_t chain_at(const uint64_t *__restrict__ keys, int64_t i, int64_t lo, int64_t hi,
+                                             int leaf, int &L0) {
+    L0 = start_level(keys, i, lo);
+    if (L0 > kMaxLevel) return 0;
+    // A level-L cell starting at i holds more than leaf stars exactly when the star leaf positions on
+    // is still inside it (cells are contiguous runs of the sorted keys).
+    const uint64_t ki = keys[i];
+    const bool ahead = i + leaf < hi;
+    const uint64_t ka = ahead ? keys[i + leaf] : 0;
+    if (i > lo) {  // the parent cell (level L0-1) contains i-1 and i; the node exists iff it holds > leaf stars
+        const int Lp = L0 - 1;
+        const uint64_t P = prefix(ki, Lp);
+        if (!(ahead && prefix(ka, Lp) == P)) {
+            // at most leaf of its stars from i on: a of them, so leaf + 1 - a before i are needed
+            int64_t x = i + 1, y = ahead ? i + leaf : hi;
+            while (x < y) {
+                const int64_t mid = (x + y) >> 1;
+                if (prefix(keys[mid], Lp) == P) x = mid + 1;
+                else y = mid;
             }
+            const int64_t j = i - (leaf + 1 - (x - i));
+            if (j < lo || prefix(keys[j], Lp) != P) return 0;
         }
     }
-    cnt[i] = c;
+    if (!ahead) return 1;
+    // the deepest level at which star i + leaf shares the cell; every such level from L0 to 20 splits
+    const uint64_t d = ki ^ ka;
+    const int S = d ? kMaxLevel - 1 - (63 - __clzll(static_cast<long long>(d))) / 3 : kMaxLevel - 1;
+    const int last = S < kMaxLevel - 1 ? S : kMaxLevel - 1;
+    return last >= L0 ? uint32_t(last - L0 + 2) : 1u;
 }
 
-// Pre-order node arrays: parent (pre-order index), level | octant << 8 | child mask << 16,
-// child count. base = exclusive scan of cnt: the pre-order index of the first node at i.
-__global__ __launch_bounds__(kThreads) void k_chain_emit(const uint64_t *__restrict__ keys, DevInfo *info,
-                                                         const uint32_t *__restrict__ cnt,
-                                                         const uint32_t *__restrict__ base,
-                                                         int32_t *__restrict__ pre_parent,
-                                                         uint32_t *__restrict__ pre_info,
-                                                         uint32_t *__restrict__ pre_nchild,
-                                                         uint32_t *__restrict__ pre_mask,
-                                                         int32_t *__restrict__ pre_star,
-                                                         int32_t *__restrict__ leaves,
-                                                         const int32_t *__restrict__ sid_sorted,
-                                                         const SysGeo *__restrict__ geo) {
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    int64_t n = info->nstars;
-    uint32_t c = i < n ? cnt[i] : 0;
-    // every position with nodes ends its chain in exactly one leaf: append it to the leaf list
-    unsigned m = __ballot_sync(0xffffffffu, c > 0);
-    if (m) {
-        int lane = threadIdx.x & 31;
-        uint32_t off = 0;
-        if (lane == __ffs(m) - 1) off = atomicAdd(&info->nleaves, uint32_t(__popc(m)));
-        off = __shfl_sync(0xffffffffu, off, __ffs(m) - 1);
-        if (c > 0) leaves[off + __popc(m & ((1u << lane) - 1u))] = int32_t(i);
+// The nodes in pre-order, chain by chain: base[i] is the pre-order index of the first node at sorted
+// position i (an exclusive scan of the chain lengths, by look-back), and each node gets its star,
+// level | octant << 8 and an empty child mask. A block takes the next tile of 1,024 positions.
+constexpr int kChainThreads = 512, kChainTile = 2 * kChainThreads;
+inline int64_t chain_tiles(int64_t n) { return (n + kChainTile - 1) / kChainTile; }
+__global__ __launch_bounds__(kChainThreads) void k_chains(const uint64_t *__restrict__ keys, DevInfo *info,
+                                                          const int32_t *__restrict__ sid_sorted,
+                                                          const SysGeo *__restrict__ geo, int leaf,
+                                                          uint32_t *__restrict__ base, int32_t *__restrict__ pre_star,
+                                                          uint32_t *__restrict__ pre_info,
+                                                          uint32_t *__restrict__ pre_mask, uint32_t *lb,
+                                                          int64_t cap_nodes) {
+    __shared__ uint32_t s_warp[kChainThreads / 32 + 1];
+    __shared__ uint32_t s_tile, s_prefix;
+    if (threadIdx.x == 0) s_tile = atomicAdd(lb, 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    const int64_t n = info->nstars;
+    const int64_t i0 = int64_t(tile) * kChainTile + threadIdx.x;
+    if (int64_t(tile) * kChainTile >= n) return;  // uniform
+    uint32_t c[2] = {0, 0};
+    int L0[2] = {0, 0};
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int64_t i = i0 + q * kChainThreads;
+        if (i >= n) continue;
+        const SysRange R = sys_range(sid_sorted, geo, i, n);
+        c[q] = chain_at(keys, i, R.lo, R.hi, leaf, L0[q]);
     }
-    if (i >= n) return;
-    if (i == n - 1) info->nnodes = int64_t(base[i]) + c;
-    if (c == 0) return;
-    const SysRange R = sys_range(sid_sorted, geo, i, n);
-    int L0 = start_level(keys, i, R.lo);
-    int32_t parent_pre = -1;
-    if (i > R.lo) {
-        int Lp = L0 - 1;
-        int64_t ps = cell_start(keys, R.lo, i, Lp);
-        int Lps = start_level(keys, ps, R.lo);  // ps starts its chain at this level; the parent is Lp - Lps deeper
-        parent_pre = int32_t(base[ps]) + (Lp - Lps);
+    uint32_t total;  // both halves in one scan: at most 512 x 22 nodes each
+    const uint32_t excl = block_excl_scan<kChainThreads>(c[0] | c[1] << 16, s_warp, total);
+    const uint32_t sum = (total & 0xffffu) + (total >> 16);
+    if (threadIdx.x < 32) {
+        const unsigned long long e = look_back(reinterpret_cast<unsigned long long *>(lb + 2), tile, sum, info);
+        if (threadIdx.x == 0) s_prefix = uint32_t(e);
     }
-    uint64_t key = keys[i];
-    uint32_t p = base[i];
-    for (uint32_t t = 0; t < c; ++t, ++p) {
-        int L = L0 + int(t);
-        uint32_t oct = L == 0 ? 0u : uint32_t(key >> (3 * (kMaxLevel - L))) & 7u;
-        int32_t par = t == 0 ? parent_pre : int32_t(p) - 1;
-        pre_parent[p] = par;
-        pre_info[p] = uint32_t(L) | oct << 8;
-        pre_star[p] = int32_t(i);
-        if (par >= 0) {  // every node marks its octant in its parent's child mask (both zeroed first)
-            atomicOr(&pre_mask[par], 1u << oct);
-            atomicAdd(&pre_nchild[par], 1u);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int64_t i = i0 + q * kChainThreads;
+        if (i >= n) continue;
+        const uint32_t b = s_prefix + (q ? (total & 0xffffu) + (excl >> 16) : excl & 0xffffu);
+        base[i] = b;
+        if (i == n - 1) info->nnodes = int64_t(b) + c[q];
+        const uint64_t key = keys[i];
+        for (uint32_t t = 0; t < c[q]; ++t) {
+            const int64_t p = int64_t(b) + t;
+            if (p >= cap_nodes) {
+                dev_error(info, 11);
+                break;
+            }
+            const int L = L0[q] + int(t);
+            pre_star[p] = int32_t(i);
+            pre_info[p] = uint32_t(L) | (L == 0 ? 0u : uint32_t(key >> (3 * (kMaxLevel - L))) & 7u) << 8;
+            pre_mask[p] = 0;
         }
     }
 }
@@ -346,87 +312,152 @@ __global__ __launch_bounds__(kThreads) void k_chain_emit(const uint64_t *__restr
 // Grid of the per-node kernels below: they loop over the nodes, whose count only the device knows.
 inline unsigned node_blocks(int64_t cap_nodes) {
     const unsigned nb = blocks_for(cap_nodes, kThreads);
-    return nb < 4096u ? nb : 4096u;
+    return nb < 2048u ? nb : 2048u;
 }
 
-// Reference index of every node: 1 + (children allocated before its parent's block) + rank
-// among the parent's non-empty octants. child_base = exclusive scan of child counts. One thread
-// per node (pre-order index p).
-__global__ __launch_bounds__(kThreads) void k_ref_index(DevInfo *info, const uint32_t *__restrict__ base,
-                                                        const int32_t *__restrict__ pre_star,
-                                                        const int32_t *__restrict__ pre_parent,
-                                                        const uint32_t *__restrict__ pre_info,
-                                                        const uint32_t *__restrict__ pre_mask,
-                                                        const uint32_t *__restrict__ child_base,
-                                                        int32_t *__restrict__ pre_ref,
-                                                        const int32_t *__restrict__ sid_sorted,
-                                                        const SysGeo *__restrict__ geo, int64_t cap_nodes) {
+// Parent (pre-order index) and end of every node's cell, one thread per node, so that the searches
+// of all nodes run side by side; every node marks its octant in its parent's child mask. The
+// parent is the node before in the same chain, or, for a chain's first node, the node at the
+// start of the cell one level up.
+__global__ __launch_bounds__(kThreads) void k_topology(const uint64_t *__restrict__ keys, DevInfo *info,
+                                                       const uint32_t *__restrict__ base,
+                                                       const int32_t *__restrict__ pre_star,
+                                                       const uint32_t *__restrict__ pre_info, uint32_t *pre_mask,
+                                                       int32_t *__restrict__ pre_parent, int32_t *__restrict__ pre_hi,
+                                                       const int32_t *__restrict__ sid_sorted,
+                                                       const SysGeo *__restrict__ geo, int64_t cap_nodes) {
     const int64_t n = info->nstars, nn = info->nnodes < cap_nodes ? info->nnodes : cap_nodes;
-    if (blockIdx.x == 0 && threadIdx.x == 0 && info->nnodes > cap_nodes) dev_error(info, 11);
     for (int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < nn; p += int64_t(gridDim.x) * blockDim.x) {
         const int64_t i = pre_star[p];
         if (i < 0 || i >= n) {
             dev_error(info, 11);
             continue;
         }
-        // a system's nodes are the pre-order block starting at its root (pre-order index of its
-        // first star's chain); its reference layout fills the same block
-        const uint32_t root = base[sys_range(sid_sorted, geo, i, n).lo];
-        const int32_t pp = pre_parent[p];
-        if (pp < 0) {
-            pre_ref[p] = int32_t(root);
-            continue;
+        const uint32_t inf = pre_info[p];
+        const int L = int(inf & 0xffu);
+        const SysRange R = sys_range(sid_sorted, geo, i, n);
+        int32_t par = -1;
+        if (L > 0) {
+            if (base[i] < uint32_t(p)) {
+                par = int32_t(p) - 1;
+            } else {
+                const int64_t ps = cell_start(keys, R.lo, i, L - 1);
+                par = int32_t(base[ps]) + (L - 1 - start_level(keys, ps, R.lo));
+            }
+            if (par < 0 || par >= nn) {
+                dev_error(info, 11);
+                par = -1;
+            }
         }
-        const uint32_t oct = (pre_info[p] >> 8) & 0xffu;
-        const uint32_t pmask = pre_mask[pp];
-        pre_ref[p] = int32_t(root + 1 + (child_base[pp] - child_base[root]) + __popc(pmask & ((1u << oct) - 1u)));
+        pre_parent[p] = par;
+        pre_hi[p] = int32_t(cell_end(keys, R.hi, i, L));
+        if (par >= 0) atomicOr(&pre_mask[par], 1u << (inf >> 8 & 0xffu));
     }
 }
 
-// Links and ranges of every node in the reference layout (bh.go:59-67). One thread per node: the
-// search for the end of its cell runs beside the other nodes' searches, not after those of the
-// shallower nodes of its chain.
-__global__ __launch_bounds__(kThreads) void k_emit_nodes(const uint64_t *__restrict__ keys, DevInfo *info,
-                                                         const uint32_t *__restrict__ cnt,
-                                                         const uint32_t *__restrict__ base,
+// Exclusive scan of the nodes' child counts (the bits of their masks), in one launch by look-back.
+inline int64_t child_tiles(int64_t cap_nodes) { return (cap_nodes + kScanTile - 1) / kScanTile; }
+__global__ __launch_bounds__(kScanThreads) void k_child_scan(const uint32_t *__restrict__ pre_mask,
+                                                             uint32_t *__restrict__ child_base, int64_t cap_nodes,
+                                                             uint32_t *lb, DevInfo *info) {
+    __shared__ uint32_t s_warp[kScanThreads / 32 + 1];
+    __shared__ uint32_t s_tile, s_prefix;
+    if (threadIdx.x == 0) s_tile = atomicAdd(lb, 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    const int64_t nn = info->nnodes < cap_nodes ? info->nnodes : cap_nodes;
+    if (int64_t(tile) * kScanTile >= nn) return;  // uniform
+    const int64_t p0 = int64_t(tile) * kScanTile + int64_t(threadIdx.x) * kScanItems;
+    uint32_t v[kScanItems], sum = 0, total;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+        v[k] = p0 + k < nn ? __popc(pre_mask[p0 + k]) : 0;
+        sum += v[k];
+    }
+    uint32_t run = block_excl_scan<kScanThreads>(sum, s_warp, total);
+    if (threadIdx.x < 32) {
+        const unsigned long long e = look_back(reinterpret_cast<unsigned long long *>(lb + 2), tile, total, info);
+        if (threadIdx.x == 0) s_prefix = uint32_t(e);
+    }
+    __syncthreads();
+    run += s_prefix;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+        if (p0 + k < nn) child_base[p0 + k] = run;
+        run += v[k];
+    }
+}
+
+// Links and ranges of every node in the reference layout (bh.go:59-67), one thread per node, and the
+// list of leaves. A node's reference index: 1 + (children allocated before its parent's block) + its
+// rank among the parent's non-empty octants, inside its system's block of the table (which starts
+// at the pre-order index of the system's first chain). It is formed where it is needed (the node's
+// own, its parent's, and that of the next node of the walk).
+__global__ __launch_bounds__(kThreads) void k_emit_nodes(DevInfo *info, const uint32_t *__restrict__ base,
                                                          const int32_t *__restrict__ pre_star,
                                                          const int32_t *__restrict__ pre_parent,
                                                          const uint32_t *__restrict__ pre_info,
                                                          const uint32_t *__restrict__ pre_mask,
+                                                         const int32_t *__restrict__ pre_hi,
                                                          const uint32_t *__restrict__ child_base,
-                                                         const int32_t *__restrict__ pre_ref, gbh_node *__restrict__ nodes,
-                                                         int32_t *__restrict__ n_parent, uint32_t *__restrict__ n_info,
-                                                         int32_t *__restrict__ n_arrive,
+                                                         gbh_node *__restrict__ nodes, int32_t *__restrict__ n_parent,
+                                                         uint32_t *__restrict__ n_info, int32_t *__restrict__ n_arrive,
+                                                         int32_t *__restrict__ leaves,
                                                          const int32_t *__restrict__ sid_sorted,
                                                          const SysGeo *__restrict__ geo, int64_t cap_nodes) {
     const int64_t n = info->nstars, nn = info->nnodes < cap_nodes ? info->nnodes : cap_nodes;
-    for (int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < nn; p += int64_t(gridDim.x) * blockDim.x) {
-        const int64_t i = pre_star[p];
-        const int32_t r = pre_ref[p];
-        if (i < 0 || i >= n || r < 0 || r >= nn) {
-            dev_error(info, 11);
-            continue;
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    // whole warps iterate together (the ballot below needs every lane)
+    for (int64_t p0 = int64_t(blockIdx.x) * blockDim.x + (threadIdx.x & ~31); p0 < nn; p0 += stride) {
+        const int64_t p = p0 + lane;
+        int32_t r = -1;
+        bool is_leaf = false;
+        if (p < nn) {
+            const int64_t i = pre_star[p];
+            const int32_t pp = pre_parent[p];
+            const uint32_t inf = pre_info[p], mask = pre_mask[p];
+            const int64_t hi = pre_hi[p];
+            const SysRange R = sys_range(sid_sorted, geo, i < 0 || i >= n ? 0 : i, n);
+            const uint32_t root = base[R.lo];
+            const uint32_t root_children = child_base[root];
+            // the reference index of the node with octant word `w` under parent q (-1: the root)
+            auto ref = [&](int32_t q, uint32_t w) {
+                if (q < 0) return int32_t(root);
+                return int32_t(root + 1 + (child_base[q] - root_children) +
+                               __popc(pre_mask[q] & ((1u << (w >> 8 & 0xffu)) - 1u)));
+            };
+            r = ref(pp, inf);
+            int32_t nx = -1;  // a system's walk ends at its own last node
+            bool ok = i >= 0 && i < n && r >= 0 && r < nn && hi > i && hi <= R.hi;
+            if (ok && hi < R.hi) {
+                const uint32_t q = base[hi];
+                ok = q < uint32_t(nn) && pre_star[q] == int32_t(hi);
+                if (ok) nx = ref(pre_parent[q], pre_info[q]);
+                ok = ok && nx >= 0 && nx < nn;
+            }
+            if (!ok) {
+                dev_error(info, 12);
+                r = -1;
+            } else {
+                is_leaf = mask == 0;
+                gbh_node &nd = nodes[r];
+                nd.first = mask ? int32_t(root + 1 + (child_base[p] - root_children)) : -1;
+                nd.next = nx;
+                nd.lo = int32_t(i);
+                nd.hi = int32_t(hi);
+                n_parent[r] = pp < 0 ? -1 : ref(pre_parent[pp], pre_info[pp]);
+                n_info[r] = (inf & 0xffu) | uint32_t(__popc(mask)) << 8;
+                n_arrive[r] = 0;
+            }
         }
-        const SysRange R = sys_range(sid_sorted, geo, i, n);
-        const uint32_t root = base[R.lo];
-        const uint32_t inf = pre_info[p];
-        const int L = int(inf & 0xffu);
-        const uint32_t mask = pre_mask[p];
-        const int64_t hi = cell_end(keys, R.hi, i, L);
-        gbh_node &nd = nodes[r];
-        nd.first = mask ? int32_t(root + 1 + (child_base[p] - child_base[root])) : -1;
-        int32_t nx = hi == R.hi ? -1 : pre_ref[base[hi]];  // a system's walk ends at its own last node
-        if (nx >= nn || (hi < R.hi && cnt[hi] == 0)) {
-            dev_error(info, 12);
-            nx = -1;
+        const unsigned m = __ballot_sync(0xffffffffu, is_leaf);
+        if (m) {
+            uint32_t off = 0;
+            if (lane == __ffs(m) - 1) off = atomicAdd(&info->nleaves, uint32_t(__popc(m)));
+            off = __shfl_sync(0xffffffffu, off, __ffs(m) - 1);
+            if (is_leaf) leaves[off + __popc(m & ((1u << lane) - 1u))] = r;
         }
-        nd.next = nx;
-        nd.lo = int32_t(i);
-        nd.hi = int32_t(hi);
-        const int32_t pp = pre_parent[p];
-        n_parent[r] = pp < 0 ? -1 : pre_ref[pp];
-        n_info[r] = uint32_t(L) | uint32_t(__popc(mask)) << 8;
-        n_arrive[r] = 0;
     }
 }
 
@@ -508,20 +539,17 @@ __device__ __forceinline__ double crit2_of(double theta, const Moments &q, doubl
 
 // Bottom-up moments: one thread per leaf; the last child to finish computes its parent.
 __global__ __launch_bounds__(kThreads) void k_upsweep(const uint64_t *__restrict__ keys, const DevInfo *info,
-                                                      const uint32_t *__restrict__ cnt, const uint32_t *__restrict__ base,
-                                                      const int32_t *__restrict__ pre_ref, const double *__restrict__ sx,
-                                                      const double *__restrict__ sy, const double *__restrict__ sz,
-                                                      const double *__restrict__ sm, gbh_node *nodes,
-                                                      const int32_t *__restrict__ n_parent,
+                                                      const int32_t *__restrict__ leaves,
+                                                      const double *__restrict__ sx, const double *__restrict__ sy,
+                                                      const double *__restrict__ sz, const double *__restrict__ sm,
+                                                      gbh_node *nodes, const int32_t *__restrict__ n_parent,
                                                       const uint32_t *__restrict__ n_info, int32_t *n_arrive, PNode *pn,
                                                       MNode *mn, int2 *mr, const int32_t *__restrict__ sid_sorted,
                                                       const SysGeo *__restrict__ geo, DevInfo *err_info) {
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= info->nstars) return;
-    uint32_t c = cnt[i];
-    if (c == 0) return;
+    const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (t >= int64_t(info->nleaves)) return;
     const DevInfo inf = *info;
-    int32_t r = pre_ref[base[i] + c - 1];  // the last node of a chain never splits: a leaf
+    const int32_t r = leaves[t];
     {
         int32_t lo = nodes[r].lo, hi = nodes[r].hi;
         int L = int(n_info[r] & 0xffu);
@@ -1087,7 +1115,7 @@ static cudaError_t scan_dyn(const Launch &L, const uint32_t *in, uint32_t *out, 
 
 void tree_free(TreeBufs &b) {
     void *ptrs[] = {b.flag, b.pos4, b.bbox_part, b.keys, b.keys_alt, b.order, b.order_alt, b.lb_state, b.tile_len, b.hist, b.sx, b.sy, b.sz, b.sm,
-                    b.st_hi, b.st_lo, b.st_off, b.chain_cnt, b.leaves, b.targets, b.geo, b.sid_sorted, b.groups, b.gcost, b.gperm, b.pre_parent, b.pre_info, b.pre_nchild, b.pre_mask, b.pre_ref, b.pre_star, b.nodes,
+                    b.st_hi, b.st_lo, b.st_off, b.chain_base, b.leaves, b.targets, b.geo, b.sid_sorted, b.groups, b.gcost, b.gperm, b.pre_parent, b.pre_info, b.child_base, b.pre_mask, b.pre_hi, b.pre_star, b.nodes,
                     b.n_parent, b.n_info, b.n_arrive, b.pnodes, b.mnodes, b.mrange, b.lnode, b.walk_ctr, b.scan_tmp, b.info, b.part_acc};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -1134,7 +1162,7 @@ cudaError_t tree_alloc(TreeBufs &b, int64_t n, int leaf, int32_t nsys) {
     GBH_ALLOC(b.st_hi, cn);
     GBH_ALLOC(b.st_lo, cn);
     GBH_ALLOC(b.st_off, cn);
-    GBH_ALLOC(b.chain_cnt, cn * 2);  // counts, then their scan
+    GBH_ALLOC(b.chain_base, cn);
     GBH_ALLOC(b.leaves, cn);
     GBH_ALLOC(b.targets, cn);
     const int32_t csys = nsys + nsys / 4 + 1;
@@ -1146,9 +1174,9 @@ cudaError_t tree_alloc(TreeBufs &b, int64_t n, int leaf, int32_t nsys) {
     GBH_ALLOC(b.gperm, cgroups + 1);
     GBH_ALLOC(b.pre_parent, cnodes);
     GBH_ALLOC(b.pre_info, cnodes);
-    GBH_ALLOC(b.pre_nchild, cnodes);
+    GBH_ALLOC(b.child_base, cnodes);
     GBH_ALLOC(b.pre_mask, cnodes);
-    GBH_ALLOC(b.pre_ref, cnodes);
+    GBH_ALLOC(b.pre_hi, cnodes);
     GBH_ALLOC(b.pre_star, cnodes);
     GBH_ALLOC(b.nodes, cnodes);
     GBH_ALLOC(b.n_parent, cnodes);
@@ -1160,8 +1188,8 @@ cudaError_t tree_alloc(TreeBufs &b, int64_t n, int leaf, int32_t nsys) {
     GBH_ALLOC(b.lnode, cnodes);
     GBH_ALLOC(b.walk_ctr, 16);
     GBH_ALLOC(b.scan_tmp, scan_cap);
-    // single-pass scans: the chain counts' and the child counts', and the large sort's
-    b.lb_sort = kLbScans * lb_words_of(lb_tiles(cn > cnodes ? cn : cnodes));
+    // single-pass scans: the chain counts', the child counts', and the large sort's
+    b.lb_sort = lb_words_of(chain_tiles(cn)) + lb_words_of(child_tiles(cnodes));
     const int64_t lb_words = b.lb_sort + sort_lb_words(cn);
     GBH_ALLOC(b.lb_state, lb_words);
     const int64_t ctiles = cn / kSortTile + csys + 1;  // sort tiles never straddle systems
@@ -1193,62 +1221,41 @@ cudaError_t tree_alloc(TreeBufs &b, int64_t n, int leaf, int32_t nsys) {
         if (e_ != cudaSuccess) return e_;          \
     } while (0)
 
-// Single-pass exclusive scan `which` (0 chain counts, 1 child counts) of a build.
-static cudaError_t scan_lb(const Launch &L, TreeBufs &b, int which, const uint32_t *in, uint32_t *out, int64_t n,
-                           const int64_t *ndyn) {
-    const int64_t tiles = lb_tiles(n);
-    if (tiles < 1) return cudaSuccess;
-    uint32_t *base = b.lb_state + int64_t(which) * lb_words_of(lb_tiles(b.cap_n > b.cap_nodes ? b.cap_n : b.cap_nodes));
-    k_scan_lb<<<unsigned(tiles), kScanThreads, 0, L.stream>>>(in, out, n, ndyn, base,
-                                                              reinterpret_cast<unsigned long long *>(base + 2), b.info);
-    ++*L.count;
-    return cudaGetLastError();
-}
-
 cudaError_t tree_build(const Launch &L, TreeBufs &b, int64_t n, const double *px, const double *py, const double *pz,
                        const double *mass, const uint8_t *kind, const uint8_t *alive, double *ax, double *ay,
                        double *az, double theta, int leaf, int dm_off, bool exact, bool plain_records,
                        const ForestTiles *forest_tiles) {
     cudaStream_t s = L.stream;
-    const int64_t cap = b.cap_n;
     const bool forest = b.nsys > 1;
     if (forest && !forest_tiles) return cudaErrorInvalidValue;
     cudaError_t e = sort_stars(L, b, n, px, py, pz, mass, kind, alive, ax, ay, az, theta, dm_off, exact,
                                forest ? forest_tiles : nullptr);
     if (e != cudaSuccess) return e;
-    const unsigned nb = blocks_for(cap, kThreads);
     // node set
-    uint32_t *cnt = b.chain_cnt, *base = b.chain_cnt + cap;
     const int32_t *sid = forest ? b.sid_sorted : nullptr;
-    k_chain_count<<<nb, kThreads, 0, s>>>(b.keys, b.info, sid, b.geo, leaf, cnt);
+    k_chains<<<unsigned(chain_tiles(n)), kChainThreads, 0, s>>>(b.keys, b.info, sid, b.geo, leaf, b.chain_base, b.pre_star,
+                                                                b.pre_info, b.pre_mask, b.lb_state, b.cap_nodes);
     GBH_LAUNCH_CHECK();
-    e = scan_lb(L, b, 0, cnt, base, cap, &b.info->nstars);
-    if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(b.pre_mask, 0, sizeof(uint32_t) * size_t(b.cap_nodes), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(b.pre_nchild, 0, sizeof(uint32_t) * size_t(b.cap_nodes), s);
-    if (e != cudaSuccess) return e;
-    k_chain_emit<<<nb, kThreads, 0, s>>>(b.keys, b.info, cnt, base, b.pre_parent, b.pre_info, b.pre_nchild, b.pre_mask,
-                                         b.pre_star, b.leaves, sid, b.geo);
-    GBH_LAUNCH_CHECK();
-    e = scan_lb(L, b, 1, b.pre_nchild, b.pre_nchild, b.cap_nodes, &b.info->nnodes);
-    if (e != cudaSuccess) return e;
     const unsigned nbn = node_blocks(b.cap_nodes);
-    k_ref_index<<<nbn, kThreads, 0, s>>>(b.info, base, b.pre_star, b.pre_parent, b.pre_info, b.pre_mask, b.pre_nchild,
-                                         b.pre_ref, sid, b.geo, b.cap_nodes);
+    k_topology<<<nbn, kThreads, 0, s>>>(b.keys, b.info, b.chain_base, b.pre_star, b.pre_info, b.pre_mask, b.pre_parent,
+                                        b.pre_hi, sid, b.geo, b.cap_nodes);
     GBH_LAUNCH_CHECK();
-    k_emit_nodes<<<nbn, kThreads, 0, s>>>(b.keys, b.info, cnt, base, b.pre_star, b.pre_parent, b.pre_info, b.pre_mask,
-                                          b.pre_nchild, b.pre_ref, b.nodes, b.n_parent, b.n_info, b.n_arrive, sid,
-                                          b.geo, b.cap_nodes);
+    k_child_scan<<<unsigned(child_tiles(b.cap_nodes)), kScanThreads, 0, s>>>(
+        b.pre_mask, b.child_base, b.cap_nodes, b.lb_state + lb_words_of(chain_tiles(b.cap_n)), b.info);
+    GBH_LAUNCH_CHECK();
+    k_emit_nodes<<<nbn, kThreads, 0, s>>>(b.info, b.chain_base, b.pre_star, b.pre_parent, b.pre_info, b.pre_mask, b.pre_hi,
+                                          b.child_base, b.nodes, b.n_parent, b.n_info, b.n_arrive, b.leaves, sid, b.geo,
+                                          b.cap_nodes);
     GBH_LAUNCH_CHECK();
     if (forest) {
-        k_sys_groups<<<unsigned(b.nsys), 128, 0, s>>>(b.group == 32 ? 32 : 64, base, b.geo, b.groups);
+        k_sys_groups<<<unsigned(b.nsys), 128, 0, s>>>(b.group == 32 ? 32 : 64, b.chain_base, b.geo, b.groups);
         GBH_LAUNCH_CHECK();
     }
     b.moments_exact = exact;
     if (!exact) return upsweep_fast(L, b, plain_records);
-    k_upsweep<<<nb, kThreads, 0, s>>>(b.keys, b.info, cnt, base, b.pre_ref, b.sx, b.sy, b.sz, b.sm, b.nodes,
-                                      b.n_parent, b.n_info, b.n_arrive, b.pnodes, b.mnodes, b.mrange, sid, b.geo,
-                                      b.info);
+    k_upsweep<<<blocks_for(n, kThreads), kThreads, 0, s>>>(b.keys, b.info, b.leaves, b.sx, b.sy, b.sz, b.sm, b.nodes,
+                                                           b.n_parent, b.n_info, b.n_arrive, b.pnodes, b.mnodes,
+                                                           b.mrange, sid, b.geo, b.info);
     GBH_LAUNCH_CHECK();
     return cudaSuccess;
 }
