@@ -414,72 +414,72 @@ cudaError_t walk_plain(const Launch &L, const TreeBufs &b, int64_t nstars_cap, f
 
 // Longest-first order for the next walk from this walk's group costs: groups bucketed by
 // floor(log2 cost), most expensive bucket first, ascending group index inside a bucket (so that
-// neighbouring warps keep walking neighbouring groups). One block of kLptThreads threads, each
-// owning a contiguous run of groups.
-constexpr int kLptThreads = 512, kLptBuckets = 16;  // 32 KB of shared counts
-static_assert(kLptThreads / 32 == kLptBuckets, "the warp totals reuse the bucket array");
+// neighbouring warps keep walking neighbouring groups). One block; each warp takes a contiguous run
+// of groups, 32 at a time, and ranks equal buckets by a match, so costs and order are read and
+// written coalesced: 16,384 groups 35 us with a run of groups per thread, 17 us so.
+constexpr int kLptThreads = 1024, kLptBuckets = 16, kLptWarps = kLptThreads / 32;
 __global__ __launch_bounds__(kLptThreads) void k_lpt_order(const DevInfo *info, int gsize, bool forest,
-                                                           const uint32_t *gcost, int32_t *gperm, int32_t perm_cap) {
-    __shared__ uint32_t cnt[kLptBuckets][kLptThreads];
-    __shared__ uint32_t base[kLptBuckets];
-    const int t = threadIdx.x;
+                                                           const uint32_t *__restrict__ gcost, int32_t *gperm,
+                                                           int32_t perm_cap) {
+    __shared__ uint32_t cnt[kLptBuckets][kLptWarps];  // then the positions of each warp's next groups
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int32_t ng = forest ? int32_t(info->ngroups) : int32_t((info->nstars + gsize - 1) / gsize);
     if (ng > perm_cap) return;  // no order: the walk keeps launch order
-    const int32_t per = (ng + kLptThreads - 1) / kLptThreads;
-    const int32_t g0 = t * per, g1 = g0 + per < ng ? g0 + per : ng;
-    auto bucket = [&](uint32_t c) {
-        int l = 31 - __clz(c | 1u);
+    const int32_t per = ((ng + kLptWarps - 1) / kLptWarps + 31) & ~31;
+    const int32_t g0 = min(warp * per, ng), g1 = min(g0 + per, ng);
+    auto bucket = [&](int32_t g) {  // beyond the run: a bucket of its own
+        if (g >= g1) return kLptBuckets;
+        const int l = 31 - __clz(gcost[g] | 1u);
         return kLptBuckets - 1 - (l < kLptBuckets ? l : kLptBuckets - 1);
     };
-    for (int k = 0; k < kLptBuckets; ++k) cnt[k][t] = 0;
-    for (int32_t g = g0; g < g1; ++g) ++cnt[bucket(gcost[g])][t];
-    __syncthreads();
-    // Exclusive scan of the counts in bucket-major order, kItems consecutive entries per thread:
-    // entry (k, q) becomes the position of thread q's first group of bucket k in the order.
-    constexpr int kItems = kLptBuckets * kLptThreads / kLptThreads;
-    uint32_t *flat = &cnt[0][0];
-    uint32_t v[kItems], sum = 0;
-#pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-        v[i] = flat[t * kItems + i];
-        sum += v[i];
+    if (lane < kLptBuckets) cnt[lane][warp] = 0;
+    __syncwarp();
+#pragma unroll 4
+    for (int32_t g = g0; g < g1; g += 32) {
+        const int k = bucket(g + lane);
+        const unsigned same = __match_any_sync(kFull, k);
+        if (k < kLptBuckets && lane == __ffs(same) - 1) cnt[k][warp] += __popc(same);
+        __syncwarp();
     }
-    const int lane = t & 31, warp = t >> 5;
-    uint32_t incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(kFull, incl, o);
-        if (lane >= o) incl += y;
-    }
-    if (lane == 31) base[warp] = incl;  // warp totals (kLptThreads / 32 == kLptBuckets of them)
     __syncthreads();
-    if (warp == 0) {
-        const uint32_t w = lane < kLptThreads / 32 ? base[lane] : 0;
-        uint32_t wi = w;
+    // exclusive scan in bucket-major order: 16 x 32 counts, warp k < 16 takes bucket k's, lane w warp w's
+    __shared__ uint32_t tot[kLptBuckets];
+    uint32_t v = 0, incl = 0;
+    if (warp < kLptBuckets) {
+        incl = v = cnt[warp][lane];
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(kFull, wi, o);
-            if (lane >= o) wi += y;
+            const uint32_t y = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += y;
         }
-        if (lane < kLptThreads / 32) base[lane] = wi - w;
+        if (lane == 31) tot[warp] = incl;
     }
     __syncthreads();
-    uint32_t run = base[warp] + incl - sum;
-#pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-        flat[t * kItems + i] = run;
-        run += v[i];
+    if (warp < kLptBuckets) {
+        uint32_t before = 0;
+        for (int k = 0; k < warp; ++k) before += tot[k];
+        cnt[warp][lane] = before + incl - v;
     }
     __syncthreads();
-    for (int32_t g = g0; g < g1; ++g) {
-        int k = bucket(gcost[g]);
-        gperm[cnt[k][t]++] = g;
+#pragma unroll 4
+    for (int32_t g = g0; g < g1; g += 32) {
+        const int k = bucket(g + lane);
+        const unsigned same = __match_any_sync(kFull, k);
+        uint32_t at = 0;
+        if (k < kLptBuckets) at = cnt[k][warp] + __popc(same & ((1u << lane) - 1u));
+        __syncwarp();
+        if (k < kLptBuckets) {
+            gperm[at] = g + lane;
+            if (lane == __ffs(same) - 1) cnt[k][warp] += __popc(same);
+        }
+        __syncwarp();
     }
-    __syncthreads();
-    if (t == 0) gperm[perm_cap] = ng;
+    if (threadIdx.x == 0) gperm[perm_cap] = ng;
 }
 
-// Sum of a split walk's parts for every walked star, in part order, to state order.
+// Sum of a split walk's parts for every walked star, in part order, to state order. One thread a
+// star and axis (blockIdx.y), eight parts' loads in flight at a time: 16,384 stars in 16 parts 11 us
+// with one thread a star and a load after the other, 6.5 us so (ncu, cold caches).
 __global__ __launch_bounds__(256) void k_split_combine(const DevInfo *info, const int32_t *__restrict__ order,
                                                        const int32_t *__restrict__ targets, int nparts,
                                                        const double *__restrict__ part_acc, int64_t stride,
@@ -488,17 +488,19 @@ __global__ __launch_bounds__(256) void k_split_combine(const DevInfo *info, cons
     const int64_t nt = targets ? int64_t(info->ntargets) : info->nstars;
     if (t >= nt) return;
     const int32_t k = targets ? targets[t] : int32_t(t);
-    double x = 0, y = 0, z = 0;
-    for (int p = 0; p < nparts; ++p) {
-        const double *q = part_acc + int64_t(p) * 3 * stride;
-        x += q[k];
-        y += q[stride + k];
-        z += q[2 * stride + k];
-    }
+    const double *q = part_acc + int64_t(blockIdx.y) * stride + k;
     const int32_t o = order[k];
-    ax[o] = x;
-    ay[o] = y;
-    az[o] = z;
+    double x = 0;
+    for (int p0 = 0; p0 < nparts; p0 += 8) {
+        double v[8];
+#pragma unroll
+        for (int p = 0; p < 8; ++p) v[p] = p0 + p < nparts ? q[int64_t(p0 + p) * 3 * stride] : 0.0;
+#pragma unroll
+        for (int p = 0; p < 8; ++p)
+            if (p0 + p < nparts) x += v[p];
+    }
+    double *out = blockIdx.y == 0 ? ax : blockIdx.y == 1 ? ay : az;
+    out[o] = x;
 }
 
 template <bool kQuad, bool kSoft, bool kPot, bool kShared>
@@ -524,10 +526,7 @@ static cudaError_t launch_mixed_t(const Launch &L, const TreeBufs &b, int64_t ns
             ++*L.count;
             cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) return e;
-            k_split_combine<<<blocks_for(nstars_cap, 256), 256, 0, L.stream>>>(
-                b.info, b.order, targets ? b.targets : nullptr, parts, b.part_acc, nstars_cap, ax, ay, az);
-            ++*L.count;
-            return cudaGetLastError();
+            return split_combine(L, b, parts, nstars_cap, targets, ax, ay, az);
         }
     }
     const bool lpt = b.lpt && !targets && !kPot;
@@ -574,8 +573,8 @@ int split_parts(const TreeBufs &b, int64_t nstars_cap, bool targets, int gsize) 
 
 cudaError_t split_combine(const Launch &L, const TreeBufs &b, int nparts, int64_t stride, bool targets, double *ax,
                           double *ay, double *az) {
-    k_split_combine<<<blocks_for(stride, 256), 256, 0, L.stream>>>(b.info, b.order, targets ? b.targets : nullptr,
-                                                                    nparts, b.part_acc, stride, ax, ay, az);
+    k_split_combine<<<dim3(blocks_for(stride, 256), 3), 256, 0, L.stream>>>(
+        b.info, b.order, targets ? b.targets : nullptr, nparts, b.part_acc, stride, ax, ay, az);
     ++*L.count;
     return cudaGetLastError();
 }
