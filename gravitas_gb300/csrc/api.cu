@@ -39,6 +39,7 @@ struct gbh_ctx {
     cudaStream_t stream = nullptr;
     cudaStream_t copy_stream = nullptr;  // device-to-host copies that overlap the walk
     cudaEvent_t copy_done = nullptr;
+    cudaEvent_t fork = nullptr;  // capture: ties the stage events' branch to the step's kernels
     cudaEvent_t ev[6] = {};
     gbh::TreeBufs tb;
     // resident state (state order)
@@ -287,13 +288,17 @@ cudaError_t next_stage_event(gbh_ctx *ctx, cudaEvent_t *ev) {
     return cudaSuccess;
 }
 
-// Records the next stage event of the call on the context's stream.
+// Records the next stage event of the call on the context's stream. In a capture the event-record
+// node hangs off the last kernel on a branch of its own (the copy stream's), so that the step's
+// kernels follow one another directly and each can start under the one before (launch_after).
 cudaError_t stage_event(gbh_ctx *ctx) {
     cudaEvent_t ev;
     cudaError_t r = next_stage_event(ctx, &ev);
     if (r != cudaSuccess) return r;
-    return ctx->capturing ? cudaEventRecordWithFlags(ev, ctx->stream, cudaEventRecordExternal)
-                          : cudaEventRecord(ev, ctx->stream);
+    if (!ctx->capturing) return cudaEventRecord(ev, ctx->stream);
+    if ((r = cudaEventRecord(ctx->fork, ctx->stream)) != cudaSuccess) return r;
+    if ((r = cudaStreamWaitEvent(ctx->copy_stream, ctx->fork, 0)) != cudaSuccess) return r;
+    return cudaEventRecordWithFlags(ev, ctx->copy_stream, cudaEventRecordExternal);
 }
 
 int h2d(gbh_ctx *ctx, void *dst, const void *src, size_t bytes) {
@@ -445,6 +450,9 @@ int capture_step(gbh_ctx *ctx, const gbh_params *p, double dt, const uint8_t *ki
         rc = forces(ctx, p, n, ctx->px, ctx->py, ctx->pz, ctx->mass, kind, alive, ctx->ax, ctx->ay, ctx->az,
                     theta_of(p), true);
     if (e == cudaSuccess && rc == GBH_OK) e = gbh::kick(L, n, h, ctx->vx, ctx->vy, ctx->vz, ctx->ax, ctx->ay, ctx->az);
+    // join the stage events' branch
+    if (e == cudaSuccess && rc == GBH_OK) e = cudaEventRecord(ctx->fork, ctx->copy_stream);
+    if (e == cudaSuccess && rc == GBH_OK) e = cudaStreamWaitEvent(ctx->stream, ctx->fork, 0);
     cudaGraph_t graph = nullptr;
     cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &graph);
     ctx->capturing = false;
@@ -792,7 +800,8 @@ int gbh_create(const gbh_config *cfg, gbh_ctx **out, char *err, int errlen) {
         }
     }
     if ((e = cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking)) != cudaSuccess ||
-        (e = cudaEventCreateWithFlags(&c->copy_done, cudaEventDisableTiming)) != cudaSuccess) {
+        (e = cudaEventCreateWithFlags(&c->copy_done, cudaEventDisableTiming)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming)) != cudaSuccess) {
         gbh_destroy(c);
         return report(GBH_ERR_CUDA, cudaGetErrorString(e));
     }
@@ -822,6 +831,7 @@ void gbh_destroy(gbh_ctx *c) {
         cudaStreamDestroy(c->copy_stream);
     }
     if (c->copy_done) cudaEventDestroy(c->copy_done);
+    if (c->fork) cudaEventDestroy(c->fork);
     for (auto &ev : c->ahead)
         if (ev) cudaEventDestroy(ev);
     if (c->stream) cudaStreamDestroy(c->stream);

@@ -187,7 +187,10 @@ __global__ __launch_bounds__(kThreads) void k_upsweep_fast(const uint64_t *__res
                                                            PNode *pn, MNode *mn, int2 *mr, LNode *ln,
                                                            bool plain_records,
                                                            const int32_t *__restrict__ sid_sorted,
-                                                           const SysGeo *__restrict__ geo, DevInfo *err_info) {
+                                                           const SysGeo *__restrict__ geo, uint32_t *walk_ctr,
+                                                           DevInfo *err_info) {
+    pdl_begin();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *walk_ctr = 0;  // for the list walk that follows
     const int lane = threadIdx.x & 31, k = lane & (kGroup - 1), src = lane & ~(kGroup - 1);
     const bool leader = k == 0;
     const int64_t ns = info->nstars, nn = info->nnodes, nleaves = info->nleaves;
@@ -388,12 +391,11 @@ cudaError_t upsweep_fast(const Launch &L, TreeBufs &b, bool plain_records) {
     // a group of 8 lanes per leaf (at most one leaf per node), grid-stride beyond 4096 blocks
     int64_t nb = (b.cap_nodes + kThreads / kGroup - 1) / (kThreads / kGroup);
     nb = nb < 1 ? 1 : nb > 4096 ? 4096 : nb;
-    k_upsweep_fast<<<unsigned(nb), kThreads, 0, L.stream>>>(
-        b.keys, b.info, b.leaves, b.st_hi, b.st_lo, b.st_off, b.nodes, b.n_parent, b.n_info,
-        b.n_arrive,
-        b.pnodes, b.mnodes, b.mrange, b.lnode, plain_records, b.nsys > 1 ? b.sid_sorted : nullptr, b.geo, b.info);
-    ++*L.count;
-    return cudaGetLastError();
+    GBH_LAUNCH_AFTER(L, k_upsweep_fast, unsigned(nb), kThreads, b.keys, b.info, b.leaves, b.st_hi, b.st_lo, b.st_off,
+                     b.nodes, b.n_parent, b.n_info, b.n_arrive, b.pnodes, b.mnodes, b.mrange, b.lnode, plain_records,
+                     b.nsys > 1 ? b.sid_sorted : nullptr, b.geo, b.walk_ctr, b.info);
+    b.ctr_clear = true;
+    return cudaSuccess;
 }
 
 cudaError_t export_fast_moments(const Launch &L, TreeBufs &b) {

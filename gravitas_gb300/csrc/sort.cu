@@ -17,6 +17,7 @@
 // order needs no extra passes.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <climits>
 
 #include "gbh_internal.cuh"
@@ -38,13 +39,6 @@ inline unsigned blocks_for(int64_t n, int threads) {
     int64_t b = (n + threads - 1) / threads;
     return unsigned(b < 1 ? 1 : b);
 }
-
-#define SORT_LAUNCH_CHECK()                  \
-    do {                                     \
-        ++*L.count;                          \
-        cudaError_t e_ = cudaGetLastError(); \
-        if (e_ != cudaSuccess) return e_;    \
-    } while (0)
 
 __device__ __forceinline__ bool is_star(uint8_t alive, uint8_t kind) { return alive && kind != GBH_BLACK_HOLE; }
 
@@ -155,6 +149,7 @@ __global__ __launch_bounds__(kThreads) void k_bbox(int64_t n, const double *__re
                                                    const uint8_t *__restrict__ alive, double theta, long long *part,
                                                    double *ax, double *ay, double *az, uint32_t *lb, int64_t lb_words,
                                                    DevInfo *info, SysGeo *geo) {
+    pdl_begin();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         info->err = 0;
         info->err_where = 0;
@@ -219,6 +214,7 @@ __global__ __launch_bounds__(kThreads) void k_bbox(int64_t n, const double *__re
 // ---------------------------------------------------------------- forests
 
 __global__ void k_sys_init(int32_t nsys, SysGeo *geo, DevInfo *info, double theta, uint32_t *lb, int64_t lb_words) {
+    pdl_begin();
     const int32_t s = int32_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t w = s; w < lb_words; w += stride) lb[w] = 0;
@@ -246,6 +242,7 @@ __global__ __launch_bounds__(kThreads) void k_bbox_sys(const int4 *__restrict__ 
                                                        const uint8_t *__restrict__ kind,
                                                        const uint8_t *__restrict__ alive, SysGeo *geo, double *ax,
                                                        double *ay, double *az) {
+    pdl_begin();
     const int4 t = tiles[blockIdx.x];
     const int64_t end = min(int64_t(t.x) + kSortTile, sys_off[t.y + 1]);
     long long mn[3] = {LLONG_MAX, LLONG_MAX, LLONG_MAX}, mx[3] = {LLONG_MIN, LLONG_MIN, LLONG_MIN};
@@ -267,6 +264,7 @@ __global__ __launch_bounds__(kThreads) void k_bbox_sys(const int4 *__restrict__ 
 
 // Per system (a warp each): root cube, FP32 views, opening bases.
 __global__ void k_sys_cube(int32_t nsys, double theta, SysGeo *geo) {
+    pdl_begin();
     const int32_t s = int32_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (s >= nsys) return;
     double mn[3], mx[3];
@@ -281,6 +279,7 @@ __global__ void k_sys_cube(int32_t nsys, double theta, SysGeo *geo) {
 // mixed walk, which never straddle two systems. One block, 1,024 systems at a time.
 constexpr int kSysScan = 1024;
 __global__ __launch_bounds__(kSysScan) void k_sys_ranges(int32_t nsys, int32_t gsize, SysGeo *geo, DevInfo *info) {
+    pdl_begin();
     __shared__ uint32_t s_w[2][32];
     __shared__ uint32_t s_run[2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -424,6 +423,7 @@ __global__ __launch_bounds__(kThreads) void k_tile_sort(int64_t n, const int4 *_
                                                         uint64_t *__restrict__ keys, int32_t *__restrict__ order,
                                                         int32_t *__restrict__ tile_len, Pos4 *__restrict__ pos4,
                                                         DevInfo *info) {
+    pdl_begin();
     __shared__ uint64_t s_key[kSortTile];  // by slot
     __shared__ uint64_t s_e[kSortTile + 1];
     const int t = threadIdx.x;
@@ -577,6 +577,7 @@ __global__ __launch_bounds__(kThreads) void k_merge(int64_t n, const int4 *__res
                                                     int32_t *__restrict__ vout, const int32_t *__restrict__ len_in,
                                                     int32_t *__restrict__ len_out, DevInfo *info, SysGeo *geo,
                                                     SortedOut o) {
+    pdl_begin();
     constexpr int kBlocksPerTile = kSortTile / kThreads;
     __shared__ uint64_t s_win[kWindow];
     __shared__ const uint64_t *s_x[kMaxWay];  // the run's window
@@ -696,25 +697,21 @@ cudaError_t run_sort(const Launch &L, int64_t n, const double *px, const double 
                      const int64_t *sys_off, int32_t nsys, int32_t gsize, uint64_t *keys, uint64_t *keys_alt,
                      int32_t *order, int32_t *order_alt, int32_t *len, int32_t *len_alt, Pos4 *pos4, DevInfo *info,
                      SysGeo *geo, const SortedOut &out) {
-    cudaStream_t s = L.stream;
     const MergePlan plan = merge_plan(most);
     // the merges ping-pong between the two buffers and end in keys / order
     uint64_t *kin = plan.levels & 1 ? keys_alt : keys, *kout = plan.levels & 1 ? keys : keys_alt;
     int32_t *vin = plan.levels & 1 ? order_alt : order, *vout = plan.levels & 1 ? order : order_alt;
-    k_tile_sort<kForest><<<unsigned(ntiles), kThreads, 0, s>>>(n, tiles, ntiles, sys_off, px, py, pz, mass, kind, alive,
-                                                               geo, kin, vin, len, pos4, info);
-    SORT_LAUNCH_CHECK();
+    GBH_LAUNCH_AFTER(L, k_tile_sort<kForest>, unsigned(ntiles), kThreads, n, tiles, ntiles, sys_off, px, py, pz, mass,
+                     kind, alive, geo, kin, vin, len, pos4, info);
     if (kForest) {
-        k_sys_ranges<<<1, kSysScan, 0, s>>>(nsys, gsize, geo, info);
-        SORT_LAUNCH_CHECK();
+        GBH_LAUNCH_AFTER(L, k_sys_ranges, 1, kSysScan, nsys, gsize, geo, info);
     }
     int64_t G = 1;
     for (int l = 0; l < plan.levels; ++l) {
         const bool last = l + 1 == plan.levels;
         auto *kernel = last ? k_merge<kForest, true> : k_merge<kForest, false>;
-        kernel<<<unsigned(ntiles) * (kSortTile / kThreads), kThreads, 0, s>>>(
-            n, tiles, ntiles, int32_t(G), plan.K, kin, vin, kout, vout, len, len_alt, info, geo, out);
-        SORT_LAUNCH_CHECK();
+        GBH_LAUNCH_AFTER(L, kernel, unsigned(ntiles) * (kSortTile / kThreads), kThreads, n, tiles, ntiles, int32_t(G),
+                         plan.K, kin, vin, kout, vout, len, len_alt, info, geo, out);
         uint64_t *tk = kin;
         kin = kout;
         kout = tk;
@@ -755,6 +752,7 @@ __global__ __launch_bounds__(kThreads) void k_compact_keys(int64_t n, const doub
                                                            const uint8_t *__restrict__ alive,
                                                            uint64_t *__restrict__ keys, int32_t *__restrict__ order,
                                                            Pos4 *__restrict__ pos4, uint32_t *lb, DevInfo *info) {
+    pdl_begin();
     __shared__ uint32_t s_warp[kThreads / 32 + 1];
     __shared__ uint32_t s_tile, s_prefix;
     const int t = threadIdx.x;
@@ -802,6 +800,7 @@ __global__ __launch_bounds__(kThreads) void k_compact_keys(int64_t n, const doub
 
 __global__ __launch_bounds__(kRsThreads) void k_rs_hist(const uint64_t *__restrict__ keys, const DevInfo *info, int shift,
                                                         uint32_t ntiles, uint32_t *__restrict__ hist) {
+    pdl_begin();
     __shared__ uint32_t h[kRsBins];
     const int64_t n = info->nstars;
     h[threadIdx.x] = 0;
@@ -820,6 +819,7 @@ __global__ __launch_bounds__(kRsThreads) void k_rs_hist(const uint64_t *__restri
 
 // Exclusive scan of the digit table in one launch (look-back over its tiles).
 __global__ __launch_bounds__(kThreads) void k_rs_scan(uint32_t *hist, int64_t n, uint32_t *lb, DevInfo *info) {
+    pdl_begin();
     __shared__ uint32_t s_warp[kThreads / 32 + 1];
     __shared__ uint32_t s_tile, s_prefix;
     if (threadIdx.x == 0) s_tile = atomicAdd(lb, 1u);
@@ -854,6 +854,7 @@ __global__ __launch_bounds__(kRsThreads) void k_rs_scatter(const uint64_t *__res
                                                            uint64_t *__restrict__ kout, int32_t *__restrict__ vout,
                                                            DevInfo *info, int shift, uint32_t ntiles,
                                                            const uint32_t *__restrict__ offs) {
+    pdl_begin();
     __shared__ uint32_t s_run[kRsBins];
     __shared__ uint32_t s_goff[kRsBins];
     __shared__ uint32_t s_w[2][kRsWarps][kRsBins];
@@ -914,6 +915,7 @@ __global__ __launch_bounds__(kRsThreads) void k_rs_scatter(const uint64_t *__res
 // The sorted copies through the order.
 __global__ __launch_bounds__(kThreads) void k_gather(const int32_t *__restrict__ order, DevInfo *info, SysGeo *geo,
                                                      SortedOut o) {
+    pdl_begin();
     const int64_t k = int64_t(blockIdx.x) * kThreads + threadIdx.x;
     if (k == 0) single_system(geo, info);
     if (k < info->nstars) o.write(k, order[k]);
@@ -921,22 +923,18 @@ __global__ __launch_bounds__(kThreads) void k_gather(const int32_t *__restrict__
 
 cudaError_t sort_large(const Launch &L, TreeBufs &b, int64_t n, const double *px, const double *py, const double *pz,
                        const double *mass, const uint8_t *kind, const uint8_t *alive, const SortedOut &out) {
-    cudaStream_t s = L.stream;
     uint32_t *lb = b.lb_state + b.lb_sort;
-    k_compact_keys<<<unsigned(sort_tiles(n)), kThreads, 0, s>>>(n, px, py, pz, mass, kind, alive, b.keys, b.order, b.pos4,
-                                                                lb, b.info);
-    SORT_LAUNCH_CHECK();
+    GBH_LAUNCH_AFTER(L, k_compact_keys, unsigned(sort_tiles(n)), kThreads, n, px, py, pz, mass, kind, alive, b.keys,
+                     b.order, b.pos4, lb, b.info);
     lb += lb_words_of(sort_tiles(n));
     const uint32_t ntiles = uint32_t(rs_tiles(n));
     uint64_t *kin = b.keys, *kout = b.keys_alt;
     int32_t *vin = b.order, *vout = b.order_alt;
     for (int p = 0; p < kRsPasses; ++p) {
-        k_rs_hist<<<ntiles, kRsThreads, 0, s>>>(kin, b.info, 8 * p, ntiles, b.hist);
-        SORT_LAUNCH_CHECK();
-        k_rs_scan<<<unsigned(hist_scan_tiles(n)), kThreads, 0, s>>>(b.hist, int64_t(ntiles) * kRsBins, lb, b.info);
-        SORT_LAUNCH_CHECK();
-        k_rs_scatter<<<ntiles, kRsThreads, 0, s>>>(kin, vin, kout, vout, b.info, 8 * p, ntiles, b.hist);
-        SORT_LAUNCH_CHECK();
+        GBH_LAUNCH_AFTER(L, k_rs_hist, ntiles, kRsThreads, kin, b.info, 8 * p, ntiles, b.hist);
+        GBH_LAUNCH_AFTER(L, k_rs_scan, unsigned(hist_scan_tiles(n)), kThreads, b.hist, int64_t(ntiles) * kRsBins, lb,
+                         b.info);
+        GBH_LAUNCH_AFTER(L, k_rs_scatter, ntiles, kRsThreads, kin, vin, kout, vout, b.info, 8 * p, ntiles, b.hist);
         lb += lb_words_of(hist_scan_tiles(n));
         uint64_t *tk = kin;
         kin = kout;
@@ -945,8 +943,7 @@ cudaError_t sort_large(const Launch &L, TreeBufs &b, int64_t n, const double *px
         vin = vout;
         vout = tv;
     }
-    k_gather<<<blocks_for(n, kThreads), kThreads, 0, s>>>(b.order, b.info, b.geo, out);
-    SORT_LAUNCH_CHECK();
+    GBH_LAUNCH_AFTER(L, k_gather, blocks_for(n, kThreads), kThreads, b.order, b.info, b.geo, out);
     return cudaSuccess;
 }
 
@@ -961,14 +958,12 @@ int64_t sort_hist_words(int64_t n) { return sort_tiles(n) <= kMergeTiles ? 1 : r
 cudaError_t sort_stars(const Launch &L, TreeBufs &b, int64_t n, const double *px, const double *py, const double *pz,
                        const double *mass, const uint8_t *kind, const uint8_t *alive, double *ax, double *ay,
                        double *az, double theta, int dm_off, bool exact, const ForestTiles *forest) {
-    cudaStream_t s = L.stream;
     const SortedOut out = {b.pos4, kind, dm_off, exact ? 1 : 0, b.sx, b.sy, b.sz, b.sm, b.st_hi, b.st_lo, b.sid_sorted};
     if (!forest) {
         unsigned nb = blocks_for(n, kThreads);
         if (nb > unsigned(kBboxBlocks)) nb = kBboxBlocks;
-        k_bbox<<<nb, kThreads, 0, s>>>(n, px, py, pz, mass, kind, alive, theta, b.bbox_part, ax, ay, az, b.lb_state,
-                                       b.lb_words, b.info, b.geo);
-        SORT_LAUNCH_CHECK();
+        GBH_LAUNCH_AFTER(L, k_bbox, nb, kThreads, n, px, py, pz, mass, kind, alive, theta, b.bbox_part, ax, ay, az,
+                         b.lb_state, b.lb_words, b.info, b.geo);
         const int32_t ntiles = int32_t(sort_tiles(n));
         if (ntiles > kMergeTiles) return sort_large(L, b, n, px, py, pz, mass, kind, alive, out);
         return run_sort<false>(L, n, px, py, pz, mass, kind, alive, nullptr, ntiles, ntiles, nullptr, 1, 64, b.keys,
@@ -977,15 +972,12 @@ cudaError_t sort_stars(const Launch &L, TreeBufs &b, int64_t n, const double *px
     }
     const int32_t nsys = b.nsys;
     const unsigned zb = blocks_for(b.lb_words > nsys ? b.lb_words : nsys, kThreads);
-    k_sys_init<<<zb < blocks_for(nsys, kThreads) ? blocks_for(nsys, kThreads) : zb, kThreads, 0, s>>>(
-        nsys, b.geo, b.info, theta, b.lb_state, b.lb_words);
-    SORT_LAUNCH_CHECK();
+    GBH_LAUNCH_AFTER(L, k_sys_init, std::max(zb, blocks_for(nsys, kThreads)), kThreads, nsys, b.geo, b.info, theta,
+                     b.lb_state, b.lb_words);
     if (forest->ntiles < 1) return cudaErrorInvalidValue;
-    k_bbox_sys<<<unsigned(forest->ntiles), kThreads, 0, s>>>(forest->tiles, forest->sys_off, px, py, pz, mass, kind,
-                                                             alive, b.geo, ax, ay, az);
-    SORT_LAUNCH_CHECK();
-    k_sys_cube<<<blocks_for(nsys, 4), 128, 0, s>>>(nsys, theta, b.geo);
-    SORT_LAUNCH_CHECK();
+    GBH_LAUNCH_AFTER(L, k_bbox_sys, unsigned(forest->ntiles), kThreads, forest->tiles, forest->sys_off, px, py, pz,
+                     mass, kind, alive, b.geo, ax, ay, az);
+    GBH_LAUNCH_AFTER(L, k_sys_cube, blocks_for(nsys, 4), 128, nsys, theta, b.geo);
     return run_sort<true>(L, n, px, py, pz, mass, kind, alive, forest->tiles, forest->ntiles, forest->most,
                           forest->sys_off, nsys, b.group == 32 ? 32 : 64, b.keys, b.keys_alt, b.order, b.order_alt,
                           b.tile_len, b.tile_len + b.cap_tiles, b.pos4, b.info, b.geo, out);
@@ -1027,9 +1019,8 @@ cudaError_t morton_sort(const Launch &L, int64_t n, const double *px, const doub
     if (e != cudaSuccess || n == 0) return e;
     unsigned nb = blocks_for(n, kThreads);
     if (nb > unsigned(kBboxBlocks)) nb = kBboxBlocks;
-    k_bbox<<<nb, kThreads, 0, L.stream>>>(n, px, py, pz, nullptr, kind, alive, 0.9, part, nullptr, nullptr, nullptr,
-                                          nullptr, 0, info, nullptr);
-    SORT_LAUNCH_CHECK();
+    GBH_LAUNCH_AFTER(L, k_bbox, nb, kThreads, n, px, py, pz, nullptr, kind, alive, 0.9, part, nullptr, nullptr, nullptr,
+                     nullptr, 0, info, nullptr);
     return run_sort<false>(L, n, px, py, pz, nullptr, kind, alive, nullptr, ntiles, ntiles, nullptr, 1, 64, keys, keys_alt,
                            order, order_alt, len, len_alt, nullptr, info, nullptr, SortedOut{});
 }

@@ -262,6 +262,7 @@ __global__ __launch_bounds__(kChainThreads) void k_chains(const uint64_t *__rest
                                                           uint32_t *__restrict__ pre_info,
                                                           uint32_t *__restrict__ pre_mask, uint32_t *lb,
                                                           int64_t cap_nodes) {
+    pdl_begin();
     __shared__ uint32_t s_warp[kChainThreads / 32 + 1];
     __shared__ uint32_t s_tile, s_prefix;
     if (threadIdx.x == 0) s_tile = atomicAdd(lb, 1u);
@@ -326,6 +327,7 @@ __global__ __launch_bounds__(kThreads) void k_topology(const uint64_t *__restric
                                                        int32_t *__restrict__ pre_parent, int32_t *__restrict__ pre_hi,
                                                        const int32_t *__restrict__ sid_sorted,
                                                        const SysGeo *__restrict__ geo, int64_t cap_nodes) {
+    pdl_begin();
     const int64_t n = info->nstars, nn = info->nnodes < cap_nodes ? info->nnodes : cap_nodes;
     for (int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < nn; p += int64_t(gridDim.x) * blockDim.x) {
         const int64_t i = pre_star[p];
@@ -360,6 +362,7 @@ inline int64_t child_tiles(int64_t cap_nodes) { return (cap_nodes + kScanTile - 
 __global__ __launch_bounds__(kScanThreads) void k_child_scan(const uint32_t *__restrict__ pre_mask,
                                                              uint32_t *__restrict__ child_base, int64_t cap_nodes,
                                                              uint32_t *lb, DevInfo *info) {
+    pdl_begin();
     __shared__ uint32_t s_warp[kScanThreads / 32 + 1];
     __shared__ uint32_t s_tile, s_prefix;
     if (threadIdx.x == 0) s_tile = atomicAdd(lb, 1u);
@@ -405,6 +408,7 @@ __global__ __launch_bounds__(kThreads) void k_emit_nodes(DevInfo *info, const ui
                                                          int32_t *__restrict__ leaves,
                                                          const int32_t *__restrict__ sid_sorted,
                                                          const SysGeo *__restrict__ geo, int64_t cap_nodes) {
+    pdl_begin();
     const int64_t n = info->nstars, nn = info->nnodes < cap_nodes ? info->nnodes : cap_nodes;
     const int lane = threadIdx.x & 31;
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
@@ -754,6 +758,7 @@ __global__ __launch_bounds__(kFp64Threads) void k_walk_fp64(const DevInfo *info,
 __global__ __launch_bounds__(kThreads) void k_kick(int64_t n, double h, double *vx, double *vy, double *vz,
                                                    const double *__restrict__ ax, const double *__restrict__ ay,
                                                    const double *__restrict__ az) {
+    pdl_begin();
     int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     vx[i] += h * ax[i];
@@ -767,6 +772,7 @@ __global__ __launch_bounds__(kThreads) void k_kick_drift(int64_t n, double h, do
                                                          double *py, double *pz, double *vx, double *vy, double *vz,
                                                          const double *__restrict__ ax, const double *__restrict__ ay,
                                                          const double *__restrict__ az) {
+    pdl_begin();
     int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double x = vx[i] + h * ax[i], y = vy[i] + h * ay[i], z = vz[i] + h * az[i];
@@ -1086,6 +1092,7 @@ namespace {
 // mixed walk's group table; a block a system.
 __global__ __launch_bounds__(128) void k_sys_groups(int32_t gsize, const uint32_t *__restrict__ base, SysGeo *geo,
                                                     int4 *__restrict__ groups) {
+    pdl_begin();
     SysGeo &g = geo[blockIdx.x];
     const int32_t lo = g.star_lo, hi = g.star_hi, glo = g.group_lo, ng = g.ngroups;
     const int32_t root = hi > lo ? int32_t(base[lo]) : -1;
@@ -1233,23 +1240,19 @@ cudaError_t tree_build(const Launch &L, TreeBufs &b, int64_t n, const double *px
     if (e != cudaSuccess) return e;
     // node set
     const int32_t *sid = forest ? b.sid_sorted : nullptr;
-    k_chains<<<unsigned(chain_tiles(n)), kChainThreads, 0, s>>>(b.keys, b.info, sid, b.geo, leaf, b.chain_base, b.pre_star,
-                                                                b.pre_info, b.pre_mask, b.lb_state, b.cap_nodes);
-    GBH_LAUNCH_CHECK();
+    GBH_LAUNCH_AFTER(L, k_chains, unsigned(chain_tiles(n)), kChainThreads, b.keys, b.info, sid, b.geo, leaf,
+                     b.chain_base, b.pre_star, b.pre_info, b.pre_mask, b.lb_state, b.cap_nodes);
     const unsigned nbn = node_blocks(b.cap_nodes);
-    k_topology<<<nbn, kThreads, 0, s>>>(b.keys, b.info, b.chain_base, b.pre_star, b.pre_info, b.pre_mask, b.pre_parent,
-                                        b.pre_hi, sid, b.geo, b.cap_nodes);
-    GBH_LAUNCH_CHECK();
-    k_child_scan<<<unsigned(child_tiles(b.cap_nodes)), kScanThreads, 0, s>>>(
-        b.pre_mask, b.child_base, b.cap_nodes, b.lb_state + lb_words_of(chain_tiles(b.cap_n)), b.info);
-    GBH_LAUNCH_CHECK();
-    k_emit_nodes<<<nbn, kThreads, 0, s>>>(b.info, b.chain_base, b.pre_star, b.pre_parent, b.pre_info, b.pre_mask, b.pre_hi,
-                                          b.child_base, b.nodes, b.n_parent, b.n_info, b.n_arrive, b.leaves, sid, b.geo,
-                                          b.cap_nodes);
-    GBH_LAUNCH_CHECK();
+    GBH_LAUNCH_AFTER(L, k_topology, nbn, kThreads, b.keys, b.info, b.chain_base, b.pre_star, b.pre_info, b.pre_mask,
+                     b.pre_parent, b.pre_hi, sid, b.geo, b.cap_nodes);
+    GBH_LAUNCH_AFTER(L, k_child_scan, unsigned(child_tiles(b.cap_nodes)), kScanThreads, b.pre_mask, b.child_base,
+                     b.cap_nodes, b.lb_state + lb_words_of(chain_tiles(b.cap_n)), b.info);
+    GBH_LAUNCH_AFTER(L, k_emit_nodes, nbn, kThreads, b.info, b.chain_base, b.pre_star, b.pre_parent, b.pre_info,
+                     b.pre_mask, b.pre_hi, b.child_base, b.nodes, b.n_parent, b.n_info, b.n_arrive, b.leaves, sid,
+                     b.geo, b.cap_nodes);
     if (forest) {
-        k_sys_groups<<<unsigned(b.nsys), 128, 0, s>>>(b.group == 32 ? 32 : 64, b.chain_base, b.geo, b.groups);
-        GBH_LAUNCH_CHECK();
+        GBH_LAUNCH_AFTER(L, k_sys_groups, unsigned(b.nsys), 128, b.group == 32 ? 32 : 64, b.chain_base, b.geo,
+                         b.groups);
     }
     b.moments_exact = exact;
     if (!exact) return upsweep_fast(L, b, plain_records);
@@ -1294,8 +1297,7 @@ cudaError_t walk_fp64(const Launch &L, const TreeBufs &b, int64_t n, double eps2
 cudaError_t kick(const Launch &L, int64_t n, double h, double *vx, double *vy, double *vz, const double *ax,
                  const double *ay, const double *az) {
     if (n == 0) return cudaSuccess;
-    k_kick<<<blocks_for(n, kThreads), kThreads, 0, L.stream>>>(n, h, vx, vy, vz, ax, ay, az);
-    GBH_LAUNCH_CHECK();
+    GBH_LAUNCH_AFTER(L, k_kick, blocks_for(n, kThreads), kThreads, n, h, vx, vy, vz, ax, ay, az);
     return cudaSuccess;
 }
 
@@ -1303,9 +1305,8 @@ cudaError_t kick_drift(const Launch &L, int64_t n, double h, double dt, double c
                        double *vx, double *vy, double *vz, const double *ax, const double *ay, const double *az) {
     if (n == 0) return cudaSuccess;
     const double inv_c2 = c > 0 ? 1 / (c * c) : 0.0;  // sim.go:335 (invC2)
-    k_kick_drift<<<blocks_for(n, kThreads), kThreads, 0, L.stream>>>(n, h, dt, inv_c2, px, py, pz, vx, vy, vz, ax, ay,
-                                                                     az);
-    GBH_LAUNCH_CHECK();
+    GBH_LAUNCH_AFTER(L, k_kick_drift, blocks_for(n, kThreads), kThreads, n, h, dt, inv_c2, px, py, pz, vx, vy, vz, ax, ay,
+                     az);
     return cudaSuccess;
 }
 

@@ -421,6 +421,7 @@ constexpr int kLptThreads = 1024, kLptBuckets = 16, kLptWarps = kLptThreads / 32
 __global__ __launch_bounds__(kLptThreads) void k_lpt_order(const DevInfo *info, int gsize, bool forest,
                                                            const uint32_t *__restrict__ gcost, int32_t *gperm,
                                                            int32_t perm_cap) {
+    pdl_begin();
     __shared__ uint32_t cnt[kLptBuckets][kLptWarps];  // then the positions of each warp's next groups
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int32_t ng = forest ? int32_t(info->ngroups) : int32_t((info->nstars + gsize - 1) / gsize);
@@ -484,6 +485,7 @@ __global__ __launch_bounds__(256) void k_split_combine(const DevInfo *info, cons
                                                        const int32_t *__restrict__ targets, int nparts,
                                                        const double *__restrict__ part_acc, int64_t stride,
                                                        double *ax, double *ay, double *az) {
+    pdl_begin();
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t nt = targets ? int64_t(info->ntargets) : info->nstars;
     if (t >= nt) return;
@@ -539,9 +541,7 @@ static cudaError_t launch_mixed_t(const Launch &L, const TreeBufs &b, int64_t ns
     ++*L.count;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || !lpt) return e;
-    k_lpt_order<<<1, kLptThreads, 0, L.stream>>>(b.info, gsize, forest, b.gcost, b.gperm, int32_t(b.cap_groups));
-    ++*L.count;
-    return cudaGetLastError();
+    return lpt_order(L, b, gsize);
 }
 
 template <bool kQuad, bool kSoft, bool kPot = false>
@@ -554,9 +554,9 @@ static cudaError_t launch_mixed(const Launch &L, const TreeBufs &b, int64_t nsta
 }
 
 cudaError_t lpt_order(const Launch &L, const TreeBufs &b, int gsize) {
-    k_lpt_order<<<1, kLptThreads, 0, L.stream>>>(b.info, gsize, b.nsys > 1, b.gcost, b.gperm, int32_t(b.cap_groups));
-    ++*L.count;
-    return cudaGetLastError();
+    GBH_LAUNCH_AFTER(L, k_lpt_order, 1, kLptThreads, b.info, gsize, b.nsys > 1, b.gcost, b.gperm,
+                     int32_t(b.cap_groups));
+    return cudaSuccess;
 }
 
 // Parts of a split walk of groups of gsize stars (1: no split), for single systems with few groups
@@ -573,10 +573,9 @@ int split_parts(const TreeBufs &b, int64_t nstars_cap, bool targets, int gsize) 
 
 cudaError_t split_combine(const Launch &L, const TreeBufs &b, int nparts, int64_t stride, bool targets, double *ax,
                           double *ay, double *az) {
-    k_split_combine<<<dim3(blocks_for(stride, 256), 3), 256, 0, L.stream>>>(
-        b.info, b.order, targets ? b.targets : nullptr, nparts, b.part_acc, stride, ax, ay, az);
-    ++*L.count;
-    return cudaGetLastError();
+    GBH_LAUNCH_AFTER(L, k_split_combine, dim3(blocks_for(stride, 256), 3), 256, b.info, b.order,
+                     targets ? b.targets : nullptr, nparts, b.part_acc, stride, ax, ay, az);
+    return cudaSuccess;
 }
 
 

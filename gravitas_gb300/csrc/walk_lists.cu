@@ -705,6 +705,7 @@ __global__ __launch_bounds__(kLwThreads, kS == 2 ? 8 : 10) void k_walk_lists(con
                                                            int node_depth, int src_depth, int nparts = 1,
                                                            double *part_acc = nullptr, int64_t part_stride = 0,
                                                            const int2 *__restrict__ ranges = nullptr) {
+    pdl_begin();
     constexpr int kG = 32 * kS;  // stars per group: lane l holds stars l, 32 + l, ...
     __shared__ WarpMem smem[kLwWarps];
     WarpMem &W = smem[threadIdx.x >> 5];
@@ -764,6 +765,13 @@ __global__ __launch_bounds__(kLwThreads, kS == 2 ? 8 : 10) void k_walk_lists(con
     }
 }
 
+// The work counter of a list walk: cleared by the FP32 upsweep of the build before it, or here.
+static cudaError_t clear_ctr(const Launch &L, const TreeBufs &b) {
+    const bool clear = b.ctr_clear;
+    b.ctr_clear = false;
+    return clear ? cudaSuccess : cudaMemsetAsync(b.walk_ctr, 0, sizeof(uint32_t), L.stream);
+}
+
 template <bool kQuad, bool kSoft, int kS, bool kSplit>
 static int lists_blocks_per_sm() {
     static int blocks_per_sm = 0;  // per instantiation; the same on every device of this architecture
@@ -780,7 +788,7 @@ template <bool kQuad, bool kSoft, int kS>
 cudaError_t launch_lists(const Launch &L, const TreeBufs &b, int64_t nstars_cap, float eps2, double *ax, double *ay,
                          double *az, int node_depth, int src_depth, bool lpt, bool targets, bool &split) {
     const bool forest = b.nsys > 1;
-    cudaError_t e = cudaMemsetAsync(b.walk_ctr, 0, sizeof(uint32_t), L.stream);
+    cudaError_t e = clear_ctr(L, b);
     if (e != cudaSuccess) return e;
     const int sms = L.num_sms > 0 ? L.num_sms : 152;
     if constexpr (kQuad && kSoft) {
@@ -791,24 +799,20 @@ cudaError_t launch_lists(const Launch &L, const TreeBufs &b, int64_t nstars_cap,
         if (split) {
             const int bps = lists_blocks_per_sm<kQuad, kSoft, kS, true>();
             if (!bps) return cudaErrorUnknown;
-            k_walk_lists<kQuad, kSoft, kS, true><<<unsigned(sms * bps), kLwThreads, 0, L.stream>>>(
-                b.info, b.lnode, b.st_hi, b.st_lo, b.order, sqrtf(eps2), eps2, ax, ay, az, nullptr,
-                targets ? b.targets : nullptr, nullptr, int32_t(b.cap_groups), nullptr, b.walk_ctr, b.info,
-                node_depth, src_depth, parts, b.part_acc, nstars_cap, b.mrange);
-            ++*L.count;
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            GBH_LAUNCH_AFTER(L, (k_walk_lists<kQuad, kSoft, kS, true>), unsigned(sms * bps), kLwThreads, b.info, b.lnode,
+                             b.st_hi, b.st_lo, b.order, sqrtf(eps2), eps2, ax, ay, az, nullptr,
+                             targets ? b.targets : nullptr, nullptr, int32_t(b.cap_groups), nullptr, b.walk_ctr,
+                             b.info, node_depth, src_depth, parts, b.part_acc, nstars_cap, b.mrange);
             return split_combine(L, b, parts, nstars_cap, targets, ax, ay, az);
         }
     }
     const int bps = lists_blocks_per_sm<kQuad, kSoft, kS, false>();
     if (!bps) return cudaErrorUnknown;
-    k_walk_lists<kQuad, kSoft, kS><<<unsigned(sms * bps), kLwThreads, 0, L.stream>>>(
-        b.info, b.lnode, b.st_hi, b.st_lo, b.order, sqrtf(eps2), eps2, ax, ay, az,
-        forest ? b.groups : nullptr, targets ? b.targets : nullptr, lpt ? b.gperm : nullptr, int32_t(b.cap_groups),
-        lpt ? b.gcost : nullptr,
-        b.walk_ctr, b.info, node_depth, src_depth);
-    ++*L.count;
-    return cudaGetLastError();
+    GBH_LAUNCH_AFTER(L, (k_walk_lists<kQuad, kSoft, kS>), unsigned(sms * bps), kLwThreads, b.info, b.lnode, b.st_hi,
+                     b.st_lo, b.order, sqrtf(eps2), eps2, ax, ay, az, forest ? b.groups : nullptr,
+                     targets ? b.targets : nullptr, lpt ? b.gperm : nullptr, int32_t(b.cap_groups),
+                     lpt ? b.gcost : nullptr, b.walk_ctr, b.info, node_depth, src_depth, 1, nullptr, 0, nullptr);
+    return cudaSuccess;
 }
 
 template <int kS>
@@ -1412,7 +1416,7 @@ static cudaError_t launch_pot(const Launch &L, const TreeBufs &b, float eps2, do
             return e;
         if (blocks_per_sm < 1) blocks_per_sm = 1;
     }
-    if ((e = cudaMemsetAsync(b.walk_ctr, 0, sizeof(uint32_t), L.stream))) return e;
+    if ((e = clear_ctr(L, b))) return e;
     const int sms = L.num_sms > 0 ? L.num_sms : 152;
     k_walk_lists_pot<kQuad, true, 2><<<unsigned(sms * blocks_per_sm), kLwThreads, 0, L.stream>>>(
         b.info, b.lnode, b.st_hi, b.st_lo, sqrtf(eps2), eps2, psi, b.nsys > 1 ? b.groups : nullptr, b.walk_ctr,
@@ -1470,7 +1474,7 @@ cudaError_t walk_lists_adjoint(const Launch &L, const TreeBufs &b, float eps2, c
     if ((e = cudaMemsetAsync(s.nadj, 0, sizeof(double) * kAdjNodeTerms * size_t(b.cap_nodes), L.stream))) return e;
     if ((e = cudaMemsetAsync(s.sadj, 0, sizeof(double) * kAdjStarTerms * size_t(b.cap_n), L.stream))) return e;
     if ((e = cudaMemsetAsync(s.star_leaf, 0xff, sizeof(int32_t) * size_t(b.cap_n), L.stream))) return e;
-    if ((e = cudaMemsetAsync(b.walk_ctr, 0, sizeof(uint32_t), L.stream))) return e;
+    if ((e = clear_ctr(L, b))) return e;
     // few groups: each group's walk shared among several warps, as the forward's (walk_lists)
     if ((e = b.group == 64 ? launch_adj<2>(L, b, n, eps2, wx, wy, wz, s) : launch_adj<1>(L, b, n, eps2, wx, wy, wz, s)))
         return e;
