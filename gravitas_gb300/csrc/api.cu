@@ -99,7 +99,8 @@ struct gbh_ctx {
     int64_t launches = 0;
     int64_t h2d = 0, d2h = 0;
     int64_t last_substeps = 1;  // substeps of the last hole-aware step
-    DevInfo info_host = {};
+    DevInfo *info_host = nullptr;  // page-locked
+    cudaEvent_t info_ev = nullptr; // the end of a copy into it (block steps)
     gbh_timings last = {};
     std::string err;
 };
@@ -364,7 +365,7 @@ int forces(gbh_ctx *ctx, const gbh_params *p, int64_t n, const double *px, const
 
 // The status of a device-side check recorded in the DevInfo the host has read back.
 int info_status(gbh_ctx *ctx) {
-    const DevInfo &i = ctx->info_host;
+    const DevInfo &i = *ctx->info_host;
     if (!i.err) return GBH_OK;
     if (i.err_where == gbh::kErrNonFinite)
         return fail(ctx, GBH_ERR_ARG, "an alive star has a non-finite position or mass (outputs are undefined)");
@@ -375,7 +376,7 @@ int info_status(gbh_ctx *ctx) {
 int finish(gbh_ctx *ctx, bool tree) {
     CK(cudaEventRecord(ctx->ev[5], ctx->stream));
     if (tree && ctx->tb.info) {
-        CK(cudaMemcpyAsync(&ctx->info_host, ctx->tb.info, sizeof(DevInfo), cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaMemcpyAsync(ctx->info_host, ctx->tb.info, sizeof(DevInfo), cudaMemcpyDeviceToHost, ctx->stream));
     }
     CK(wait_stream(ctx));
     float ms = 0;
@@ -391,8 +392,8 @@ int finish(gbh_ctx *ctx, bool tree) {
     t.h2d_bytes = ctx->h2d;
     t.d2h_bytes = ctx->d2h;
     if (tree) {
-        t.nstars = ctx->info_host.nstars;
-        t.nnodes = ctx->info_host.nnodes;
+        t.nstars = ctx->info_host->nstars;
+        t.nnodes = ctx->info_host->nnodes;
         return info_status(ctx);
     }
     return GBH_OK;
@@ -595,24 +596,31 @@ int run_steps(gbh_ctx *ctx, const gbh_params *p, double dt, int64_t nsteps) {
     return GBH_OK;
 }
 
-// Forces on the stars whose step ends at tick (block steps): tree of all stars, walk of the
-// active ones only.
-int forces_active(gbh_ctx *ctx, const gbh_params *p, const uint8_t *kind, const uint8_t *alive, const int32_t *end,
-                  int32_t tick) {
+// A block step's event in two parts. The drift of all bodies from tick t to the event's tick (which
+// the device knows) and the tree of all stars ...
+int event_build(gbh_ctx *ctx, const gbh_params *p, const uint8_t *kind, const uint8_t *alive, int32_t t, double tick_len) {
     Launch L = launch_of(ctx);
     int leaf = leaf_of(p);
     int64_t n = ctx->n;
     CK(gbh::tree_alloc(ctx->tb, n, leaf));
+    CK(gbh::block_drift(L, ctx->tb, n, t, tick_len, p->c, ctx->px, ctx->py, ctx->pz, ctx->vx, ctx->vy, ctx->vz));
     ctx->tb.group = group_of(p, n, false);  // as the global step, so that one level is that step
     ctx->tb.list_depth = p->list_depth;
     ctx->tb.lpt = ctx->use_lpt;
     ctx->tb.split = ctx->use_split;
     ctx->tb.paired = ctx->use_paired;
-    ctx->tb.walk_hint = ctx->active_hint;  // this event's list is not known on the host yet
     CK(stage_event(ctx));
     CK(gbh::tree_build(L, ctx->tb, n, ctx->px, ctx->py, ctx->pz, ctx->mass, kind, alive, ctx->ax, ctx->ay, ctx->az,
                        theta_of(p), leaf, p->dark_matter_off, p->walk == GBH_WALK_FP64, p->walk == GBH_WALK_PLAIN));
-    CK(gbh::select_targets(L, ctx->tb, end, tick));
+    return GBH_OK;
+}
+
+// ... and the forces on the stars whose step ends at tick (about active_hint of them).
+int event_walk(gbh_ctx *ctx, const gbh_params *p, const int32_t *end, int32_t tick) {
+    Launch L = launch_of(ctx);
+    int64_t n = ctx->n;
+    ctx->tb.walk_hint = ctx->active_hint;
+    CK(gbh::select_targets(L, ctx->tb, n, end, tick));
     CK(stage_event(ctx));
     double eps2 = p->softening * p->softening;
     int quad = !p->monopole_only;
@@ -632,14 +640,26 @@ int forces_active(gbh_ctx *ctx, const gbh_params *p, const uint8_t *kind, const 
     return GBH_OK;
 }
 
-// Reads the device scalars (next event tick, active count) after the work issued so far.
-int read_info(gbh_ctx *ctx) {
-    CK(cudaMemcpyAsync(&ctx->info_host, ctx->tb.info, sizeof(DevInfo), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(wait_stream(ctx));
+// Issues the copy of the device scalars (next event tick, its bodies, active count) ...
+int copy_info(gbh_ctx *ctx) {
+    CK(cudaMemcpyAsync(ctx->info_host, ctx->tb.info, sizeof(DevInfo), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaEventRecord(ctx->info_ev, ctx->stream));
+    return GBH_OK;
+}
+
+// ... and waits for it, not for the work issued after it. Sizes the next event's walk (split or not)
+// by the bodies due at its tick.
+int wait_info(gbh_ctx *ctx) {
+    CK(cudaEventSynchronize(ctx->info_ev));
+    if (ctx->info_host->next_count > 0) ctx->active_hint = int64_t(ctx->info_host->next_count);
     return info_status(ctx);
 }
 
-// Block-step KDK on the resident state (see block_open in tree.cu for the scheme).
+// Block-step KDK on the resident state (see block_open in tree.cu for the scheme). The host reads
+// each next event's tick and body count to size that event's walk; the event's drift and tree build
+// need neither, so they are issued before the host waits, and run meanwhile: the 131,072-body
+// galaxy's block step of 8 events took 4.44 ms with the wait first (and five
+// more launches an event), 4.20 ms so.
 int run_block_steps(gbh_ctx *ctx, const gbh_params *p, double T, double eta, int levels, int64_t nsteps,
                     gbh_blockstats *st) {
     Launch L = launch_of(ctx);
@@ -647,7 +667,7 @@ int run_block_steps(gbh_ctx *ctx, const gbh_params *p, double T, double eta, int
     const uint8_t *kind = ctx->state_has_kind ? ctx->kind : nullptr;
     const uint8_t *alive = ctx->state_has_alive ? ctx->alive : nullptr;
     const int32_t ticks = 1 << (levels - 1);
-    const double eps = p->softening;
+    const double eps = p->softening, tick_len = T / double(ticks);
     CK(grow(ctx->rung, ctx->rung_cap, n));
     CK(grow(ctx->end_tick, ctx->end_cap, n));
     if (!ctx->acc_valid) {  // initForces (gas.go:14-17)
@@ -662,27 +682,25 @@ int run_block_steps(gbh_ctx *ctx, const gbh_params *p, double T, double eta, int
     for (int64_t s = 0; s < nsteps; ++s) {
         CK(gbh::block_open(L, ctx->tb, n, T, levels, eta, eps, ctx->ax, ctx->ay, ctx->az, ctx->vx, ctx->vy, ctx->vz,
                            ctx->rung, ctx->end_tick));
-        if ((rc = read_info(ctx))) return rc;
-        if (ctx->info_host.next_count > 0) ctx->active_hint = int64_t(ctx->info_host.next_count);
         int32_t t = 0;
         while (t < ticks) {
-            int32_t tn = ctx->info_host.next_tick;
+            if ((rc = copy_info(ctx)) || (rc = event_build(ctx, p, kind, alive, t, tick_len)) || (rc = wait_info(ctx)))
+                return rc;
+            const int32_t tn = ctx->info_host->next_tick;
+            if (st && t > 0) st->evaluations += ctx->info_host->ntargets;  // of the event before
             if (tn <= t || tn > ticks) return fail(ctx, GBH_ERR_LIMIT, "block steps: next event %d after %d", tn, t);
-            if (st && (st->min_substep_ticks == 0 || tn - t < st->min_substep_ticks)) st->min_substep_ticks = tn - t;
-            CK(gbh::block_drift(L, n, double(tn - t) * (T / double(ticks)), p->c, ctx->px, ctx->py, ctx->pz, ctx->vx,
-                                ctx->vy, ctx->vz));
+            if (st) {
+                if (st->min_substep_ticks == 0 || tn - t < st->min_substep_ticks) st->min_substep_ticks = tn - t;
+                st->substeps += 1;
+            }
             t = tn;
-            if ((rc = forces_active(ctx, p, kind, alive, ctx->end_tick, t))) return rc;
+            if ((rc = event_walk(ctx, p, ctx->end_tick, t))) return rc;
             CK(gbh::block_close(L, ctx->tb, n, t, T, levels, eta, eps, ctx->ax, ctx->ay, ctx->az, ctx->vx, ctx->vy,
                                 ctx->vz, ctx->rung, ctx->end_tick));
-            if ((rc = read_info(ctx))) return rc;
-            // the next event walks the bodies due at its tick: size its walk (split or not) by them
-            if (ctx->info_host.next_count > 0) ctx->active_hint = int64_t(ctx->info_host.next_count);
-            if (st) {
-                st->substeps += 1;
-                st->evaluations += ctx->info_host.ntargets;
-            }
         }
+        // the step's last event: its count for the statistics, and its errors
+        if ((rc = copy_info(ctx)) || (rc = wait_info(ctx))) return rc;
+        if (st) st->evaluations += ctx->info_host->ntargets;
     }
     return GBH_OK;
 }
@@ -799,6 +817,14 @@ int gbh_create(const gbh_config *cfg, gbh_ctx **out, char *err, int errlen) {
             return report(GBH_ERR_CUDA, cudaGetErrorString(e));
         }
     }
+    const unsigned info_flags =
+        cudaEventDisableTiming | (cfg && (cfg->flags & GBH_CFG_BLOCKING_SYNC) ? cudaEventBlockingSync : 0u);
+    if ((e = cudaEventCreateWithFlags(&c->info_ev, info_flags)) != cudaSuccess ||
+        (e = cudaMallocHost(&c->info_host, sizeof(DevInfo))) != cudaSuccess) {
+        gbh_destroy(c);
+        return report(e == cudaErrorMemoryAllocation ? GBH_ERR_NOMEM : GBH_ERR_CUDA, cudaGetErrorString(e));
+    }
+    std::memset(static_cast<void *>(c->info_host), 0, sizeof(DevInfo));
     if ((e = cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&c->copy_done, cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming)) != cudaSuccess) {
@@ -826,6 +852,8 @@ void gbh_destroy(gbh_ctx *c) {
         if (ev) cudaEventDestroy(ev);
     for (auto &ev : c->evpool) cudaEventDestroy(ev);
     if (c->wait_ev) cudaEventDestroy(c->wait_ev);
+    if (c->info_ev) cudaEventDestroy(c->info_ev);
+    if (c->info_host) cudaFreeHost(c->info_host);
     if (c->copy_stream) {
         cudaStreamSynchronize(c->copy_stream);
         cudaStreamDestroy(c->copy_stream);
@@ -1061,7 +1089,10 @@ int gbh_state_step_block(gbh_ctx *ctx, const gbh_params *p, double dt, double et
     if (ctx->nsys > 1) return fail(ctx, GBH_ERR_UNSUPPORTED, "block steps of a forest are not supported");
     if (stats) *stats = gbh_blockstats{};
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-    if (ctx->n > 0 && (rc = run_block_steps(ctx, p, dt, eta, levels, nsteps, stats))) return rc;
+    if (ctx->n > 0 && (rc = run_block_steps(ctx, p, dt, eta, levels, nsteps, stats))) {
+        cudaStreamSynchronize(ctx->stream);  // work issued ahead of the failed check
+        return rc;
+    }
     return finish(ctx, ctx->n > 0);
 }
 
@@ -1194,7 +1225,7 @@ int gbh_forest_layout(gbh_ctx *ctx, int32_t nsys, int64_t *star_range, int64_t *
     if (nsys != ctx->tb.nsys) return fail(ctx, GBH_ERR_ARG, "the last tree has %d systems", ctx->tb.nsys);
     std::vector<gbh::SysGeo> geo(static_cast<size_t>(nsys));
     CK(cudaMemcpy(geo.data(), ctx->tb.geo, sizeof(gbh::SysGeo) * size_t(nsys), cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(&ctx->info_host, ctx->tb.info, sizeof(DevInfo), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(ctx->info_host, ctx->tb.info, sizeof(DevInfo), cudaMemcpyDeviceToHost));
     for (int32_t q = 0; q < nsys; ++q) {
         if (star_range) {
             star_range[2 * q] = geo[size_t(q)].star_lo;
@@ -1203,7 +1234,7 @@ int gbh_forest_layout(gbh_ctx *ctx, int32_t nsys, int64_t *star_range, int64_t *
         if (node_range) {
             int64_t lo = geo[size_t(q)].root, hi = lo;
             if (lo >= 0) {  // the next non-empty system's root, or the end of the table
-                hi = ctx->info_host.nnodes;
+                hi = ctx->info_host->nnodes;
                 for (int32_t r = q + 1; r < nsys; ++r)
                     if (geo[size_t(r)].root >= 0) {
                         hi = geo[size_t(r)].root;
@@ -1223,9 +1254,9 @@ int gbh_tree_size(gbh_ctx *ctx, int64_t *nstars, int64_t *nnodes) {
     int rc = begin(ctx);
     if (rc) return rc;
     if (!ctx->tb.info) return fail(ctx, GBH_ERR_STATE, "no tree built yet");
-    CK(cudaMemcpy(&ctx->info_host, ctx->tb.info, sizeof(DevInfo), cudaMemcpyDeviceToHost));
-    if (nstars) *nstars = ctx->info_host.nstars;
-    if (nnodes) *nnodes = ctx->info_host.nnodes;
+    CK(cudaMemcpy(ctx->info_host, ctx->tb.info, sizeof(DevInfo), cudaMemcpyDeviceToHost));
+    if (nstars) *nstars = ctx->info_host->nstars;
+    if (nnodes) *nnodes = ctx->info_host->nnodes;
     return GBH_OK;
 }
 
@@ -1234,8 +1265,8 @@ int gbh_tree_export(gbh_ctx *ctx, uint64_t *keys, int32_t *order, gbh_node *node
     int rc = begin(ctx);
     if (rc) return rc;
     if (!ctx->tb.info) return fail(ctx, GBH_ERR_STATE, "no tree built yet");
-    CK(cudaMemcpy(&ctx->info_host, ctx->tb.info, sizeof(DevInfo), cudaMemcpyDeviceToHost));
-    int64_t ns = ctx->info_host.nstars, nn = ctx->info_host.nnodes;
+    CK(cudaMemcpy(ctx->info_host, ctx->tb.info, sizeof(DevInfo), cudaMemcpyDeviceToHost));
+    int64_t ns = ctx->info_host->nstars, nn = ctx->info_host->nnodes;
     if (keys && ns) CK(cudaMemcpy(keys, ctx->tb.keys, sizeof(uint64_t) * size_t(ns), cudaMemcpyDeviceToHost));
     if (order && ns) CK(cudaMemcpy(order, ctx->tb.order, sizeof(int32_t) * size_t(ns), cudaMemcpyDeviceToHost));
     int64_t cnt = std::min(nn, node_cap);

@@ -44,6 +44,7 @@ struct DevInfo {
     int32_t next_tick;        // block steps: the earliest step end over all bodies
     uint32_t next_count;      // block steps: the bodies whose step ends at next_tick
     uint32_t bbox_done;       // blocks of k_bbox that have finished (wraps to 0 by itself)
+    uint32_t next_done;       // the same of the kernels that find next_tick
     // FP32 views for the FP32 upsweep: min corner and side as hi + lo pairs, and the
     // opening base 2 * half_L / theta per level L
     float min_hi[3], min_lo[3];
@@ -101,7 +102,6 @@ struct TreeBufs {
     int32_t group = 64;     // stars per mixed-walk group (32: the list walk, or 64), set before tree_build
     int32_t list_depth = 0; // the list walk's node-list depth (0: kDefaultListDepth), set per call
     // compaction / bbox
-    uint32_t *flag = nullptr;     // active flags of a block step's event, then their exclusive scan
     Pos4 *pos4 = nullptr;         // (x, y, z, m) of every star in state order, one 32-byte record
     long long *bbox_part = nullptr;  // per-block parts of the bounding box
     // sort
@@ -111,7 +111,7 @@ struct TreeBufs {
     int64_t cap_tiles = 0;
     // single-pass scans: tile counters and look-back words (cleared by the build's first kernel)
     uint32_t *lb_state = nullptr;
-    int64_t lb_words = 0, lb_sort = 0;  // lb_sort: where the large sort's words start
+    int64_t lb_words = 0, lb_targets = 0, lb_sort = 0;  // where the active-star lists' and the large sort's start
     uint32_t *hist = nullptr;           // digit table of the large sort's radix passes
     // sorted stars
     double *sx = nullptr, *sy = nullptr, *sz = nullptr, *sm = nullptr;
@@ -161,9 +161,7 @@ struct TreeBufs {
     bool paired = false;            // 64-star groups take the paired walk (set per call)
     int64_t walk_hint = 0;          // a target-list walk's expected list length (0: the body count)
     bool moments_exact = false;     // the last build ran the bit-exact FP64 upsweep
-    // scan temporaries
-    uint32_t *scan_tmp = nullptr;
-    int64_t scan_tmp_cap = 0;
+    unsigned long long *next_part = nullptr;  // blocks' parts of a block step's next event
     DevInfo *info = nullptr;
 };
 
@@ -232,14 +230,15 @@ cudaError_t sort_stars(const Launch &L, TreeBufs &b, int64_t n, const double *px
 size_t sort_part_bytes();              // of bbox_part
 int64_t sort_lb_words(int64_t n);      // look-back words of a sort of up to n bodies
 int64_t sort_hist_words(int64_t n);    // digit table words of the same
-// Block time steps (see tree.cu): tick-0 opening kicks and rungs, drift of all bodies, and the
-// closing/opening kicks of the bodies whose step ends at tick. DevInfo.next_tick receives the
-// earliest step end over all bodies.
+// Block time steps (see tree.cu): tick-0 opening kicks and rungs, drift of all bodies from tick t to
+// DevInfo.next_tick (ticks of tick_len), and the
+// closing/opening kicks of the bodies whose step ends at tick. DevInfo.next_tick and next_count
+// receive the earliest step end over all bodies and the bodies that end there.
 cudaError_t block_open(const Launch &L, const TreeBufs &b, int64_t n, double T, int levels, double eta, double eps,
                        const double *ax, const double *ay, const double *az, double *vx, double *vy, double *vz,
                        uint8_t *rung, int32_t *end);
-cudaError_t block_drift(const Launch &L, int64_t n, double dt, double c, double *px, double *py, double *pz, const double *vx,
-                        const double *vy, const double *vz);
+cudaError_t block_drift(const Launch &L, const TreeBufs &b, int64_t n, int32_t t, double tick_len, double c, double *px,
+                        double *py, double *pz, const double *vx, const double *vy, const double *vz);
 cudaError_t block_close(const Launch &L, const TreeBufs &b, int64_t n, int32_t tick, double T, int levels, double eta,
                         double eps, const double *ax, const double *ay, const double *az, double *vx, double *vy,
                         double *vz, uint8_t *rung, int32_t *end);
@@ -283,7 +282,7 @@ cudaError_t export_fast_moments(const Launch &L, TreeBufs &b);
 cudaError_t walk_fp64(const Launch &L, const TreeBufs &b, int64_t n, double eps2, int quad,
                       double *ax, double *ay, double *az, bool targets = false);
 // Lists in b.targets the sorted positions whose body has end[order[k]] == tick.
-cudaError_t select_targets(const Launch &L, TreeBufs &b, const int32_t *end, int32_t tick);
+cudaError_t select_targets(const Launch &L, TreeBufs &b, int64_t n, const int32_t *end, int32_t tick);
 cudaError_t kick(const Launch &L, int64_t n, double h, double *vx, double *vy, double *vz,
                  const double *ax, const double *ay, const double *az);
 cudaError_t kick_drift(const Launch &L, int64_t n, double h, double dt, double c, double *px, double *py,

@@ -157,6 +157,7 @@ __global__ __launch_bounds__(kThreads) void k_bbox(int64_t n, const double *__re
         info->nnodes = 0;
         info->work = 0;
         info->nleaves = 0;
+        info->ntargets = 0;
         info->theta = theta;
     }
     const int64_t stride = int64_t(gridDim.x) * kThreads, t0 = int64_t(blockIdx.x) * kThreads + threadIdx.x;
@@ -224,6 +225,7 @@ __global__ void k_sys_init(int32_t nsys, SysGeo *geo, DevInfo *info, double thet
         info->nnodes = 0;
         info->work = 0;
         info->nleaves = 0;
+        info->ntargets = 0;
         info->theta = theta;
     }
     if (s >= nsys) return;

@@ -310,6 +310,11 @@ __global__ __launch_bounds__(kChainThreads) void k_chains(const uint64_t *__rest
     }
 }
 
+constexpr int kNextBlocks = 1024;  // most blocks of the kernels that find a block step's next event
+// Tiles of the active-star lists (block steps).
+constexpr int kTargetThreads = 256, kTargetItems = 4, kTargetTile = kTargetThreads * kTargetItems;
+inline int64_t target_tiles(int64_t n) { return (n + kTargetTile - 1) / kTargetTile; }
+
 // Grid of the per-node kernels below: they loop over the nodes, whose count only the device knows.
 inline unsigned node_blocks(int64_t cap_nodes) {
     const unsigned nb = blocks_for(cap_nodes, kThreads);
@@ -1115,15 +1120,10 @@ cudaError_t scan_u32(const Launch &L, const uint32_t *in, uint32_t *out, int64_t
     return scan_rec(L, in, out, n, nullptr, tmp, tmp_cap);
 }
 
-static cudaError_t scan_dyn(const Launch &L, const uint32_t *in, uint32_t *out, int64_t n, const int64_t *ndyn,
-                            uint32_t *tmp, int64_t tmp_cap) {
-    return scan_rec(L, in, out, n, ndyn, tmp, tmp_cap);
-}
-
 void tree_free(TreeBufs &b) {
-    void *ptrs[] = {b.flag, b.pos4, b.bbox_part, b.keys, b.keys_alt, b.order, b.order_alt, b.lb_state, b.tile_len, b.hist, b.sx, b.sy, b.sz, b.sm,
+    void *ptrs[] = {b.pos4, b.bbox_part, b.keys, b.keys_alt, b.order, b.order_alt, b.lb_state, b.tile_len, b.hist, b.sx, b.sy, b.sz, b.sm,
                     b.st_hi, b.st_lo, b.st_off, b.chain_base, b.leaves, b.targets, b.geo, b.sid_sorted, b.groups, b.gcost, b.gperm, b.pre_parent, b.pre_info, b.child_base, b.pre_mask, b.pre_hi, b.pre_star, b.nodes,
-                    b.n_parent, b.n_info, b.n_arrive, b.pnodes, b.mnodes, b.mrange, b.lnode, b.walk_ctr, b.scan_tmp, b.info, b.part_acc};
+                    b.n_parent, b.n_info, b.n_arrive, b.pnodes, b.mnodes, b.mrange, b.lnode, b.walk_ctr, b.next_part, b.info, b.part_acc};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     b = TreeBufs{};
@@ -1148,14 +1148,11 @@ cudaError_t tree_alloc(TreeBufs &b, int64_t n, int leaf, int32_t nsys) {
     tree_free(b);
     b.generation = gen;
     cn = cn < 1 ? 1 : cn;
-    int64_t scan_cap = scan_tmp_size(cnodes > cn * 1 ? cnodes : cn);
-    b.scan_tmp_cap = scan_cap;
     cudaError_t e = cudaSuccess;
 #define GBH_ALLOC(ptr, count)                                                     \
     do {                                                                          \
         if (e == cudaSuccess) e = dev_alloc(&(ptr), sizeof(*(ptr)) * size_t(count)); \
     } while (0)
-    GBH_ALLOC(b.flag, cn);
     GBH_ALLOC(b.pos4, cn);
     if (e == cudaSuccess) e = dev_alloc(&b.bbox_part, sort_part_bytes());
     GBH_ALLOC(b.keys, cn);
@@ -1194,14 +1191,15 @@ cudaError_t tree_alloc(TreeBufs &b, int64_t n, int leaf, int32_t nsys) {
     GBH_ALLOC(b.mrange, cnodes);
     GBH_ALLOC(b.lnode, cnodes);
     GBH_ALLOC(b.walk_ctr, 16);
-    GBH_ALLOC(b.scan_tmp, scan_cap);
-    // single-pass scans: the chain counts', the child counts', and the large sort's
-    b.lb_sort = lb_words_of(chain_tiles(cn)) + lb_words_of(child_tiles(cnodes));
+    // single-pass scans: the chain counts', the child counts', the active-star lists' and the large sort's
+    b.lb_targets = lb_words_of(chain_tiles(cn)) + lb_words_of(child_tiles(cnodes));
+    b.lb_sort = b.lb_targets + lb_words_of(target_tiles(cn));
     const int64_t lb_words = b.lb_sort + sort_lb_words(cn);
     GBH_ALLOC(b.lb_state, lb_words);
     const int64_t ctiles = cn / kSortTile + csys + 1;  // sort tiles never straddle systems
     GBH_ALLOC(b.tile_len, 2 * ctiles);
     GBH_ALLOC(b.hist, sort_hist_words(cn));
+    GBH_ALLOC(b.next_part, kNextBlocks);
     GBH_ALLOC(b.info, 1);
 #undef GBH_ALLOC
     if (e != cudaSuccess) {
@@ -1535,35 +1533,45 @@ namespace gbh {
 
 namespace {
 
-__global__ __launch_bounds__(kThreads) void k_target_flags(const DevInfo *info, const int32_t *__restrict__ order,
-                                                           const int32_t *__restrict__ end, int32_t tick,
-                                                           uint32_t *__restrict__ flag) {
-    int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k >= info->nstars) return;
-    flag[k] = end[order[k]] == tick;
-}
-
-__global__ __launch_bounds__(kThreads) void k_target_write(DevInfo *info, const int32_t *__restrict__ order,
-                                                           const int32_t *__restrict__ end, int32_t tick,
-                                                           const uint32_t *__restrict__ pos, int32_t *__restrict__ targets) {
-    int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    int64_t ns = info->nstars;
-    if (k >= ns) return;
-    bool on = end[order[k]] == tick;
-    if (on) targets[pos[k]] = int32_t(k);
-    if (k == ns - 1) info->ntargets = pos[k] + (on ? 1u : 0u);
+// The active stars' sorted positions in order, in one launch: flags ranked by ballots, tiles by
+// look-back. A block takes the next tile of 1,024 positions.
+__global__ __launch_bounds__(kTargetThreads) void k_targets(DevInfo *info, const int32_t *__restrict__ order,
+                                                            const int32_t *__restrict__ end, int32_t tick,
+                                                            int32_t *__restrict__ targets, uint32_t *lb) {
+    pdl_begin();
+    __shared__ uint32_t s_warp[kTargetThreads / 32 + 1];
+    __shared__ uint32_t s_tile, s_prefix;
+    if (threadIdx.x == 0) s_tile = atomicAdd(lb, 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    const int64_t ns = info->nstars;
+    const int64_t k0 = int64_t(tile) * kTargetTile + int64_t(threadIdx.x) * kTargetItems;
+    if (int64_t(tile) * kTargetTile >= ns) return;  // uniform
+    uint32_t on = 0, total;
+#pragma unroll
+    for (int q = 0; q < kTargetItems; ++q)
+        if (k0 + q < ns && end[order[k0 + q]] == tick) on |= 1u << q;
+    const uint32_t cnt = __popc(on);
+    uint32_t at = block_excl_scan<kTargetThreads>(cnt, s_warp, total);
+    if (threadIdx.x < 32) {
+        const unsigned long long e = look_back(reinterpret_cast<unsigned long long *>(lb + 2), tile, total, info);
+        if (threadIdx.x == 0) {
+            s_prefix = uint32_t(e);
+            if ((int64_t(tile) + 1) * kTargetTile >= ns) info->ntargets = uint32_t(e) + total;
+        }
+    }
+    __syncthreads();
+    at += s_prefix;
+#pragma unroll
+    for (int q = 0; q < kTargetItems; ++q)
+        if (on >> q & 1u) targets[at++] = int32_t(k0) + q;
 }
 
 }  // namespace
 
-cudaError_t select_targets(const Launch &L, TreeBufs &b, const int32_t *end, int32_t tick) {
-    const unsigned nb = blocks_for(b.cap_n, kThreads);
-    k_target_flags<<<nb, kThreads, 0, L.stream>>>(b.info, b.order, end, tick, b.flag);
-    GBH_LAUNCH_CHECK();
-    cudaError_t e = scan_dyn(L, b.flag, b.flag, b.cap_n, &b.info->nstars, b.scan_tmp, b.scan_tmp_cap);
-    if (e != cudaSuccess) return e;
-    k_target_write<<<nb, kThreads, 0, L.stream>>>(b.info, b.order, end, tick, b.flag, b.targets);
-    GBH_LAUNCH_CHECK();
+cudaError_t select_targets(const Launch &L, TreeBufs &b, int64_t n, const int32_t *end, int32_t tick) {
+    GBH_LAUNCH_AFTER(L, k_targets, unsigned(target_tiles(n)), kTargetThreads, b.info, b.order, end, tick, b.targets,
+                     b.lb_state + b.lb_targets);
     return cudaSuccess;
 }
 
@@ -1599,33 +1607,90 @@ __device__ __forceinline__ double body_dt(double ax, double ay, double az, doubl
     return a > 0 ? eta * sqrt(eps / a) : INFINITY;
 }
 
+// The earliest step end over all bodies, and the bodies that end there (the host sizes that event's
+// walk by them): every thread's (tick, bodies) over its bodies, reduced by block, and by the last
+// block to finish over the blocks' parts (a counter that wraps to 0 by itself). A tick of INT_MAX
+// holds no bodies.
+__device__ __forceinline__ unsigned long long next_join(unsigned long long a, unsigned long long b) {
+    const uint32_t ta = uint32_t(a >> 32), tb = uint32_t(b >> 32);
+    return ta < tb ? a : tb < ta ? b : a + uint32_t(b);
+}
+__device__ __forceinline__ void reduce_next(int32_t tick, uint32_t bodies, unsigned long long *part, DevInfo *info) {
+    __shared__ unsigned long long s_w[kThreads / 32];
+    __shared__ bool s_last;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto block_join = [&](unsigned long long v) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v = next_join(v, __shfl_xor_sync(0xffffffffu, v, o));
+        __syncthreads();
+        if (lane == 0) s_w[warp] = v;
+        __syncthreads();
+        v = s_w[0];
+        for (int w = 1; w < kThreads / 32; ++w) v = next_join(v, s_w[w]);
+        return v;
+    };
+    unsigned long long v = block_join(static_cast<unsigned long long>(uint32_t(tick)) << 32 | bodies);
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = v;
+        __threadfence();
+        s_last = atomicInc(&info->next_done, gridDim.x - 1) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    v = static_cast<unsigned long long>(uint32_t(INT_MAX)) << 32;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += kThreads) v = next_join(v, __ldcg(part + b));
+    v = block_join(v);
+    if (threadIdx.x == 0) {
+        info->next_tick = int32_t(v >> 32);
+        info->next_count = uint32_t(v);
+    }
+}
+// Adds a body that ends at e to a thread's (tick, bodies).
+__device__ __forceinline__ void add_end(int32_t e, int32_t &tick, uint32_t &bodies) {
+    if (e < tick) {
+        tick = e;
+        bodies = 1;
+    } else if (e == tick) {
+        ++bodies;
+    }
+}
+
 // Tick 0 of a global step: every body starts a step (rung from its acceleration) with the
 // opening half kick.
 __global__ __launch_bounds__(kThreads) void k_block_open(int64_t n, double T, int32_t ticks, int levels, double eta,
                                                          double eps, const double *__restrict__ ax,
                                                          const double *__restrict__ ay, const double *__restrict__ az,
                                                          double *vx, double *vy, double *vz, uint8_t *rung,
-                                                         int32_t *end, DevInfo *info) {
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double a0 = ax[i], a1 = ay[i], a2 = az[i];
-    int r = rung_for(body_dt(a0, a1, a2, eta, eps), T, levels - 1);
-    rung[i] = uint8_t(r);
-    int32_t e = ticks >> r;
-    end[i] = e;
-    double h = 0.5 * (T / double(1 << r));
-    vx[i] += h * a0;
-    vy[i] += h * a1;
-    vz[i] += h * a2;
-    atomicMin(&info->next_tick, e);
+                                                         int32_t *end, unsigned long long *part, DevInfo *info) {
+    pdl_begin();
+    int32_t tick = INT_MAX;
+    uint32_t bodies = 0;
+    for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < n; i += int64_t(gridDim.x) * kThreads) {
+        double a0 = ax[i], a1 = ay[i], a2 = az[i];
+        int r = rung_for(body_dt(a0, a1, a2, eta, eps), T, levels - 1);
+        rung[i] = uint8_t(r);
+        int32_t e = ticks >> r;
+        end[i] = e;
+        double h = 0.5 * (T / double(1 << r));
+        vx[i] += h * a0;
+        vy[i] += h * a1;
+        vz[i] += h * a2;
+        add_end(e, tick, bodies);
+    }
+    reduce_next(tick, bodies, part, info);
 }
 
-// driftOne (sim.go:345-350): x += dt u / gamma(u, c), gamma = 1 for c <= 0 (relativity.go:15-20).
-__global__ __launch_bounds__(kThreads) void k_block_drift(int64_t n, double dt, double c, double *px, double *py,
-                                                          double *pz, const double *__restrict__ vx,
-                                                          const double *__restrict__ vy, const double *__restrict__ vz) {
+// driftOne (sim.go:345-350) of every body from tick t to the next event's tick: x += dt u / gamma(u, c),
+// gamma = 1 for c <= 0 (relativity.go:15-20).
+__global__ __launch_bounds__(kThreads) void k_block_drift(int64_t n, int32_t t, double tick_len, double c, double *px,
+                                                          double *py, double *pz, const double *__restrict__ vx,
+                                                          const double *__restrict__ vy, const double *__restrict__ vz,
+                                                          const DevInfo *info) {
+    pdl_begin();
     int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    const double dt = double(info->next_tick - t) * tick_len;
     double ux = vx[i], uy = vy[i], uz = vz[i];
     double f = dt / (c <= 0 ? 1.0 : sqrt(1 + (ux * ux + uy * uy + uz * uz) / (c * c)));
     px[i] += f * ux;
@@ -1639,45 +1704,39 @@ __global__ __launch_bounds__(kThreads) void k_block_close(int64_t n, int32_t tic
                                                           double eta, double eps, const double *__restrict__ ax,
                                                           const double *__restrict__ ay, const double *__restrict__ az,
                                                           double *vx, double *vy, double *vz, uint8_t *rung,
-                                                          int32_t *end, DevInfo *info) {
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int32_t e = end[i];
-    if (e == tick) {
-        double a0 = ax[i], a1 = ay[i], a2 = az[i];
-        double h = 0.5 * (T / double(1 << rung[i]));
-        vx[i] += h * a0;
-        vy[i] += h * a1;
-        vz[i] += h * a2;
-        if (tick < ticks) {
-            int r = rung_for(body_dt(a0, a1, a2, eta, eps), T, levels - 1);
-            while (tick % (ticks >> r) != 0) ++r;
-            rung[i] = uint8_t(r);
-            e = tick + (ticks >> r);
-            end[i] = e;
-            double h2 = 0.5 * (T / double(1 << r));
-            vx[i] += h2 * a0;
-            vy[i] += h2 * a1;
-            vz[i] += h2 * a2;
+                                                          int32_t *end, unsigned long long *part, DevInfo *info) {
+    pdl_begin();
+    int32_t next = INT_MAX;
+    uint32_t bodies = 0;
+    for (int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x; i < n; i += int64_t(gridDim.x) * kThreads) {
+        int32_t e = end[i];
+        if (e == tick) {
+            double a0 = ax[i], a1 = ay[i], a2 = az[i];
+            double h = 0.5 * (T / double(1 << rung[i]));
+            double u = vx[i] + h * a0, v = vy[i] + h * a1, w = vz[i] + h * a2;
+            if (tick < ticks) {
+                int r = rung_for(body_dt(a0, a1, a2, eta, eps), T, levels - 1);
+                while (tick % (ticks >> r) != 0) ++r;
+                rung[i] = uint8_t(r);
+                e = tick + (ticks >> r);
+                end[i] = e;
+                double h2 = 0.5 * (T / double(1 << r));
+                u += h2 * a0;
+                v += h2 * a1;
+                w += h2 * a2;
+            }
+            vx[i] = u;
+            vy[i] = v;
+            vz[i] = w;
         }
+        add_end(e, next, bodies);
     }
-    atomicMin(&info->next_tick, e);
+    reduce_next(next, bodies, part, info);
 }
 
-// The bodies whose step ends at the next event tick (the host sizes that event's walk by them).
-__global__ __launch_bounds__(kThreads) void k_count_next(int64_t n, const int32_t *__restrict__ end, DevInfo *info) {
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int32_t tn = info->next_tick;
-    const unsigned m = __ballot_sync(0xffffffffu, i < n && end[i] == tn);  // whole warps: no early return
-    if ((threadIdx.x & 31) == 0 && m) atomicAdd(&info->next_count, uint32_t(__popc(m)));
-}
-
-cudaError_t count_next(const Launch &L, const TreeBufs &b, int64_t n, const int32_t *end) {
-    cudaError_t e = cudaMemsetAsync(&b.info->next_count, 0, sizeof(uint32_t), L.stream);
-    if (e != cudaSuccess) return e;
-    k_count_next<<<blocks_for(n, kThreads), kThreads, 0, L.stream>>>(n, end, b.info);
-    GBH_LAUNCH_CHECK();
-    return cudaSuccess;
+inline unsigned next_blocks(int64_t n) {
+    const unsigned nb = blocks_for(n, kThreads);
+    return nb < unsigned(kNextBlocks) ? nb : unsigned(kNextBlocks);
 }
 
 }  // namespace
@@ -1685,30 +1744,24 @@ cudaError_t count_next(const Launch &L, const TreeBufs &b, int64_t n, const int3
 cudaError_t block_open(const Launch &L, const TreeBufs &b, int64_t n, double T, int levels, double eta, double eps,
                        const double *ax, const double *ay, const double *az, double *vx, double *vy, double *vz,
                        uint8_t *rung, int32_t *end) {
-    cudaError_t e = cudaMemsetAsync(&b.info->next_tick, 0x7f, sizeof(int32_t), L.stream);
-    if (e != cudaSuccess) return e;
-    k_block_open<<<blocks_for(n, kThreads), kThreads, 0, L.stream>>>(n, T, 1 << (levels - 1), levels, eta, eps, ax, ay,
-                                                                     az, vx, vy, vz, rung, end, b.info);
-    GBH_LAUNCH_CHECK();
-    return count_next(L, b, n, end);
+    GBH_LAUNCH_AFTER(L, k_block_open, next_blocks(n), kThreads, n, T, 1 << (levels - 1), levels, eta, eps, ax, ay, az, vx,
+                     vy, vz, rung, end, b.next_part, b.info);
+    return cudaSuccess;
 }
 
-cudaError_t block_drift(const Launch &L, int64_t n, double dt, double c, double *px, double *py, double *pz,
-                        const double *vx, const double *vy, const double *vz) {
-    k_block_drift<<<blocks_for(n, kThreads), kThreads, 0, L.stream>>>(n, dt, c, px, py, pz, vx, vy, vz);
-    GBH_LAUNCH_CHECK();
+cudaError_t block_drift(const Launch &L, const TreeBufs &b, int64_t n, int32_t t, double tick_len, double c, double *px,
+                        double *py, double *pz, const double *vx, const double *vy, const double *vz) {
+    GBH_LAUNCH_AFTER(L, k_block_drift, blocks_for(n, kThreads), kThreads, n, t, tick_len, c, px, py, pz, vx, vy, vz,
+                     b.info);
     return cudaSuccess;
 }
 
 cudaError_t block_close(const Launch &L, const TreeBufs &b, int64_t n, int32_t tick, double T, int levels, double eta,
                         double eps, const double *ax, const double *ay, const double *az, double *vx, double *vy,
                         double *vz, uint8_t *rung, int32_t *end) {
-    cudaError_t e = cudaMemsetAsync(&b.info->next_tick, 0x7f, sizeof(int32_t), L.stream);
-    if (e != cudaSuccess) return e;
-    k_block_close<<<blocks_for(n, kThreads), kThreads, 0, L.stream>>>(n, tick, 1 << (levels - 1), T, levels, eta, eps,
-                                                                      ax, ay, az, vx, vy, vz, rung, end, b.info);
-    GBH_LAUNCH_CHECK();
-    return count_next(L, b, n, end);
+    GBH_LAUNCH_AFTER(L, k_block_close, next_blocks(n), kThreads, n, tick, 1 << (levels - 1), T, levels, eta, eps, ax, ay, az,
+                     vx, vy, vz, rung, end, b.next_part, b.info);
+    return cudaSuccess;
 }
 
 }  // namespace gbh
