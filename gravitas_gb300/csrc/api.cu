@@ -90,6 +90,8 @@ struct gbh_ctx {
     cudaEvent_t wait_ev = nullptr;  // GBH_CFG_BLOCKING_SYNC: host waits sleep on this event
     cudaEvent_t ahead[4] = {};      // GBH_CFG_BLOCKING_SYNC: ends of the last steps launched
     bool capturing = false;  // stage events become graph event-record nodes
+    bool host_access = false;  // kernels can read and write the callers' arrays (pageable memory)
+    bool touching = false;     // a kernel that does may be in flight
     // The corrupt-link test hook: with GBH_FAULT_LINK set (non-empty) when the context is created,
     // the next tree built outside graph capture gets a cycle (the last leaf's skip link points back
     // at node 0) before its walk, so the walk runs into its step bound and the call returns
@@ -316,6 +318,87 @@ int d2h(gbh_ctx *ctx, void *dst, const void *src, size_t bytes) {
     return GBH_OK;
 }
 
+// Copies of a call's arrays between the caller's memory and the device: up to 12 arrays of n doubles
+// and 2 of n bytes (null pairs are skipped).
+struct Arrays {
+    static constexpr int kDoubles = 12, kBytes = 2;
+    const double *src[kDoubles];
+    double *dst[kDoubles];
+    const uint8_t *bsrc[kBytes];
+    uint8_t *bdst[kBytes];
+    int nd = 0, nb = 0;
+    void add(double *d, const double *s) {
+        if (!d || !s) return;
+        dst[nd] = d;
+        src[nd++] = s;
+    }
+    void add(uint8_t *d, const uint8_t *s) {
+        if (!d || !s) return;
+        bdst[nb] = d;
+        bsrc[nb++] = s;
+    }
+};
+
+// Element i of every array, a thread each; all loads go out before the first store.
+constexpr int kCopyThreads = 256;
+__global__ __launch_bounds__(kCopyThreads) void k_copy_arrays(int64_t n, Arrays a) {
+    gbh::pdl_begin();
+    const int64_t i = int64_t(blockIdx.x) * kCopyThreads + threadIdx.x;
+    if (i >= n) return;
+    double v[Arrays::kDoubles];
+    uint8_t b[Arrays::kBytes];
+#pragma unroll
+    for (int k = 0; k < Arrays::kDoubles; ++k)
+        if (k < a.nd) v[k] = a.src[k][i];
+#pragma unroll
+    for (int k = 0; k < Arrays::kBytes; ++k)
+        if (k < a.nb) b[k] = a.bsrc[k][i];
+#pragma unroll
+    for (int k = 0; k < Arrays::kDoubles; ++k)
+        if (k < a.nd) a.dst[k][i] = v[k];
+#pragma unroll
+    for (int k = 0; k < Arrays::kBytes; ++k)
+        if (k < a.nb) a.bdst[k][i] = b[k];
+}
+
+// One kernel copies a call's arrays of up to kCopyKernelMax elements where the GPU reads and writes
+// pageable memory through the host's page tables (Grace over C2C); otherwise, for misaligned arrays
+// and for larger ones, a copy each. Measured with 9 pageable arrays, kernel against copies: 1,013
+// elements 12 / 19 us in and 10 / 74 out, 16,384 16 / 86 and 16 / 80, 60,000 33 / 105 and 36 / 102,
+// 262,144 108 / 190 and 129 / 177, 1,048,576 391 / 512 and 506 / 472.
+constexpr int64_t kCopyKernelMax = int64_t(1) << 18;
+int copy_arrays(gbh_ctx *ctx, cudaStream_t stream, int64_t n, const Arrays &a, bool to_host) {
+    (to_host ? ctx->d2h : ctx->h2d) += n * (int64_t(sizeof(double)) * a.nd + a.nb);
+    if (n <= 0 || a.nd + a.nb == 0) return GBH_OK;
+    uintptr_t bits = 0;
+    for (int k = 0; k < a.nd; ++k) bits |= reinterpret_cast<uintptr_t>(a.src[k]) | reinterpret_cast<uintptr_t>(a.dst[k]);
+    if (ctx->host_access && n <= kCopyKernelMax && bits % sizeof(double) == 0) {
+        ctx->touching = true;
+        Launch L{stream, &ctx->launches, ctx->num_sms};
+        CK(gbh::launch_after(L, k_copy_arrays, unsigned((n + kCopyThreads - 1) / kCopyThreads), kCopyThreads, n, a));
+        return GBH_OK;
+    }
+    const cudaMemcpyKind dir = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
+    for (int k = 0; k < a.nd; ++k) CK(cudaMemcpyAsync(a.dst[k], a.src[k], sizeof(double) * size_t(n), dir, stream));
+    for (int k = 0; k < a.nb; ++k) CK(cudaMemcpyAsync(a.bdst[k], a.bsrc[k], size_t(n), dir, stream));
+    return GBH_OK;
+}
+
+// Whichever way an entry point returns, no kernel touches the caller's arrays afterwards (finish has
+// waited on the ordinary way out).
+struct Settle {
+    gbh_ctx *ctx;
+    explicit Settle(gbh_ctx *c) : ctx(c) {}
+    ~Settle() {
+        if (!ctx->touching) return;
+        cudaStreamSynchronize(ctx->stream);
+        cudaStreamSynchronize(ctx->copy_stream);
+        ctx->touching = false;
+    }
+    Settle(const Settle &) = delete;
+    Settle &operator=(const Settle &) = delete;
+};
+
 // Tree build + walk on device arrays; accelerations of alive non-hole bodies, holes zeroed.
 // forest: the resident state's systems (each its own tree) instead of one system.
 int forces(gbh_ctx *ctx, const gbh_params *p, int64_t n, const double *px, const double *py, const double *pz,
@@ -379,6 +462,7 @@ int finish(gbh_ctx *ctx, bool tree) {
         CK(cudaMemcpyAsync(ctx->info_host, ctx->tb.info, sizeof(DevInfo), cudaMemcpyDeviceToHost, ctx->stream));
     }
     CK(wait_stream(ctx));
+    ctx->touching = false;  // a copy on the copy stream has been joined
     float ms = 0;
     gbh_timings &t = ctx->last;
     if (cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[5]) == cudaSuccess) t.total_ms = ms;
@@ -712,25 +796,23 @@ int upload_state(gbh_ctx *ctx, int64_t n, const double *px, const double *py, co
     if (n > 0 && (!px || !py || !pz || !vx || !vy || !vz || !mass))
         return fail(ctx, GBH_ERR_ARG, "state arrays must not be NULL");
     CK(ensure_state(ctx, n));
-    size_t b = sizeof(double) * size_t(n);
-    int rc;
-    const double *src[] = {px, py, pz, vx, vy, vz, mass};
-    double *dst[] = {ctx->px, ctx->py, ctx->pz, ctx->vx, ctx->vy, ctx->vz, ctx->mass};
-    for (int k = 0; k < 7; ++k)
-        if ((rc = h2d(ctx, dst[k], src[k], b))) return rc;
-    bool acc = ax && ay && az;
-    if (acc) {
-        if ((rc = h2d(ctx, ctx->ax, ax, b)) || (rc = h2d(ctx, ctx->ay, ay, b)) || (rc = h2d(ctx, ctx->az, az, b)))
-            return rc;
-    } else if (n > 0) {
+    const bool acc = ax && ay && az;
+    const double *src[] = {px, py, pz, vx, vy, vz, mass, acc ? ax : nullptr, acc ? ay : nullptr, acc ? az : nullptr};
+    double *dst[] = {ctx->px, ctx->py, ctx->pz, ctx->vx, ctx->vy, ctx->vz, ctx->mass, ctx->ax, ctx->ay, ctx->az};
+    Arrays in;
+    for (int k = 0; k < 10; ++k) in.add(dst[k], src[k]);
+    in.add(ctx->kind, kind);
+    in.add(ctx->alive, alive);
+    int rc = copy_arrays(ctx, ctx->stream, n, in, false);
+    if (rc) return rc;
+    if (!acc && n > 0) {
+        const size_t b = sizeof(double) * size_t(n);
         CK(cudaMemsetAsync(ctx->ax, 0, b, ctx->stream));
         CK(cudaMemsetAsync(ctx->ay, 0, b, ctx->stream));
         CK(cudaMemsetAsync(ctx->az, 0, b, ctx->stream));
     }
     ctx->state_has_kind = kind != nullptr;
     ctx->state_has_alive = alive != nullptr;
-    if (kind && (rc = h2d(ctx, ctx->kind, kind, size_t(n)))) return rc;
-    if (alive && (rc = h2d(ctx, ctx->alive, alive, size_t(n)))) return rc;
     ctx->n = n;
     ctx->have_state = true;
     ctx->acc_valid = acc;
@@ -749,15 +831,11 @@ int upload_state(gbh_ctx *ctx, int64_t n, const double *px, const double *py, co
 
 int download_state(gbh_ctx *ctx, double *px, double *py, double *pz, double *vx, double *vy, double *vz, double *ax,
                    double *ay, double *az) {
-    size_t b = sizeof(double) * size_t(ctx->n);
     double *dst[] = {px, py, pz, vx, vy, vz, ax, ay, az};
     const double *src[] = {ctx->px, ctx->py, ctx->pz, ctx->vx, ctx->vy, ctx->vz, ctx->ax, ctx->ay, ctx->az};
-    for (int k = 0; k < 9; ++k)
-        if (dst[k]) {
-            int rc = d2h(ctx, dst[k], src[k], b);
-            if (rc) return rc;
-        }
-    return GBH_OK;
+    Arrays out;
+    for (int k = 0; k < 9; ++k) out.add(dst[k], src[k]);
+    return copy_arrays(ctx, ctx->stream, ctx->n, out, true);
 }
 
 }  // namespace
@@ -807,6 +885,7 @@ int gbh_create(const gbh_config *cfg, gbh_ctx **out, char *err, int errlen) {
         }
     }
     c->num_sms = prop.multiProcessorCount;
+    c->host_access = prop.pageableMemoryAccess && prop.pageableMemoryAccessUsesHostPageTables;
     if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess) {
         delete c;
         return report(GBH_ERR_CUDA, cudaGetErrorString(e));
@@ -885,24 +964,28 @@ int gbh_accelerations(gbh_ctx *ctx, const gbh_params *p, int64_t n, const double
     gbh::NvtxRange nvtx_range_(__func__);
     int rc = begin(ctx);
     if (rc || (rc = check_params(ctx, p))) return rc;
+    Settle settle_(ctx);
     if (n < 0 || n > (int64_t(1) << 30)) return fail(ctx, GBH_ERR_ARG, "n = %lld out of range", (long long)n);
     if (n == 0) return GBH_OK;
     if (!px || !py || !pz || !mass || !ax || !ay || !az) return fail(ctx, GBH_ERR_ARG, "array argument is NULL");
     CK(ensure_state(ctx, n));
     ctx->have_state = false;  // the state buffers now hold this call's arrays
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-    size_t b = sizeof(double) * size_t(n);
-    if ((rc = h2d(ctx, ctx->px, px, b)) || (rc = h2d(ctx, ctx->py, py, b)) || (rc = h2d(ctx, ctx->pz, pz, b)) ||
-        (rc = h2d(ctx, ctx->mass, mass, b)))
-        return rc;
     // Dead bodies keep their entries (bh.go:92-101 writes only stars and holes).
-    if ((rc = h2d(ctx, ctx->ax, ax, b)) || (rc = h2d(ctx, ctx->ay, ay, b)) || (rc = h2d(ctx, ctx->az, az, b))) return rc;
-    if (kind && (rc = h2d(ctx, ctx->kind, kind, size_t(n)))) return rc;
-    if (alive && (rc = h2d(ctx, ctx->alive, alive, size_t(n)))) return rc;
+    const double *src[] = {px, py, pz, mass, ax, ay, az};
+    double *dst[] = {ctx->px, ctx->py, ctx->pz, ctx->mass, ctx->ax, ctx->ay, ctx->az};
+    Arrays in, out;
+    for (int k = 0; k < 7; ++k) in.add(dst[k], src[k]);
+    in.add(ctx->kind, kind);
+    in.add(ctx->alive, alive);
+    if ((rc = copy_arrays(ctx, ctx->stream, n, in, false))) return rc;
     rc = forces(ctx, p, n, ctx->px, ctx->py, ctx->pz, ctx->mass, kind ? ctx->kind : nullptr,
                 alive ? ctx->alive : nullptr, ctx->ax, ctx->ay, ctx->az, theta_of(p));
     if (rc) return rc;
-    if ((rc = d2h(ctx, ax, ctx->ax, b)) || (rc = d2h(ctx, ay, ctx->ay, b)) || (rc = d2h(ctx, az, ctx->az, b))) return rc;
+    out.add(ax, ctx->ax);
+    out.add(ay, ctx->ay);
+    out.add(az, ctx->az);
+    if ((rc = copy_arrays(ctx, ctx->stream, n, out, true))) return rc;
     return finish(ctx, true);
 }
 
@@ -912,6 +995,7 @@ int gbh_potential_energy(gbh_ctx *ctx, const gbh_params *p, int64_t n, const dou
     gbh::NvtxRange nvtx_range_(__func__);
     int rc = begin(ctx);
     if (rc || (rc = check_params(ctx, p))) return rc;
+    Settle settle_(ctx);
     if (!u) return fail(ctx, GBH_ERR_ARG, "u is NULL");
     *u = 0;
     if (n < 0 || n > (int64_t(1) << 30)) return fail(ctx, GBH_ERR_ARG, "n out of range");
@@ -920,12 +1004,14 @@ int gbh_potential_energy(gbh_ctx *ctx, const gbh_params *p, int64_t n, const dou
     CK(ensure_state(ctx, n));
     ctx->have_state = false;
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-    size_t b = sizeof(double) * size_t(n);
-    if ((rc = h2d(ctx, ctx->px, px, b)) || (rc = h2d(ctx, ctx->py, py, b)) || (rc = h2d(ctx, ctx->pz, pz, b)) ||
-        (rc = h2d(ctx, ctx->mass, mass, b)))
-        return rc;
-    if (kind && (rc = h2d(ctx, ctx->kind, kind, size_t(n)))) return rc;
-    if (alive && (rc = h2d(ctx, ctx->alive, alive, size_t(n)))) return rc;
+    Arrays in;
+    in.add(ctx->px, px);
+    in.add(ctx->py, py);
+    in.add(ctx->pz, pz);
+    in.add(ctx->mass, mass);
+    in.add(ctx->kind, kind);
+    in.add(ctx->alive, alive);
+    if ((rc = copy_arrays(ctx, ctx->stream, n, in, false))) return rc;
     // Holes in state order (collect, build.go:65-69).
     std::vector<int32_t> holes;
     if (kind)
@@ -968,6 +1054,7 @@ int gbh_direct_accelerations(gbh_ctx *ctx, const gbh_params *p, int64_t n, const
     gbh::NvtxRange nvtx_range_(__func__);
     int rc = begin(ctx);
     if (rc || (rc = check_params(ctx, p))) return rc;
+    Settle settle_(ctx);
     if (n < 0 || n > (int64_t(1) << 30)) return fail(ctx, GBH_ERR_ARG, "n out of range");
     if (!targets) ntargets = n;
     if (ntargets < 0) return fail(ctx, GBH_ERR_ARG, "ntargets < 0");
@@ -979,11 +1066,13 @@ int gbh_direct_accelerations(gbh_ctx *ctx, const gbh_params *p, int64_t n, const
     CK(ensure_state(ctx, n));
     ctx->have_state = false;
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-    size_t b = sizeof(double) * size_t(n);
-    if ((rc = h2d(ctx, ctx->px, px, b)) || (rc = h2d(ctx, ctx->py, py, b)) || (rc = h2d(ctx, ctx->pz, pz, b)) ||
-        (rc = h2d(ctx, ctx->mass, mass, b)))
-        return rc;
-    if (kind && (rc = h2d(ctx, ctx->kind, kind, size_t(n)))) return rc;
+    Arrays in, out;
+    in.add(ctx->px, px);
+    in.add(ctx->py, py);
+    in.add(ctx->pz, pz);
+    in.add(ctx->mass, mass);
+    in.add(ctx->kind, kind);
+    if ((rc = copy_arrays(ctx, ctx->stream, n, in, false))) return rc;
     CK(grow_targets(ctx, ntargets));
     if (targets && (rc = h2d(ctx, ctx->targets, targets, sizeof(int64_t) * size_t(ntargets)))) return rc;
     double *tx = ctx->tout, *ty = tx + ctx->targets_cap, *tz = ty + ctx->targets_cap;
@@ -991,8 +1080,10 @@ int gbh_direct_accelerations(gbh_ctx *ctx, const gbh_params *p, int64_t n, const
     CK(gbh::direct_fp64(L, n, ctx->px, ctx->py, ctx->pz, ctx->mass, kind ? ctx->kind : nullptr,
                         p->softening * p->softening, p->dark_matter_off, targets ? ctx->targets : nullptr, ntargets,
                         tx, ty, tz));
-    size_t tb = sizeof(double) * size_t(ntargets);
-    if ((rc = d2h(ctx, ax, tx, tb)) || (rc = d2h(ctx, ay, ty, tb)) || (rc = d2h(ctx, az, tz, tb))) return rc;
+    out.add(ax, tx);
+    out.add(ay, ty);
+    out.add(az, tz);
+    if ((rc = copy_arrays(ctx, ctx->stream, ntargets, out, true))) return rc;
     return finish(ctx, false);
 }
 
@@ -1002,6 +1093,7 @@ int gbh_step_kdk(gbh_ctx *ctx, const gbh_params *p, double dt, int64_t nsteps, i
     gbh::NvtxRange nvtx_range_(__func__);
     int rc = begin(ctx);
     if (rc || (rc = check_params(ctx, p))) return rc;
+    Settle settle_(ctx);
     if (nsteps < 0) return fail(ctx, GBH_ERR_ARG, "nsteps < 0");
     if (!ax || !ay || !az) return fail(ctx, GBH_ERR_ARG, "acceleration arrays must not be NULL");
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
@@ -1014,13 +1106,14 @@ int gbh_step_kdk(gbh_ctx *ctx, const gbh_params *p, double dt, int64_t nsteps, i
     if (n > 0 && ctx->evused >= 3) {
         // The positions are final once the last force evaluation starts (its first stage event):
         // copy them back on the copy stream while that tree build and walk run.
-        size_t b = sizeof(double) * size_t(n);
         CK(cudaStreamWaitEvent(ctx->copy_stream, ctx->evpool[ctx->evused - 3], 0));
-        double *dst[3] = {px, py, pz};
-        const double *src[3] = {ctx->px, ctx->py, ctx->pz};
-        for (int k = 0; k < 3; ++k) {
-            CK(cudaMemcpyAsync(dst[k], src[k], b, cudaMemcpyDeviceToHost, ctx->copy_stream));
-            ctx->d2h += int64_t(b);
+        Arrays pos;
+        pos.add(px, ctx->px);
+        pos.add(py, ctx->py);
+        pos.add(pz, ctx->pz);
+        if ((rc = copy_arrays(ctx, ctx->copy_stream, n, pos, true))) {
+            cudaStreamSynchronize(ctx->copy_stream);  // no copy into the caller's arrays after return
+            return rc;
         }
         cudaError_t e = cudaEventRecord(ctx->copy_done, ctx->copy_stream);
         if (e == cudaSuccess) rc = download_state(ctx, nullptr, nullptr, nullptr, vx, vy, vz, ax, ay, az);
@@ -1041,6 +1134,7 @@ int gbh_state_upload(gbh_ctx *ctx, int64_t n, const double *px, const double *py
     gbh::NvtxRange nvtx_range_(__func__);
     int rc = begin(ctx);
     if (rc) return rc;
+    Settle settle_(ctx);
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
     if ((rc = upload_state(ctx, n, px, py, pz, vx, vy, vz, ax, ay, az, mass, kind, alive))) return rc;
     return finish(ctx, false);
@@ -1051,6 +1145,7 @@ int gbh_state_download(gbh_ctx *ctx, double *px, double *py, double *pz, double 
     gbh::NvtxRange nvtx_range_(__func__);
     int rc = begin(ctx);
     if (rc) return rc;
+    Settle settle_(ctx);
     if (!ctx->have_state) return fail(ctx, GBH_ERR_STATE, "no resident state");
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
     if ((rc = download_state(ctx, px, py, pz, vx, vy, vz, ax, ay, az))) return rc;
@@ -1189,6 +1284,7 @@ int gbh_forest_upload(gbh_ctx *ctx, int32_t nsys, const int64_t *offsets, const 
     gbh::NvtxRange nvtx_range_(__func__);
     int rc = begin(ctx);
     if (rc) return rc;
+    Settle settle_(ctx);
     if (nsys < 1 || nsys > 65535) return fail(ctx, GBH_ERR_ARG, "nsys %d outside [1, 65535]", nsys);
     if (!offsets) return fail(ctx, GBH_ERR_ARG, "offsets is NULL");
     if (offsets[0] != 0) return fail(ctx, GBH_ERR_ARG, "offsets[0] must be 0");
@@ -1287,6 +1383,7 @@ int gbh_fwd_save(gbh_ctx *ctx, const gbh_adjoint_params *ap, int64_t n, const do
     gbh::NvtxRange nvtx_range_(__func__);
     int rc = begin(ctx);
     if (rc) return rc;
+    Settle settle_(ctx);
     ctx->adj.valid = false;
     if (!ap) return fail(ctx, GBH_ERR_ARG, "adjoint params are NULL");
     if (!(ap->softening > 0)) return fail(ctx, GBH_ERR_ARG, "softening %g must be > 0", ap->softening);
@@ -1313,17 +1410,17 @@ int gbh_fwd_save(gbh_ctx *ctx, const gbh_adjoint_params *ap, int64_t n, const do
         CK(gbh::tree_alloc(ctx->tb, n, t.leaf, 1));
         CK(gbh::adj_tree_reserve(t.tbs, ctx->tb));
     }
-    size_t b = sizeof(double) * size_t(n);
-    if ((rc = h2d(ctx, t.x, px, b)) || (rc = h2d(ctx, t.x + n, py, b)) || (rc = h2d(ctx, t.x + 2 * n, pz, b)) ||
-        (rc = h2d(ctx, t.v, vx, b)) || (rc = h2d(ctx, t.v + n, vy, b)) || (rc = h2d(ctx, t.v + 2 * n, vz, b)) ||
-        (rc = h2d(ctx, t.m, mass, b)))
-        return rc;
+    const double *src[] = {px, py, pz, vx, vy, vz, mass};
+    double *dst[] = {t.x, t.x + n, t.x + 2 * n, t.v, t.v + n, t.v + 2 * n, t.m};
+    Arrays in, out;
+    for (int k = 0; k < 7; ++k) in.add(dst[k], src[k]);
+    if ((rc = copy_arrays(ctx, ctx->stream, n, in, false))) return rc;
     t.mark = [](void *c) { return stage_event(static_cast<gbh_ctx *>(c)); };
     t.mark_arg = ctx;
     CK(gbh::adj_forward(launch_of(ctx), t));
     double *outs[6] = {out_px, out_py, out_pz, out_vx, out_vy, out_vz};
-    for (int k = 0; k < 6; ++k)
-        if (outs[k] && (rc = d2h(ctx, outs[k], (k < 3 ? t.x : t.v) + (k % 3) * n, b))) return rc;
+    for (int k = 0; k < 6; ++k) out.add(outs[k], (k < 3 ? t.x : t.v) + (k % 3) * n);
+    if ((rc = copy_arrays(ctx, ctx->stream, n, out, true))) return rc;
     t.valid = false;
     if ((rc = finish(ctx, false))) return rc;
     t.valid = true;
@@ -1335,6 +1432,7 @@ int gbh_bwd(gbh_ctx *ctx, const double *gx, const double *gy, const double *gz, 
     gbh::NvtxRange nvtx_range_(__func__);
     int rc = begin(ctx);
     if (rc) return rc;
+    Settle settle_(ctx);
     gbh::AdjTape &t = ctx->adj;
     if (!t.valid) return fail(ctx, GBH_ERR_STATE, "no adjoint tape: call gbh_fwd_save first");
     const int64_t n = t.n;
@@ -1345,18 +1443,17 @@ int gbh_bwd(gbh_ctx *ctx, const double *gx, const double *gy, const double *gz, 
         CK(gbh::adj_tree_reserve(t.tbs, ctx->tb));
     }
     const double *gin[6] = {gx, gy, gz, gvx, gvy, gvz};
+    Arrays in, out;
     for (int k = 0; k < 6; ++k) {
-        if (gin[k]) {
-            if ((rc = h2d(ctx, t.lam + k * n, gin[k], b))) return rc;
-        } else {
-            CK(cudaMemsetAsync(t.lam + k * n, 0, b, ctx->stream));
-        }
+        in.add(t.lam + k * n, gin[k]);
+        if (!gin[k]) CK(cudaMemsetAsync(t.lam + k * n, 0, b, ctx->stream));
     }
+    if ((rc = copy_arrays(ctx, ctx->stream, n, in, false))) return rc;
     CK(cudaMemsetAsync(t.lam + 6 * n, 0, b, ctx->stream));
     CK(gbh::adj_backward(launch_of(ctx), t));
     double *outs[7] = {dx, dy, dz, dvx, dvy, dvz, dm};
-    for (int k = 0; k < 7; ++k)
-        if (outs[k] && (rc = d2h(ctx, outs[k], t.lam + k * n, b))) return rc;
+    for (int k = 0; k < 7; ++k) out.add(outs[k], t.lam + k * n);
+    if ((rc = copy_arrays(ctx, ctx->stream, n, out, true))) return rc;
     return finish(ctx, false);
 }
 
