@@ -690,8 +690,22 @@ __device__ __forceinline__ void store_acc(const GroupStars<kS> &G, const Acc (&a
     }
 }
 
-// kSplit: work item i walks part i % nparts of group i / nparts (walk_group's split mode) and
-// writes its sums by sorted index to part_acc[part][axis][star]; k_split_combine adds the parts.
+// The part that a split walk's item of rank r walks, for a group whose first star is at sorted place
+// k: the part that holds the star first, then its neighbours on both sides, farther and farther. A
+// part's work falls with its distance from the group (the near one opens leaves, the far ones
+// accept a few nodes), so taking all groups' near parts first is longest first, and the items left
+// for the end are short. Walks against taking each group's parts one after the other: Plummer spheres
+// (theta 0.5) of 16,384 stars 0.122 -> 0.111 ms, 60,000 0.341 -> 0.296; theta 0.9 0.075 -> 0.060 and
+// 0.144 -> 0.126.
+__device__ __forceinline__ int split_part(int r, int32_t k, int32_t ns, int nparts) {
+    const int own = min(int(int64_t(k) * nparts / ns), nparts - 1);
+    const int d = (r & 1) ? (r + 1) / 2 : nparts - r / 2;  // 0, +1, -1, +2, ... modulo nparts
+    return (own + d) % nparts;
+}
+
+// kSplit: work item i walks a part (split_part of rank i / groups) of group i % groups (walk_group's
+// split mode) and writes its sums by sorted index to part_acc[part][axis][star]; k_split_combine
+// adds the parts.
 template <bool kQuad, bool kSoft, int kS, bool kSplit = false>
 __global__ __launch_bounds__(kLwThreads, kS == 2 ? 8 : 10) void k_walk_lists(const DevInfo *info, const LNode *__restrict__ nodes,
                                                            const float4 *__restrict__ st_hi,
@@ -722,13 +736,14 @@ __global__ __launch_bounds__(kLwThreads, kS == 2 ? 8 : 10) void k_walk_lists(con
         if (lane == 0) idx = int32_t(atomicAdd(work_ctr, 1u));
         idx = __shfl_sync(kFull, idx, 0);
         if (idx >= items) break;
-        const int part = kSplit ? idx % nparts : 0;
-        if constexpr (kSplit) idx /= nparts;
+        const int rank = kSplit ? idx / ng : 0;
+        if constexpr (kSplit) idx %= ng;
         const int32_t g = lpt ? gperm[idx] : idx;
-        const int32_t s_lo = kSplit ? int32_t(int64_t(ns) * part / nparts) : 0;
-        const int32_t s_hi = kSplit ? int32_t(int64_t(ns) * (part + 1) / nparts) : ns;
         const GroupRange R = group_range<kG>(g, groups, nt);
         if (R.cnt <= 0) continue;
+        const int part = kSplit ? split_part(rank, targets ? targets[R.base] : R.base, ns, nparts) : 0;
+        const int32_t s_lo = kSplit ? int32_t(int64_t(ns) * part / nparts) : 0;
+        const int32_t s_hi = kSplit ? int32_t(int64_t(ns) * (part + 1) / nparts) : ns;
         GroupStars<kS> G;
         group_stars<kS>(lane, R, targets, st_hi, st_lo, G);
         const GroupBox B = group_box<kS>(lane, R.cnt, G.t, eps);
@@ -1095,12 +1110,13 @@ __global__ __launch_bounds__(kLwThreads) void k_walk_lists_adj(const DevInfo *in
         if (lane == 0) idx = int32_t(atomicAdd(work_ctr, 1u));
         idx = __shfl_sync(kFull, idx, 0);
         if (idx >= items) break;
-        const int part = kSplit ? idx % nparts : 0;
-        if constexpr (kSplit) idx /= nparts;
-        const int32_t s_lo = kSplit ? int32_t(int64_t(ns) * part / nparts) : 0;
-        const int32_t s_hi = kSplit ? int32_t(int64_t(ns) * (part + 1) / nparts) : ns;
+        const int rank = kSplit ? idx / ng : 0;
+        if constexpr (kSplit) idx %= ng;
         const GroupRange R = group_range<kG>(idx, nullptr, ns);
         if (R.cnt <= 0) continue;
+        const int part = kSplit ? split_part(rank, R.base, ns, nparts) : 0;
+        const int32_t s_lo = kSplit ? int32_t(int64_t(ns) * part / nparts) : 0;
+        const int32_t s_hi = kSplit ? int32_t(int64_t(ns) * (part + 1) / nparts) : ns;
         GroupStars<kS> G;
         group_stars<kS>(lane, R, nullptr, st_hi, st_lo, G);
         const GroupBox B = group_box<kS>(lane, R.cnt, G.t, eps);
