@@ -911,9 +911,11 @@ __device__ __forceinline__ double pair_potential(double mi, double mj, double r2
 // order. Bound by the FP64 pipe (about 28 operations a pair). A block takes T rows, few enough
 // that the blocks fill every SM several times over (the rows shorten, so the longest blocks are
 // launched first and the short ones fill the end). 30,000 bodies: 44.8 ms with one thread a row
-// and one thread adding the rows from global memory, 28.3 ms so.
+// and one thread adding the rows from global memory, 28.3 ms so, 25.8 without a radius to form and
+// compare (kNewton: every pair, when there is no speed of light).
 constexpr int kPotRows = 32, kPotJ = 64;
 constexpr int kPotStride = kPotJ + 1;
+template <bool kNewton>
 __global__ __launch_bounds__(kDirCompute + 32) void k_pot_exact_rows(int64_t n, const double *__restrict__ px,
                                                                      const double *__restrict__ py,
                                                                      const double *__restrict__ pz,
@@ -961,9 +963,10 @@ __global__ __launch_bounds__(kDirCompute + 32) void k_pot_exact_rows(int64_t n, 
                 const double dx = xj - s_x[k], dy = yj - s_y[k], dz = zj - s_z[k];
                 const uint8_t ki = s_k[k];
                 const double mi = s_m[k];
-                const double rs = pair_rs(ki, mi, kj, mj, c);
                 const double smi = dm_off && ki == GBH_DARK_MATTER ? 0.0 : mi;
-                const double v = pair_potential(smi, smj, dx * dx + dy * dy + dz * dz, eps2, rs);
+                const double r2 = dx * dx + dy * dy + dz * dz;
+                const double v = kNewton ? -smi * smj / sqrt(r2 + eps2)
+                                         : pair_potential(smi, smj, r2, eps2, pair_rs(ki, mi, kj, mj, c));
                 s_term[t & 1][k][jj] = j < n && j > i0 + k ? v : 0.0;
             }
         } else if (adder && t > 0 && a < nt) {
@@ -1397,8 +1400,9 @@ cudaError_t potential_exact_fp64(const Launch &L, int64_t n, const double *px, c
     // about four blocks a SM or more
     const int64_t per = n / (4 * int64_t(L.num_sms > 0 ? L.num_sms : 152));
     const int T = int(per < 1 ? 1 : per > kPotRows ? kPotRows : per);
-    k_pot_exact_rows<<<blocks_for(n, T), kDirCompute + 32, 0, L.stream>>>(n, px, py, pz, mass, kind, eps2, c, dm_off, T,
-                                                                          rows);
+    // without a speed of light every pair is Newtonian (pair.go:14-23): no radius to form and compare
+    auto *kernel = c <= 0 ? k_pot_exact_rows<true> : k_pot_exact_rows<false>;
+    kernel<<<blocks_for(n, T), kDirCompute + 32, 0, L.stream>>>(n, px, py, pz, mass, kind, eps2, c, dm_off, T, rows);
     GBH_LAUNCH_CHECK();
     k_pot_exact_final<<<1, kThreads, 0, L.stream>>>(n, rows, u_dev);
     GBH_LAUNCH_CHECK();

@@ -47,7 +47,7 @@ def upload(ctx, s):
 def test_exact_potential_bit_identical(ctx, n):
     s = disk(n)
     upload(ctx, s)
-    for dm_off, c in ((False, 0.0), (True, 4.0)):
+    for dm_off, c in ((False, 0.0), (True, 0.0), (True, 4.0), (False, 4.0), (False, -1.0)):
         d = ctx.diagnostics(abi.make_params(0.5, 0.03, 8, False, dm_off, "mixed"), c)
         assert d["quality"] == 2
         assert d["potential"] == O.potential_exact(s["px"], s["py"], s["pz"], s["mass"], s["kind"], 0.03, c, dm_off)
