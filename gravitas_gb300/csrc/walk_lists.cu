@@ -287,6 +287,13 @@ __device__ __forceinline__ GroupOut walk_group(TravMem &W, Sink &sink, int lane,
                                                const int2 *__restrict__ ranges = nullptr, int32_t s_lo = 0,
                                                int32_t s_hi = 0) {
     using Lay = Layout<kExact>;
+    // A node's whole record at once: measured faster with two stars a lane, and for a part, whose few
+    // steps wait for their loads (its range test no longer goes before them: 16,384-star Plummer walk
+    // 0.111 -> 0.103 ms, with the rest of the record and the root below 0.098; 60,000 0.294 -> 0.285).
+    // What a split walk does not gain from, measured here: one warp traversing and the block's other
+    // one evaluating (0.104 and 0.34 ms), the next item drawn ahead (0.128, 0.39), 9 or 11 blocks per
+    // SM, longer unrolls, two staging rounds' loads in flight (within 2 %).
+    constexpr bool kAll = kS == 2 || kSplit;
     constexpr int kNodeFields = kExact ? 13 : 10;
     constexpr int kSrcFields = kExact ? 7 : 4;
     const unsigned lt = (1u << lane) - 1u, upto = kFull >> (31 - lane);
@@ -329,6 +336,32 @@ __device__ __forceinline__ GroupOut walk_group(TravMem &W, Sink &sink, int lane,
     const float2 smx = make_float2(-__shfl_sync(kFull, t[0].tx, 0), -__shfl_sync(kFull, t[kS - 1].tx, 31));
     const float2 smy = make_float2(-__shfl_sync(kFull, t[0].ty, 0), -__shfl_sync(kFull, t[kS - 1].ty, 31));
     const float2 smz = make_float2(-__shfl_sync(kFull, t[0].tz, 0), -__shfl_sync(kFull, t[kS - 1].tz, 31));
+    if constexpr (kSplit) {
+        // A part's walk has few steps, so the root, which every group but a far one opens, gets no
+        // step of its own where the two stars settle it (the whole test decides the same).
+        const float4 ra = nodes[root].a, rb = nodes[root].b;  // root < nn: no group of an empty tree
+        const uint32_t rl = __float_as_uint(rb.w);
+        const float rx = (ra.x - Ox) + rb.x, ry = (ra.y - Oy) + rb.y, rz = (ra.z - Oz) + rb.z;
+        const float slack = (fmaxf(fabsf(rx), fmaxf(fabsf(ry), fabsf(rz))) + ext) * 4.2e-7f;
+        const float crit = fabsf(ra.w);
+        const float cr = fmaf(crit, 9.6e-7f, crit) + slack;
+        const float rlim = cr * cr * (1.f + 4.8e-7f);
+        const float2 ex = add2(f2(rx), smx), ey = add2(f2(ry), smy), ez = add2(f2(rz), smz);
+        const float2 d2 = fma2(ez, ez, fma2(ey, ey, mul2(ex, ex)));
+        const float qx = fmaxf(0.f, fmaxf(bx0 - rx, rx - bx1));
+        const float qy = fmaxf(0.f, fmaxf(by0 - ry, ry - by1));
+        const float qz = fmaxf(0.f, fmaxf(bz0 - rz, rz - bz1));
+        if (!(ra.w < 0.f) && !(qx * qx + qy * qy + qz * qz >= rlim) && (d2.x < rlim || d2.y < rlim) &&
+            int64_t(rl & 0x1fffffffu) + int64_t(rl >> 29) + 1 <= nn) {
+            if (lane == 0) {
+                W.stack[0] = rl;
+                W.lvl[1] = 0;
+            }
+            dtop = 1;
+            tested = 1;
+            __syncwarp();
+        }
+    }
     while (sp > 0) {
         // ---- pop the sibling ranges of the deepest level, at most 32 nodes; lane j takes node j
         // of their concatenation (the range holding it is the last one starting at or before j)
@@ -355,23 +388,24 @@ __device__ __forceinline__ GroupOut walk_group(TravMem &W, Sink &sink, int lane,
         tested += uint32_t(total);
         // ---- test: the group's box, then (all lanes at once) every star for what the box keeps
         bool acc = false, bad = node >= nn, own = true;
-        if constexpr (kSplit) {
-            if (node >= 0 && !bad) {
-                const int2 rg = ranges[node];
-                if (rg.x >= s_hi || rg.y <= s_lo) node = -1;  // no star of this part below it
-                else own = rg.x >= s_lo;
-            }
-        }
         float4 na = make_float4(0.f, 0.f, 0.f, 0.f), nb = na, nc = na, nd = na;
         float cx = 0.f, cy = 0.f, cz = 0.f, lim = 0.f;
         bool keep = false;
         if (node >= 0 && !bad) {
+            int2 rg = make_int2(0, 0);
+            if constexpr (kSplit) rg = ranges[node];
             na = nodes[node].a;
             nb = nodes[node].b;
-            if constexpr (kS == 2) {  // the whole record at once (measured faster with two stars a lane)
+            if constexpr (kAll) {
                 nc = nodes[node].c;
                 nd = nodes[node].d;
             }
+            if constexpr (kSplit) {
+                if (rg.x >= s_hi || rg.y <= s_lo) node = -1;  // no star of this part below it
+                else own = rg.x >= s_lo;
+            }
+        }
+        if (node >= 0 && !bad) {
             cx = (na.x - Ox) + nb.x;
             cy = (na.y - Oy) + nb.y;
             cz = (na.z - Oz) + nb.z;
@@ -459,7 +493,7 @@ __device__ __forceinline__ GroupOut walk_group(TravMem &W, Sink &sink, int lane,
         if (ma) {
             if (add) {
                 const int en = ncount + __popc(ma & lt);
-                const float4 qc = kS == 2 ? nc : nodes[node].c, qd = kS == 2 ? nd : nodes[node].d;
+                const float4 qc = kAll ? nc : nodes[node].c, qd = kAll ? nd : nodes[node].d;
                 constexpr int P = Lay::kNodePair;
                 if constexpr (kExact) {
                     put(sink.nbuf, P, en, 0, na.x);
@@ -492,7 +526,7 @@ __device__ __forceinline__ GroupOut walk_group(TravMem &W, Sink &sink, int lane,
         const unsigned ml = __ballot_sync(kFull, open_leaf);
         if (ml) {
             int lo = open_leaf ? int(link) : 0;
-            int hi = open_leaf ? __float_as_int(kS == 2 ? nd.w : nodes[node].d.w) : 0;
+            int hi = open_leaf ? __float_as_int(kAll ? nd.w : nodes[node].d.w) : 0;
             if (__any_sync(kFull, open_leaf && (lo < 0 || hi > ns || lo >= hi))) {
                 if (lane == 0) set_err(err_info, 8);
                 return GroupOut{0, false};
