@@ -890,8 +890,8 @@ cudaError_t walk_lists_s(const Launch &L, const TreeBufs &b, int64_t nstars_cap,
 //     quadrupole component its derivative of w_i.a;
 //   leaf star j (softened pair, bh.go:145-150): K = I / r^3 - 3 d d^T / r^5, star i gets -m_j K w_i,
 //     star j gets +m_j K w_i and (d.w_i) / r^3 on its mass; a star paired with itself adds nothing.
-// Each warp sums a list entry's source terms over its 32 stars (a reduce-scatter: lane l ends
-// with term l) and adds them to the node's or star's FP64 accumulators with atomics.
+// Each warp sums a list entry's source terms over its 32 stars (a reduce-scatter: each lane ends
+// with one term) and adds them to the node's or star's FP64 accumulators with atomics.
 
 constexpr int kAdjNodeTerms = 10;  // centre of mass (3), mass, Q xx yy zz xy xz yz
 constexpr int kAdjStarTerms = 4;   // position (3), mass
@@ -902,36 +902,43 @@ struct AdjAcc {
     double gx, gy, gz;    // its own terms, summed over the flushed lists
 };
 
-// Sums v[0..31] over the warp; afterwards lane l holds the sum of term l in v[0].
-__device__ __forceinline__ void reduce_scatter32(float (&v)[32], int lane) {
+// Reduce-scatters over the warp: at each step a lane sends half of its terms' partial sums to the
+// lane 16, 8, ... away and takes the other half's, so a term's sum is the same tree over the lanes
+// wherever it ends. The upper lane keeps the upper terms; an odd count leaves it one fewer.
+template <int kLower, int kUpper>
+__device__ __forceinline__ void scatter_step(float *v, int lane, int sft) {
+    const bool up = (lane & sft) != 0;
 #pragma unroll
-    for (int sft = 16; sft >= 1; sft >>= 1) {
-        const bool up = (lane & sft) != 0;
-#pragma unroll
-        for (int i = 0; i < sft; ++i) {
-            const float send = up ? v[i] : v[i + sft];
-            const float keep = up ? v[i + sft] : v[i];
-            v[i] = keep + __shfl_xor_sync(kFull, send, sft);
-        }
+    for (int i = 0; i < kLower; ++i) {
+        const float hi = i < kUpper ? v[kLower + i] : 0.f;
+        const float send = up ? v[i] : hi;
+        const float keep = up ? hi : v[i];
+        v[i] = keep + __shfl_xor_sync(kFull, send, sft);
     }
 }
-// The same for 8 terms: full sums over the two upper lane bits, then a scatter over the lower
-// three (lane l < 8 ends with term l).
-__device__ __forceinline__ void reduce_scatter8(float (&v)[8], int lane) {
-#pragma unroll
-    for (int sft = 16; sft >= 8; sft >>= 1)
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] += __shfl_xor_sync(kFull, v[i], sft);
-#pragma unroll
-    for (int sft = 4; sft >= 1; sft >>= 1) {
-        const bool up = (lane & sft) != 0;
-#pragma unroll
-        for (int i = 0; i < sft; ++i) {
-            const float send = up ? v[i] : v[i + sft];
-            const float keep = up ? v[i + sft] : v[i];
-            v[i] = keep + __shfl_xor_sync(kFull, send, sft);
-        }
-    }
+// Two nodes' terms (21 shuffles; 31 for a power of two of terms): afterwards v[0] of the lane is the
+// sum of term pair_term(lane), if that is not negative.
+static_assert(2 * kAdjNodeTerms == 20 && 4 * kAdjStarTerms == 16, "the scatters' halves");
+__device__ __forceinline__ void reduce_scatter20(float (&v)[20], int lane) {
+    scatter_step<10, 10>(v, lane, 16);
+    scatter_step<5, 5>(v, lane, 8);
+    scatter_step<3, 2>(v, lane, 4);
+    scatter_step<2, 1>(v, lane, 2);
+    scatter_step<1, 1>(v, lane, 1);
+}
+__device__ __forceinline__ int pair_term(int lane) {
+    const int low = lane & 7;  // 0 1 2 - 3 4 - -
+    if (low == 3 || low >= 6) return -1;
+    return 10 * (lane >> 4) + 5 * (lane >> 3 & 1) + (low < 4 ? low : low - 1);
+}
+// Four stars' terms: scattered over the four upper lane bits, then a full sum over the last (16
+// shuffles). Lane l holds the sum of term l / 2.
+__device__ __forceinline__ void reduce_scatter16(float (&v)[16], int lane) {
+    scatter_step<8, 8>(v, lane, 16);
+    scatter_step<4, 4>(v, lane, 8);
+    scatter_step<2, 2>(v, lane, 4);
+    scatter_step<1, 1>(v, lane, 2);
+    v[0] += __shfl_xor_sync(kFull, v[0], 1);
 }
 
 struct AdjSink {
@@ -949,6 +956,7 @@ struct AdjSink {
         static_assert(kQuad && kSoft, "the adjoint walk: quadrupoles, softening");
         using Lay = Layout<kExact>;
         const float2 e2 = f2(eps2);
+        const int my = pair_term(lane);
         float2 gx[kS], gy[kS], gz[kS];
 #pragma unroll
         for (int q = 0; q < kS; ++q) gx[q] = gy[q] = gz[q] = f2(0.f);
@@ -966,9 +974,9 @@ struct AdjSink {
             const float2 m = hi2(r1);
             // the record holds -Q: n = -Q
             const float2 nxx = lo2(r2a), nyy = hi2(r2a), nzz = lo2(r3), nxy = hi2(r3), nxz = lo2(r4), nyz = hi2(r4);
-            float v[32];
+            float v[2 * kAdjNodeTerms];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = 0.f;
+            for (int i = 0; i < 2 * kAdjNodeTerms; ++i) v[i] = 0.f;
 #pragma unroll
             for (int q = 0; q < kS; ++q) {
                 const Target &t = tt[q];
@@ -1018,10 +1026,10 @@ struct AdjSink {
                 }
             }
             const bool hasB = 2 * p + 1 < count;  // the padded last entry is no node
-            reduce_scatter32(v, lane);
-            if (lane < kAdjNodeTerms || (hasB && lane < 2 * kAdjNodeTerms)) {
-                const int e = 2 * p + (lane >= kAdjNodeTerms ? 1 : 0);
-                const int term = lane >= kAdjNodeTerms ? lane - kAdjNodeTerms : lane;
+            reduce_scatter20(v, lane);
+            if (my >= 0 && (hasB || my < kAdjNodeTerms)) {
+                const int e = 2 * p + (my >= kAdjNodeTerms ? 1 : 0);
+                const int term = my >= kAdjNodeTerms ? my - kAdjNodeTerms : my;
                 atomicAdd(&nadj[int64_t(nidx[e]) * kAdjNodeTerms + term], double(v[0]));
             }
         }
@@ -1043,60 +1051,62 @@ struct AdjSink {
 #pragma unroll
         for (int q = 0; q < kS; ++q) gx[q] = gy[q] = gz[q] = f2(0.f);
         const int np = (count + 1) >> 1;
-        for (int p = 0; p < np; ++p) {
-            const float4 *r = &sbuf[p * Lay::kSrcPair];
-            const float4 r0 = r[0], r1 = r[1];
-            float2 lx = f2(0.f), ly = f2(0.f), lz = f2(0.f);
-            if constexpr (kExact) {
-                const float4 r2a = r[2], r3 = r[3];
-                lx = lo2(r2a);
-                ly = hi2(r2a);
-                lz = lo2(r3);
-            }
-            const bool hasB = 2 * p + 1 < count;
-            const int32_t sA = sidx[2 * p], sB = hasB ? sidx[2 * p + 1] : -1;
-            float v[8];
+        // two pairs of stars at once: their chains overlap, and one reduction serves four stars
+        for (int p = 0; p < np; p += 2) {
+            float v[4 * kAdjStarTerms];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = 0.f;
+            for (int i = 0; i < 4 * kAdjStarTerms; ++i) v[i] = 0.f;
 #pragma unroll
-            for (int q = 0; q < kS; ++q) {
-                const Target &t = tt[q];
-                const float2 wx = f2(aa[q].wx), wy = f2(aa[q].wy), wz = f2(aa[q].wz);
-                const float2 dx = sep<kExact>(lo2(r0), lx, -t.tx, -t.hx, -t.lx);
-                const float2 dy = sep<kExact>(hi2(r0), ly, -t.ty, -t.hy, -t.ly);
-                const float2 dz = sep<kExact>(lo2(r1), lz, -t.tz, -t.hz, -t.lz);
-                const float2 rr = fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, e2)));
-                const float2 ir = make_float2(rsqrtf(rr.x), rsqrtf(rr.y));
-                const float2 ir2 = mul2(ir, ir), ir3 = mul2(ir2, ir), ir5 = mul2(ir3, ir2);
-                // a star and its own pair, and the padded last entry, contribute nothing
-                const float keepA = sA == aa[q].k ? 0.f : 1.f;
-                const float keepB = hasB && sB != aa[q].k ? 1.f : 0.f;
-                const float2 m = mul2(hi2(r1), make_float2(keepA, keepB));
-                const float2 dw = fma2(dz, wz, fma2(dy, wy, mul2(dx, wx)));
-                // m K w = m (w / r^3 - 3 d dw / r^5)
-                const float2 c3 = mul2(mul2(ir5, dw), f2(-3.f));
-                const float2 kx = mul2(m, fma2(c3, dx, mul2(ir3, wx)));
-                const float2 ky = mul2(m, fma2(c3, dy, mul2(ir3, wy)));
-                const float2 kz = mul2(m, fma2(c3, dz, mul2(ir3, wz)));
-                gx[q] = add2(gx[q], kx);
-                gy[q] = add2(gy[q], ky);
-                gz[q] = add2(gz[q], kz);
-                const float2 am = mul2(mul2(dw, ir3), make_float2(keepA, keepB));
-                v[0] += kx.x;
-                v[1] += ky.x;
-                v[2] += kz.x;
-                v[3] += am.x;
-                v[4] += kx.y;
-                v[5] += ky.y;
-                v[6] += kz.y;
-                v[7] += am.y;
+            for (int u = 0; u < 2; ++u) {
+                const bool has = p + u < np;  // else the last pair again, for nothing
+                const int pu = has ? p + u : p;
+                const float4 *r = &sbuf[pu * Lay::kSrcPair];
+                const float4 r0 = r[0], r1 = r[1];
+                float2 lx = f2(0.f), ly = f2(0.f), lz = f2(0.f);
+                if constexpr (kExact) {
+                    const float4 r2a = r[2], r3 = r[3];
+                    lx = lo2(r2a);
+                    ly = hi2(r2a);
+                    lz = lo2(r3);
+                }
+                const int32_t sA = sidx[2 * pu], sB = 2 * pu + 1 < count ? sidx[2 * pu + 1] : -1;
+#pragma unroll
+                for (int q = 0; q < kS; ++q) {
+                    const Target &t = tt[q];
+                    const float2 wx = f2(aa[q].wx), wy = f2(aa[q].wy), wz = f2(aa[q].wz);
+                    const float2 dx = sep<kExact>(lo2(r0), lx, -t.tx, -t.hx, -t.lx);
+                    const float2 dy = sep<kExact>(hi2(r0), ly, -t.ty, -t.hy, -t.ly);
+                    const float2 dz = sep<kExact>(lo2(r1), lz, -t.tz, -t.hz, -t.lz);
+                    const float2 rr = fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, e2)));
+                    const float2 ir = make_float2(rsqrtf(rr.x), rsqrtf(rr.y));
+                    const float2 ir2 = mul2(ir, ir), ir3 = mul2(ir2, ir), ir5 = mul2(ir3, ir2);
+                    // a star and its own pair, and the padded last entry, contribute nothing
+                    const float keepA = has && sA != aa[q].k ? 1.f : 0.f;
+                    const float keepB = has && sB >= 0 && sB != aa[q].k ? 1.f : 0.f;
+                    const float2 m = mul2(hi2(r1), make_float2(keepA, keepB));
+                    const float2 dw = fma2(dz, wz, fma2(dy, wy, mul2(dx, wx)));
+                    // m K w = m (w / r^3 - 3 d dw / r^5)
+                    const float2 c3 = mul2(mul2(ir5, dw), f2(-3.f));
+                    const float2 kx = mul2(m, fma2(c3, dx, mul2(ir3, wx)));
+                    const float2 ky = mul2(m, fma2(c3, dy, mul2(ir3, wy)));
+                    const float2 kz = mul2(m, fma2(c3, dz, mul2(ir3, wz)));
+                    gx[q] = add2(gx[q], kx);
+                    gy[q] = add2(gy[q], ky);
+                    gz[q] = add2(gz[q], kz);
+                    const float2 am = mul2(mul2(dw, ir3), make_float2(keepA, keepB));
+                    v[8 * u + 0] += kx.x;
+                    v[8 * u + 1] += ky.x;
+                    v[8 * u + 2] += kz.x;
+                    v[8 * u + 3] += am.x;
+                    v[8 * u + 4] += kx.y;
+                    v[8 * u + 5] += ky.y;
+                    v[8 * u + 6] += kz.y;
+                    v[8 * u + 7] += am.y;
+                }
             }
-            reduce_scatter8(v, lane);
-            if (lane < kAdjStarTerms || (hasB && lane < 2 * kAdjStarTerms)) {
-                const int e = 2 * p + (lane >= kAdjStarTerms ? 1 : 0);
-                const int term = lane >= kAdjStarTerms ? lane - kAdjStarTerms : lane;
-                atomicAdd(&sadj[int64_t(sidx[e]) * kAdjStarTerms + term], double(v[0]));
-            }
+            reduce_scatter16(v, lane);
+            if (!(lane & 1) && 2 * p + (lane >> 3) < count)
+                atomicAdd(&sadj[int64_t(sidx[2 * p + (lane >> 3)]) * kAdjStarTerms + (lane >> 1 & 3)], double(v[0]));
         }
 #pragma unroll
         for (int q = 0; q < kS; ++q) {
@@ -1115,12 +1125,16 @@ struct __align__(16) AdjWarpMem {
     TravMem tm;
 };
 
+// Bound by latency (3.4 warps a scheduler, issue slots half busy) and by the shuffles and selects of
+// the reductions: with 31 shuffles for two nodes' terms and 23 for two stars' (now 21, and 16 for
+// four stars'), 32,768 bodies' walk took 0.593 ms, 0.50 so; 100,000 bodies' gradient 21.4 -> 19.3 ms.
+// Eight blocks per SM (128 registers); ten fit in 96 without a spill, but are 4 % slower.
 // The adjoint walk over groups of 32 kS stars (the forward's groups in adjoint mode): the same
 // traversal as k_walk_lists<quad, soft, kS, kSplit>, with the adjoint sink. w: the weights in
 // state order (three arrays); tgt: each sorted star's own terms (3 doubles), or with kSplit each
 // part's by sorted index in part_tgt (k_adj_part_combine adds the parts).
 template <int kS, bool kSplit>
-__global__ __launch_bounds__(kLwThreads) void k_walk_lists_adj(const DevInfo *info, const LNode *__restrict__ nodes,
+__global__ __launch_bounds__(kLwThreads, kS == 1 ? 8 : 1) void k_walk_lists_adj(const DevInfo *info, const LNode *__restrict__ nodes,
                                                                const float4 *__restrict__ st_hi,
                                                                const float4 *__restrict__ st_lo,
                                                                const int32_t *__restrict__ order, float eps,
