@@ -75,3 +75,14 @@ def test_hole_steps_bit_identical(ctx, n, nholes, scale):
     O.split_kdk(ref, 4e-3, 0.06, 0.5, 8, 3, acc_valid=True)
     for k in f9:
         assert np.array_equal(got[k], ref[k]), k
+
+
+@pytest.mark.parametrize("n", [1, 5, 2432, 2433, 4863, 4865, 9728, 9729, 12001])
+def test_fp64_walk_bit_identical(ctx, n):
+    """4, 8, 16 and 32 stars a warp, the last warp full or not."""
+    s = disk(n)
+    got = [np.zeros(n) for _ in range(3)]
+    ctx.call("gbh_accelerations", abi.make_params(0.7, 0.03, 8, walk="fp64"), n, P(s["px"]), P(s["py"]), P(s["pz"]),
+             P(s["mass"]), P(s["kind"]), P(s["alive"]), *[P(g) for g in got])
+    tree = O.Tree(s["px"], s["py"], s["pz"], s["mass"], s["kind"], s["alive"], theta=0.7, leaf=8)
+    assert np.array_equal(np.stack(got, 1), tree.accelerations(0.03))
