@@ -321,7 +321,7 @@ cudaError_t scan_u32(const Launch &L, const uint32_t *in, uint32_t *out, int64_t
                      uint32_t *tmp, int64_t tmp_cap);
 int64_t scan_tmp_size(int64_t n);
 
-// Stable Morton order of the alive non-hole bodies (collect, keys and radix sort of tree_build)
+// Stable Morton order of the alive non-hole bodies (collect, keys and sort of tree_build)
 // with all temporaries in one caller-provided device block of scratch_bytes; keys/order get the
 // sorted keys and state indices, *info_out points at the DevInfo inside the block.
 size_t morton_sort_scratch_bytes(int64_t nmax);

@@ -5,7 +5,7 @@
 // fails or fragments that pool), code that must not take the device-wide synchronisation that
 // cudaMalloc/cudaFree can imply while other streams are running, and fixed-budget loops that
 // must never allocate after start-up. They already own their inputs and outputs.
-// gbh_morton_order_noalloc serves them: it runs the collect, Morton-key and stable radix-sort
+// gbh_morton_order_noalloc serves them: it runs the collect, Morton-key and stable sort
 // kernels of the tree build with every temporary taken from one file-scope device array
 // (g_scratch) instead of an allocation.
 //
@@ -103,7 +103,7 @@ extern "C" int gbh_morton_order_noalloc(int32_t device, void *stream, int64_t n,
     if (e != cudaSuccess) return report_cuda(err, errlen, "Morton ordering", e);
     if (h.err && h.err_where == gbh::kErrNonFinite)
         return report(err, errlen, GBH_ERR_ARG, "an alive star has a non-finite position (outputs are undefined)");
-    if (h.err) return report(err, errlen, GBH_ERR_LIMIT, "device-side consistency check failed in the radix sort");
+    if (h.err) return report(err, errlen, GBH_ERR_LIMIT, "device-side consistency check failed in the sort");
     *nstars = n > 0 ? h.nstars : 0;
     return GBH_OK;
 }

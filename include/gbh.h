@@ -392,7 +392,7 @@ int gbh_probe_fp32_peak(gbh_ctx *ctx, double ms, double *tflops);
  *
  * Sorted Morton keys and state indices of the alive non-hole bodies, exactly the keys and
  * order gbh_tree_export returns after gbh_accelerations on the same arrays (collect, keys
- * and the stable radix sort of the tree build). All pointers except nstars, err and stream
+ * and the stable sort of the tree build). All pointers except nstars, err and stream
  * are device pointers owned by the caller: px/py/pz hold n doubles, kind/alive n bytes (each
  * may be NULL: all stars, all alive), keys and order room for n entries; *nstars (host)
  * receives the number of sorted bodies. stream is a cudaStream_t (NULL: the legacy default
