@@ -18,13 +18,6 @@ namespace {
 constexpr int kEw = 256;
 constexpr int kHoleChunk = 256;
 
-#define SPLIT_LAUNCH_CHECK()                 \
-    do {                                     \
-        ++*L.count;                          \
-        cudaError_t e_ = cudaGetLastError(); \
-        if (e_ != cudaSuccess) return e_;    \
-    } while (0)
-
 inline unsigned ew_blocks(int64_t n) { return unsigned(std::max<int64_t>(1, (n + kEw - 1) / kEw)); }
 
 // pair.go:26-35 (PairForce): f such that the acceleration is f d; capped inside 1.5 rs.
@@ -88,6 +81,7 @@ __global__ void k_classify(int64_t n, const double *__restrict__ px, const doubl
                            const uint8_t *__restrict__ kind, const int32_t *__restrict__ holes, int32_t nh,
                            double eps2, double c, double limit, uint8_t *near8, uint32_t *near32,
                            unsigned long long *tau_bits) {
+    pdl_begin();
     __shared__ double smin[kEw / 32];
     int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     double local = __longlong_as_double(0x7ff0000000000000LL);
@@ -122,6 +116,7 @@ __global__ void k_classify(int64_t n, const double *__restrict__ px, const doubl
 // Near list in index order from the exclusive scan of the flags; out[1] = its length.
 __global__ void k_near_list(int64_t n, const uint8_t *__restrict__ near8, const uint32_t *__restrict__ scan,
                             int32_t *near, unsigned long long *out) {
+    pdl_begin();
     int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     if (near8[i]) near[scan[i]] = int32_t(i);
@@ -146,6 +141,7 @@ __global__ __launch_bounds__(kHoleChunk) void k_far_part(int64_t n, const double
                                                          const uint8_t *__restrict__ near8, int dm_off,
                                                          const int32_t *__restrict__ holes, int32_t nh, double eps2,
                                                          double c, double *fx, double *fy, double *fz, double *part) {
+    pdl_begin();
     __shared__ double s_term[3 * kHoleBatch][kTermStride];
     const int64_t i = int64_t(blockIdx.x) * kHoleChunk + threadIdx.x;
     const bool far = i < n && kind[i] != GBH_BLACK_HOLE && !near8[i];
@@ -204,6 +200,7 @@ __global__ __launch_bounds__(kEw) void k_kick_outer(int64_t n, double h, bool dr
                                                     const double *__restrict__ fy, const double *__restrict__ fz,
                                                     const int32_t *__restrict__ holes, int32_t nh, int64_t nchunks,
                                                     const double *__restrict__ part) {
+    pdl_begin();
     const int64_t nb = int64_t(gridDim.x) - nh;
     if (int64_t(blockIdx.x) >= nb) {
         __shared__ double s[3][kEw + 1];
@@ -259,6 +256,7 @@ __global__ __launch_bounds__(kFastThreads) void k_fast(int32_t nnear, const int3
                                                        const int32_t *__restrict__ holes, int32_t nh, double eps2,
                                                        double c, bool kick, double h, double *vx, double *vy,
                                                        double *vz, double *fx, double *fy, double *fz) {
+    pdl_begin();
     if (int32_t(blockIdx.x) >= nh) {
         const int32_t q = (int32_t(blockIdx.x) - nh) * kFastThreads + threadIdx.x;
         if (q >= nnear) return;
@@ -326,6 +324,7 @@ __global__ void k_fast_open(int32_t nnear, const int32_t *__restrict__ near, con
                             int32_t nh, double h, double dt, double c, double *px, double *py, double *pz, double *vx,
                             double *vy, double *vz, const double *__restrict__ fx, const double *__restrict__ fy,
                             const double *__restrict__ fz) {
+    pdl_begin();
     int32_t q = int32_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (q >= nnear + nh) return;
     int32_t i = q < nnear ? near[q] : holes[q - nnear];
@@ -398,30 +397,26 @@ cudaError_t split_classify(const Launch &L, SplitBufs &s, int64_t n, const doubl
     static const unsigned long long kInit[2] = {0x7ff0000000000000ULL, 0};  // +inf, no near stars
     cudaError_t e = cudaMemcpyAsync(s.scalars, kInit, sizeof kInit, cudaMemcpyHostToDevice, L.stream);
     if (e != cudaSuccess) return e;
-    k_classify<<<ew_blocks(n), kEw, 0, L.stream>>>(n, px, py, pz, mass, kind, s.holes, s.nholes, eps2, c, limit,
-                                                   s.near8, s.near32, s.scalars);
-    SPLIT_LAUNCH_CHECK();
+    GBH_LAUNCH_AFTER(L, k_classify, ew_blocks(n), kEw, n, px, py, pz, mass, kind, s.holes, s.nholes, eps2, c, limit,
+                     s.near8, s.near32, s.scalars);
     if ((e = scan_u32(L, s.near32, s.near32, n, s.scan_tmp, s.scan_cap))) return e;
-    k_near_list<<<ew_blocks(n), kEw, 0, L.stream>>>(n, s.near8, s.near32, s.near, s.scalars);
-    SPLIT_LAUNCH_CHECK();
+    GBH_LAUNCH_AFTER(L, k_near_list, ew_blocks(n), kEw, n, s.near8, s.near32, s.near, s.scalars);
     return cudaSuccess;
 }
 
 cudaError_t split_outer(const Launch &L, SplitBufs &s, int64_t n, const double *px, const double *py,
                         const double *pz, const double *mass, const uint8_t *kind, int dm_off, double eps2, double c) {
-    k_far_part<<<unsigned((n + kHoleChunk - 1) / kHoleChunk), kHoleChunk, 0, L.stream>>>(
-        n, px, py, pz, mass, kind, s.near8, dm_off, s.holes, s.nholes, eps2, c, s.far, s.far + n, s.far + 2 * n, s.part);
-    SPLIT_LAUNCH_CHECK();
+    GBH_LAUNCH_AFTER(L, k_far_part, unsigned((n + kHoleChunk - 1) / kHoleChunk), kHoleChunk, n, px, py, pz, mass, kind,
+                     s.near8, dm_off, s.holes, s.nholes, eps2, c, s.far, s.far + n, s.far + 2 * n, s.part);
     return cudaSuccess;
 }
 
 cudaError_t split_kick_outer(const Launch &L, SplitBufs &s, int64_t n, double h, bool drift, double dt, double c,
                              const uint8_t *kind, double *px, double *py, double *pz, double *vx, double *vy,
                              double *vz, const double *ax, const double *ay, const double *az) {
-    k_kick_outer<<<ew_blocks(n) + unsigned(s.nholes), kEw, 0, L.stream>>>(
-        n, h, drift, dt, c, kind, s.near8, px, py, pz, vx, vy, vz, ax, ay, az, s.far, s.far + n, s.far + 2 * n, s.holes,
-        s.nholes, (n + kHoleChunk - 1) / kHoleChunk, s.part);
-    SPLIT_LAUNCH_CHECK();
+    GBH_LAUNCH_AFTER(L, k_kick_outer, ew_blocks(n) + unsigned(s.nholes), kEw, n, h, drift, dt, c, kind, s.near8, px,
+                     py, pz, vx, vy, vz, ax, ay, az, s.far, s.far + n, s.far + 2 * n, s.holes, s.nholes, (n +
+                     kHoleChunk - 1) / kHoleChunk, s.part);
     return cudaSuccess;
 }
 
@@ -429,18 +424,15 @@ cudaError_t split_fast(const Launch &L, SplitBufs &s, int64_t n, int32_t nnear, 
                        const double *py, const double *pz, double *vx, double *vy, double *vz, const double *mass,
                        const uint8_t *kind, int dm_off, double eps2, double c) {
     const unsigned nb = unsigned(s.nholes) + unsigned((nnear + kFastThreads - 1) / kFastThreads);
-    k_fast<<<nb, kFastThreads, 0, L.stream>>>(nnear, s.near, px, py, pz, mass, kind, dm_off, s.holes, s.nholes, eps2, c,
-                                              kick, h, vx, vy, vz, s.fast, s.fast + n, s.fast + 2 * n);
-    SPLIT_LAUNCH_CHECK();
+    GBH_LAUNCH_AFTER(L, k_fast, nb, kFastThreads, nnear, s.near, px, py, pz, mass, kind, dm_off, s.holes, s.nholes,
+                     eps2, c, kick, h, vx, vy, vz, s.fast, s.fast + n, s.fast + 2 * n);
     return cudaSuccess;
 }
 
 cudaError_t split_fast_open(const Launch &L, SplitBufs &s, int64_t n, int32_t nnear, double h, double dt, double c,
                             double *px, double *py, double *pz, double *vx, double *vy, double *vz) {
-    k_fast_open<<<ew_blocks(int64_t(nnear) + s.nholes), kEw, 0, L.stream>>>(nnear, s.near, s.holes, s.nholes, h, dt, c,
-                                                                            px, py, pz, vx, vy, vz, s.fast, s.fast + n,
-                                                                            s.fast + 2 * n);
-    SPLIT_LAUNCH_CHECK();
+    GBH_LAUNCH_AFTER(L, k_fast_open, ew_blocks(int64_t(nnear) + s.nholes), kEw, nnear, s.near, s.holes, s.nholes, h,
+                     dt, c, px, py, pz, vx, vy, vz, s.fast, s.fast + n, s.fast + 2 * n);
     return cudaSuccess;
 }
 
