@@ -603,15 +603,16 @@ int run_split_steps(gbh_ctx *ctx, const gbh_params *p, double dt, int64_t nsteps
         if (rc) return rc;
         ctx->acc_valid = true;
     }
-    unsigned long long sc[2];
     for (int64_t step = 0; step < nsteps; ++step) {
         // classify (split.go:39-85): the host needs the substep count
         CK(gbh::split_classify(L, sb, n, px, py, pz, ctx->mass, kind, eps2, c, 20.0 * dt));
-        CK(cudaMemcpyAsync(sc, sb.scalars, sizeof sc, cudaMemcpyDeviceToHost, ctx->stream));
         CK(wait_stream(ctx));
+        if (sb.host->info.err)
+            return fail(ctx, GBH_ERR_LIMIT, "device scan exceeded its wait bound (kernel %d)", sb.host->info.err_where);
+        const unsigned long long bits = ~sb.host->tau_inv;
         double tau_min;
-        std::memcpy(&tau_min, &sc[0], sizeof tau_min);
-        const int32_t nnear = int32_t(sc[1]);
+        std::memcpy(&tau_min, &bits, sizeof tau_min);
+        const int32_t nnear = int32_t(sb.host->nnear);
         int64_t k = 1;
         if (!std::isinf(tau_min))
             while (double(k) * tau_min < 20.0 * dt && k < 256) k *= 2;

@@ -316,10 +316,6 @@ int diag_parts();
 cudaError_t diagnostics(const Launch &L, int64_t n, const double *px, const double *py, const double *pz,
                         const double *vx, const double *vy, const double *vz, const double *mass, const uint8_t *kind,
                         double c, int dm_off, double *part, double *out);
-// Exclusive scan of n uint32 in place (in may equal out).
-cudaError_t scan_u32(const Launch &L, const uint32_t *in, uint32_t *out, int64_t n,
-                     uint32_t *tmp, int64_t tmp_cap);
-int64_t scan_tmp_size(int64_t n);
 
 // Stable Morton order of the alive non-hole bodies (collect, keys and sort of tree_build)
 // with all temporaries in one caller-provided device block of scratch_bytes; keys/order get the
@@ -330,22 +326,27 @@ cudaError_t morton_sort(const Launch &L, int64_t n, const double *px, const doub
                         size_t scratch_bytes, DevInfo **info_out);
 
 // ---- split.cu (the hole-aware step of split.go with c = 0) ----
+// What the host reads after split_classify.
+struct SplitScalars {
+    unsigned long long tau_inv;  // complement of the bits of the minimum timescale (0: none)
+    unsigned long long nnear;    // near stars
+    DevInfo info;                // err alone: the near list's look-back
+};
 struct SplitBufs {
     int32_t *holes = nullptr;  // alive holes, ascending state index
     int32_t nholes = 0, cap_holes = 0;
     uint8_t *near8 = nullptr;   // near flags
-    uint32_t *near32 = nullptr; // near flags, then their exclusive scan
     int32_t *near = nullptr;    // near stars, ascending
-    uint32_t *scan_tmp = nullptr;
-    int64_t scan_cap = 0;
     double *far = nullptr, *fast = nullptr;  // 3n each (x, y, z blocks)
     double *part = nullptr;                  // per 256-body chunk and hole: 3 partial sums
     int64_t cap_n = 0, cap_part = 0;
-    unsigned long long *scalars = nullptr;   // [0] bits of the minimum timescale, [1] near count
+    SplitScalars *scalars = nullptr;         // then the near list's tile counter and look-back words
+    size_t scalar_bytes = 0;
+    SplitScalars *host = nullptr;            // page-locked
 };
 cudaError_t split_reserve(SplitBufs &s, int64_t n, const std::vector<int32_t> &holes);
 void split_free(SplitBufs &s);
-// Near flags and list, minimum timescale (scalars) for the current positions.
+// Near flags and list, minimum timescale for the current positions; the scalars copied to s.host.
 cudaError_t split_classify(const Launch &L, SplitBufs &s, int64_t n, const double *px, const double *py,
                            const double *pz, const double *mass, const uint8_t *kind, double eps2, double c,
                            double limit);

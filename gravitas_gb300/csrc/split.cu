@@ -11,6 +11,7 @@
 #include <algorithm>
 
 #include "gbh_internal.cuh"
+#include "lookback.cuh"
 
 namespace gbh {
 namespace {
@@ -74,19 +75,27 @@ __device__ __forceinline__ double source_mass(int64_t i, const double *mass, con
     return dm_off && kind[i] == GBH_DARK_MATTER ? 0.0 : mass[i];  // Params.SourceMass, sim.go:93-98
 }
 
-// classify (split.go:39-85): near flags (byte and u32 for the scan) and the minimum timescale
-// (as the bits of a positive double, ordered like the value) over near stars and hole pairs.
-__global__ void k_classify(int64_t n, const double *__restrict__ px, const double *__restrict__ py,
-                           const double *__restrict__ pz, const double *__restrict__ mass,
-                           const uint8_t *__restrict__ kind, const int32_t *__restrict__ holes, int32_t nh,
-                           double eps2, double c, double limit, uint8_t *near8, uint32_t *near32,
-                           unsigned long long *tau_bits) {
+// classify (split.go:39-85): near flags, the near stars' list in index order, and the minimum
+// timescale over near stars and hole pairs (a positive double orders like its bits; their complement
+// is kept, so that the scalars start at 0). Blocks take tiles of 256 bodies in counter order and rank
+// their near stars by look-back. 20,002-body step with the list scanned and written by four more
+// launches 434 us, 420 so.
+__global__ __launch_bounds__(kEw) void k_classify(int64_t n, const double *__restrict__ px,
+                                                  const double *__restrict__ py, const double *__restrict__ pz,
+                                                  const double *__restrict__ mass, const uint8_t *__restrict__ kind,
+                                                  const int32_t *__restrict__ holes, int32_t nh, double eps2, double c,
+                                                  double limit, uint8_t *near8, int32_t *near, SplitScalars *out,
+                                                  unsigned long long *lb) {
     pdl_begin();
     __shared__ double smin[kEw / 32];
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    __shared__ uint32_t s_warp[kEw / 32 + 1], s_tile, s_prefix;
+    if (threadIdx.x == 0) s_tile = atomicAdd(reinterpret_cast<uint32_t *>(lb), 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    const int64_t i = int64_t(tile) * kEw + threadIdx.x;
     double local = __longlong_as_double(0x7ff0000000000000LL);
+    bool nr = false;
     if (i < n) {
-        bool nr = false;
         if (kind[i] != GBH_BLACK_HOLE)
             for (int32_t k = 0; k < nh; ++k) {
                 double tau = timescale(i, holes[k], px, py, pz, mass, kind, eps2, c);
@@ -96,31 +105,30 @@ __global__ void k_classify(int64_t n, const double *__restrict__ px, const doubl
                 }
             }
         near8[i] = nr;
-        near32[i] = nr;
     }
     for (int o = 16; o > 0; o >>= 1) local = fmin(local, __shfl_xor_sync(0xffffffffu, local, o));
     if ((threadIdx.x & 31) == 0) smin[threadIdx.x >> 5] = local;
+    uint32_t total;
+    const uint32_t at = block_excl_scan<kEw>(nr, s_warp, total);  // its barriers order smin too
+    if (threadIdx.x < 32) {
+        const unsigned long long before = look_back(lb + 1, tile, total, &out->info);
+        if (threadIdx.x == 0) {
+            s_prefix = uint32_t(before);
+            if ((int64_t(tile) + 1) * kEw >= n) out->nnear = before + total;
+        }
+    }
     __syncthreads();
+    if (nr) near[s_prefix + at] = int32_t(i);
     if (threadIdx.x == 0) {
-        for (int w = 1; w < int(blockDim.x >> 5); ++w) local = fmin(local, smin[w]);
-        if (blockIdx.x == 0)  // hole pairs: each with the mass of the later one (split.go:64-70)
+        for (int w = 1; w < kEw / 32; ++w) local = fmin(local, smin[w]);
+        if (tile == 0)  // hole pairs: each with the mass of the later one (split.go:64-70)
             for (int32_t a = 0; a < nh; ++a)
                 for (int32_t b = a + 1; b < nh; ++b) {
                     double tau = timescale(holes[a], holes[b], px, py, pz, mass, kind, eps2, c);
                     if (tau < limit) local = fmin(local, tau);
                 }
-        atomicMin(tau_bits, static_cast<unsigned long long>(__double_as_longlong(local)));
+        atomicMax(&out->tau_inv, ~static_cast<unsigned long long>(__double_as_longlong(local)));
     }
-}
-
-// Near list in index order from the exclusive scan of the flags; out[1] = its length.
-__global__ void k_near_list(int64_t n, const uint8_t *__restrict__ near8, const uint32_t *__restrict__ scan,
-                            int32_t *near, unsigned long long *out) {
-    pdl_begin();
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (near8[i]) near[scan[i]] = int32_t(i);
-    if (i == n - 1) out[1] = scan[i] + near8[i];
 }
 
 // outerHoleForces (split.go:83-116) of one 256-body chunk. Each body: far stars feel every hole;
@@ -341,9 +349,10 @@ __global__ void k_fast_open(int32_t nnear, const int32_t *__restrict__ near, con
 }  // namespace
 
 void split_free(SplitBufs &s) {
-    void *ptrs[] = {s.holes, s.near8, s.near32, s.near, s.scan_tmp, s.far, s.fast, s.part, s.scalars};
+    void *ptrs[] = {s.holes, s.near8, s.near, s.far, s.fast, s.part, s.scalars};
     for (void *p : ptrs)
         if (p) cudaFree(p);
+    if (s.host) cudaFreeHost(s.host);
     s = SplitBufs{};
 }
 
@@ -351,21 +360,19 @@ cudaError_t split_reserve(SplitBufs &s, int64_t n, const std::vector<int32_t> &h
     cudaError_t e = cudaSuccess;
     const int32_t nh = int32_t(holes.size());
     if (n > s.cap_n) {
-        void *ptrs[] = {s.near8, s.near32, s.near, s.scan_tmp, s.far, s.fast};
+        void *ptrs[] = {s.near8, s.near, s.far, s.fast, s.scalars};
         for (void *p : ptrs)
             if (p) cudaFree(p);
         s.near8 = nullptr;
-        s.near32 = nullptr;
         s.near = nullptr;
-        s.scan_tmp = nullptr;
+        s.scalars = nullptr;
         s.far = s.fast = nullptr;
         s.cap_n = 0;
         int64_t cap = n + n / 4;
-        s.scan_cap = scan_tmp_size(cap);
+        s.scalar_bytes = sizeof(SplitScalars) + sizeof(unsigned long long) * (1 + size_t(ew_blocks(cap)));
         if (e == cudaSuccess) e = dev_alloc(&s.near8, size_t(cap));
-        if (e == cudaSuccess) e = dev_alloc(&s.near32, sizeof(uint32_t) * size_t(cap));
         if (e == cudaSuccess) e = dev_alloc(&s.near, sizeof(int32_t) * size_t(cap));
-        if (e == cudaSuccess) e = dev_alloc(&s.scan_tmp, sizeof(uint32_t) * size_t(s.scan_cap));
+        if (e == cudaSuccess) e = dev_alloc(&s.scalars, s.scalar_bytes);
         if (e == cudaSuccess) e = dev_alloc(&s.far, sizeof(double) * 3 * size_t(cap));
         if (e == cudaSuccess) e = dev_alloc(&s.fast, sizeof(double) * 3 * size_t(cap));
         if (e != cudaSuccess) return e;
@@ -386,7 +393,7 @@ cudaError_t split_reserve(SplitBufs &s, int64_t n, const std::vector<int32_t> &h
         if ((e = dev_alloc(&s.holes, sizeof(int32_t) * size_t(nh)))) return e;
         s.cap_holes = nh;
     }
-    if (!s.scalars && (e = dev_alloc(&s.scalars, 2 * sizeof(unsigned long long)))) return e;
+    if (!s.host && (e = cudaMallocHost(&s.host, sizeof(SplitScalars)))) return e;
     s.nholes = nh;
     return cudaSuccess;
 }
@@ -394,14 +401,11 @@ cudaError_t split_reserve(SplitBufs &s, int64_t n, const std::vector<int32_t> &h
 cudaError_t split_classify(const Launch &L, SplitBufs &s, int64_t n, const double *px, const double *py,
                            const double *pz, const double *mass, const uint8_t *kind, double eps2, double c,
                            double limit) {
-    static const unsigned long long kInit[2] = {0x7ff0000000000000ULL, 0};  // +inf, no near stars
-    cudaError_t e = cudaMemcpyAsync(s.scalars, kInit, sizeof kInit, cudaMemcpyHostToDevice, L.stream);
+    cudaError_t e = cudaMemsetAsync(s.scalars, 0, s.scalar_bytes, L.stream);
     if (e != cudaSuccess) return e;
     GBH_LAUNCH_AFTER(L, k_classify, ew_blocks(n), kEw, n, px, py, pz, mass, kind, s.holes, s.nholes, eps2, c, limit,
-                     s.near8, s.near32, s.scalars);
-    if ((e = scan_u32(L, s.near32, s.near32, n, s.scan_tmp, s.scan_cap))) return e;
-    GBH_LAUNCH_AFTER(L, k_near_list, ew_blocks(n), kEw, n, s.near8, s.near32, s.near, s.scalars);
-    return cudaSuccess;
+                     s.near8, s.near, s.scalars, reinterpret_cast<unsigned long long *>(s.scalars + 1));
+    return cudaMemcpyAsync(s.host, s.scalars, sizeof(SplitScalars), cudaMemcpyDeviceToHost, L.stream);
 }
 
 cudaError_t split_outer(const Launch &L, SplitBufs &s, int64_t n, const double *px, const double *py,

@@ -41,110 +41,6 @@ inline unsigned blocks_for(int64_t n, int threads) {
     return unsigned(b < 1 ? 1 : b);
 }
 
-// ---------------------------------------------------------------- exclusive scan (uint32)
-
-__device__ __forceinline__ int64_t dyn_len(int64_t n, const int64_t *ndyn) {
-    if (ndyn) {
-        int64_t m = *ndyn;
-        return m < n ? m : n;
-    }
-    return n;
-}
-
-__global__ __launch_bounds__(kScanThreads) void k_scan_reduce(const uint32_t *__restrict__ in, int64_t n,
-                                                              const int64_t *ndyn, uint32_t *__restrict__ sums) {
-    __shared__ uint32_t s_warp[kScanThreads / 32 + 1];
-    int64_t ne = dyn_len(n, ndyn);
-    int64_t base = int64_t(blockIdx.x) * kScanTile + int64_t(threadIdx.x) * kScanItems;
-    uint32_t v = 0;
-    if (int64_t(blockIdx.x) * kScanTile < ne) {
-#pragma unroll
-        for (int k = 0; k < kScanItems; ++k)
-            if (base + k < ne) v += in[base + k];
-    }
-    uint32_t total;
-    block_excl_scan<kScanThreads>(v, s_warp, total);
-    if (threadIdx.x == 0) sums[blockIdx.x] = total;
-}
-
-__global__ __launch_bounds__(kScanThreads) void k_scan_apply(const uint32_t *in, uint32_t *out, int64_t n,
-                                                             const int64_t *ndyn, const uint32_t *__restrict__ sums) {
-    __shared__ uint32_t s_warp[kScanThreads / 32 + 1];
-    int64_t ne = dyn_len(n, ndyn);
-    if (int64_t(blockIdx.x) * kScanTile >= ne) return;
-    int64_t base = int64_t(blockIdx.x) * kScanTile + int64_t(threadIdx.x) * kScanItems;
-    uint32_t v[kScanItems];
-    uint32_t s = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        v[k] = base + k < ne ? in[base + k] : 0;
-        s += v[k];
-    }
-    uint32_t total;
-    uint32_t run = block_excl_scan<kScanThreads>(s, s_warp, total) + (sums ? sums[blockIdx.x] : 0);
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        if (base + k < ne) out[base + k] = run;
-        run += v[k];
-    }
-}
-
-// One block of kSingleThreads scanning up to kSingleThreads * kSingleItems entries in one launch
-// (each thread a run of consecutive entries): the small scans of a small build take one launch
-// instead of three.
-constexpr int kSingleThreads = 1024, kSingleItems = 8;
-__global__ __launch_bounds__(kSingleThreads) void k_scan_single(const uint32_t *in, uint32_t *out, int64_t n,
-                                                                const int64_t *ndyn) {
-    __shared__ uint32_t s_warp[kSingleThreads / 32];
-    const int64_t ne = dyn_len(n, ndyn);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t base = int64_t(threadIdx.x) * kSingleItems;
-    uint32_t v[kSingleItems];
-    uint32_t sum = 0;
-#pragma unroll
-    for (int k = 0; k < kSingleItems; ++k) {
-        v[k] = base + k < ne ? in[base + k] : 0;
-        sum += v[k];
-    }
-    const uint32_t incl = warp_incl_scan(sum);
-    if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        const uint32_t w = s_warp[lane];  // kSingleThreads / 32 == 32 warp totals
-        s_warp[lane] = warp_incl_scan(w) - w;
-    }
-    __syncthreads();
-    uint32_t run = s_warp[warp] + incl - sum;
-#pragma unroll
-    for (int k = 0; k < kSingleItems; ++k) {
-        if (base + k < ne) out[base + k] = run;
-        run += v[k];
-    }
-}
-
-cudaError_t scan_rec(const Launch &L, const uint32_t *in, uint32_t *out, int64_t n, const int64_t *ndyn,
-                     uint32_t *tmp, int64_t tmp_cap) {
-    int64_t tiles = (n + kScanTile - 1) / kScanTile;
-    if (tiles > 1 && n <= int64_t(kSingleThreads) * kSingleItems) {
-        k_scan_single<<<1, kSingleThreads, 0, L.stream>>>(in, out, n, ndyn);
-        ++*L.count;
-        return cudaGetLastError();
-    }
-    if (tiles <= 1) {
-        k_scan_apply<<<1, kScanThreads, 0, L.stream>>>(in, out, n, ndyn, nullptr);
-        ++*L.count;
-        return cudaGetLastError();
-    }
-    if (tiles > tmp_cap) return cudaErrorInvalidValue;
-    k_scan_reduce<<<unsigned(tiles), kScanThreads, 0, L.stream>>>(in, n, ndyn, tmp);
-    ++*L.count;
-    cudaError_t e = scan_rec(L, tmp, tmp, tiles, nullptr, tmp + tiles, tmp_cap - tiles);
-    if (e != cudaSuccess) return e;
-    k_scan_apply<<<unsigned(tiles), kScanThreads, 0, L.stream>>>(in, out, n, ndyn, tmp);
-    ++*L.count;
-    return cudaGetLastError();
-}
-
 // ---------------------------------------------------------------- node set (chains)
 
 // Sorted star range [lo, hi) of the system that sorted position i belongs to (the whole array
@@ -1112,16 +1008,6 @@ __global__ __launch_bounds__(128) void k_sys_groups(int32_t gsize, const uint32_
 }
 
 }  // namespace
-
-int64_t scan_tmp_size(int64_t n) {
-    int64_t total = 0;
-    for (int64_t t = (n + kScanTile - 1) / kScanTile; t > 1; t = (t + kScanTile - 1) / kScanTile) total += t;
-    return total + 64;
-}
-
-cudaError_t scan_u32(const Launch &L, const uint32_t *in, uint32_t *out, int64_t n, uint32_t *tmp, int64_t tmp_cap) {
-    return scan_rec(L, in, out, n, nullptr, tmp, tmp_cap);
-}
 
 void tree_free(TreeBufs &b) {
     void *ptrs[] = {b.pos4, b.bbox_part, b.keys, b.keys_alt, b.order, b.order_alt, b.lb_state, b.tile_len, b.hist, b.sx, b.sy, b.sz, b.sm,

@@ -53,7 +53,7 @@ def test_exact_potential_bit_identical(ctx, n):
         assert d["potential"] == O.potential_exact(s["px"], s["py"], s["pz"], s["mass"], s["kind"], 0.03, c, dm_off)
 
 
-@pytest.mark.parametrize("n,nholes,scale", [(3, 1, 1.0), (255, 2, 1.0), (257, 8, 0.3), (600, 15, 0.3), (1200, 3, 0.1)])
+@pytest.mark.parametrize("n,nholes,scale", [(3, 1, 1.0), (255, 2, 1.0), (256, 1, 0.1), (257, 8, 0.3), (512, 2, 0.1), (513, 2, 0.1), (600, 15, 0.3), (1200, 3, 0.1)])
 def test_hole_steps_bit_identical(ctx, n, nholes, scale):
     """Hole counts at the edges of the batches, few to all stars near a hole (scale shrinks the disk),
     a dead hole with an acceleration of its own."""
