@@ -404,15 +404,17 @@ __device__ __forceinline__ void bitonic_sort(uint64_t (&e)[kPer], uint64_t *s_e)
 }
 
 // Keys of a tile's bodies, sorted by (key, state index), its stars in front. The network sorts one
-// 64-bit word an element: the key's upper 54 bits (down to level 18 of 21) and the slot in the tile,
-// which settles equal keys by state index; dead bodies, holes and slots beyond the tile take the
-// largest words. Where neighbours agree in all 54 bits (levels 19 to 21 tell them apart, if
-// anything) each such run is then put in order by the lower 9 bits. Against (key, index) pairs
+// 64-bit word an element: 0, the key's upper 53 bits (down to the second axis of level 18 of 21) and
+// the slot in the tile, which settles equal keys by state index; dead bodies, holes and slots beyond
+// the tile have the top bit set, above every star (a star in the root cube's highest corner has a key
+// of all ones). Where neighbours agree in all 53 bits (levels 18 to 21 tell them apart, if
+// anything) each such run is then put in order by the whole key. Against (key, index) pairs
 // of three registers: 16,384 bodies 16.6 -> 11.6 us, the 1.1M-body forest 57 -> 40 (ncu, cold caches).
 // 1,024 bodies a tile spread a small state over more SMs than 2,048 would, and a million
 // bodies are 6.7 tiles a SM. pos4 (may be null): each star's position and mass in one record, for
 // the last merge's reads through the order.
 constexpr int kSlotBits = 10;
+constexpr uint64_t kNoStar = uint64_t(1) << 63;
 static_assert(kSortTile == 1 << kSlotBits, "a word holds the slot");
 template <bool kForest>
 __global__ __launch_bounds__(kThreads) void k_tile_sort(int64_t n, const int4 *__restrict__ tiles, int32_t ntiles,
@@ -449,8 +451,8 @@ __global__ __launch_bounds__(kThreads) void k_tile_sort(int64_t n, const int4 *_
             if (star) k = spread(cell(x, minx, sc)) << 2 | spread(cell(y, miny, sc)) << 1 | spread(cell(z, minz, sc));
         }
         s_key[slot] = k;
-        // a key has 63 bits: its upper 54 in bits 10 to 63; the largest words are no star's
-        e[j] = star ? (k >> 9) << kSlotBits | uint64_t(slot) : ~uint64_t(kSortTile - 1) | uint64_t(slot);
+        // a key has 63 bits: its upper 53 in bits 10 to 62, bit 63 for what is no star
+        e[j] = (star ? k >> kSlotBits << kSlotBits : kNoStar) | uint64_t(slot);
         cnt += __syncthreads_count(star);
     }
     bitonic_sort(e, s_e);
@@ -464,7 +466,7 @@ __global__ __launch_bounds__(kThreads) void k_tile_sort(int64_t n, const int4 *_
         tie |= 4 * t + j + 1 < cnt && (s_e[4 * t + j] >> kSlotBits) == (s_e[4 * t + j + 1] >> kSlotBits);
     if (__syncthreads_or(tie)) {
         // rank every element of a run of equal words by its whole key and slot (a run of m takes m
-        // steps a thread; only coincident or nearly coincident stars share 54 bits)
+        // steps a thread; only coincident or nearly coincident stars share 53 bits)
         int rank[kPer];
 #pragma unroll
         for (int j = 0; j < kPer; ++j) {
