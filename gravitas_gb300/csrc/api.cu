@@ -407,7 +407,7 @@ int forces(gbh_ctx *ctx, const gbh_params *p, int64_t n, const double *px, const
     Launch L = launch_of(ctx);
     int leaf = leaf_of(p);
     forest = forest && ctx->nsys > 1;
-    CK(gbh::tree_alloc(ctx->tb, n, leaf, forest ? ctx->nsys : 1));
+    CK(gbh::tree_alloc(ctx->tb, ctx->stream, n, leaf, forest ? ctx->nsys : 1));
     ctx->tb.group = group_of(p, n, forest);
     ctx->tb.list_depth = p->list_depth;
     ctx->tb.lpt = ctx->use_lpt;
@@ -647,7 +647,7 @@ int run_steps(gbh_ctx *ctx, const gbh_params *p, double dt, int64_t nsteps) {
     }
     if (ctx->use_graphs && nsteps > 0) {
         // One captured step per replay: the ~50 kernels of a step launch as one graph.
-        CK(gbh::tree_alloc(ctx->tb, n, leaf_of(p), ctx->nsys));  // any growth happens outside the capture
+        CK(gbh::tree_alloc(ctx->tb, ctx->stream, n, leaf_of(p), ctx->nsys));  // any growth happens outside the capture
         StepGraph &g = ctx->step_graph;
         if (!(g.exec && g.n == n && same_params(g.p, *p) && g.dt == dt && g.tree_gen == ctx->tb.generation &&
               g.state_gen == ctx->state_gen && g.sys_gen == ctx->sys_gen && g.kind == kind && g.alive == alive)) {
@@ -687,7 +687,7 @@ int event_build(gbh_ctx *ctx, const gbh_params *p, const uint8_t *kind, const ui
     Launch L = launch_of(ctx);
     int leaf = leaf_of(p);
     int64_t n = ctx->n;
-    CK(gbh::tree_alloc(ctx->tb, n, leaf));
+    CK(gbh::tree_alloc(ctx->tb, ctx->stream, n, leaf));
     CK(gbh::block_drift(L, ctx->tb, n, t, tick_len, p->c, ctx->px, ctx->py, ctx->pz, ctx->vx, ctx->vy, ctx->vz));
     ctx->tb.group = group_of(p, n, false);  // as the global step, so that one level is that step
     ctx->tb.list_depth = p->list_depth;
@@ -761,7 +761,7 @@ int run_block_steps(gbh_ctx *ctx, const gbh_params *p, double T, double eta, int
         if (rc) return rc;
         ctx->acc_valid = true;
     }
-    CK(gbh::tree_alloc(ctx->tb, n, leaf_of(p)));
+    CK(gbh::tree_alloc(ctx->tb, ctx->stream, n, leaf_of(p)));
     int rc;
     ctx->active_hint = n;  // the first event is sized for all bodies
     for (int64_t s = 0; s < nsteps; ++s) {
@@ -1026,7 +1026,7 @@ int gbh_potential_energy(gbh_ctx *ctx, const gbh_params *p, int64_t n, const dou
     double theta = std::min(theta_of(p), 0.9);  // diagTheta, potential.go:12-14
     // FP64 walk: the reference's sums bit for bit; other walks: the mixed walk's potential
     const bool fp64 = p->walk == GBH_WALK_FP64;
-    CK(gbh::tree_alloc(ctx->tb, n, leaf, 1));
+    CK(gbh::tree_alloc(ctx->tb, ctx->stream, n, leaf, 1));
     ctx->tb.group = 64;
     CK(gbh::tree_build(L, ctx->tb, n, ctx->px, ctx->py, ctx->pz, ctx->mass, kind ? ctx->kind : nullptr,
                        alive ? ctx->alive : nullptr, ctx->ax, ctx->ay, ctx->az, theta, leaf, p->dark_matter_off, fp64,
@@ -1240,7 +1240,7 @@ int gbh_state_diagnostics(gbh_ctx *ctx, const gbh_params *p, double c, gbh_diagn
         // the build zeroes alive holes' accelerations: use the force scratch of the potential path.
         // FP64 walk: the reference's sums bit for bit; other walks: the mixed walk's potential.
         const bool fp64 = p->walk == GBH_WALK_FP64;
-        CK(gbh::tree_alloc(ctx->tb, n, leaf, ctx->nsys));
+        CK(gbh::tree_alloc(ctx->tb, ctx->stream, n, leaf, ctx->nsys));
         CK(grow(ctx->scratch3, ctx->scratch3_cap, 3 * ctx->tb.cap_n));
         sa = ctx->scratch3;
         ctx->tb.group = 64;
@@ -1408,7 +1408,7 @@ int gbh_fwd_save(gbh_ctx *ctx, const gbh_adjoint_params *ap, int64_t n, const do
         t.theta = ap->theta == 0 ? 0.9 : ap->theta;  // bh.go:69-74
         t.leaf = ap->leaf_size > 0 ? ap->leaf_size : 24;
         t.tb = &ctx->tb;
-        CK(gbh::tree_alloc(ctx->tb, n, t.leaf, 1));
+        CK(gbh::tree_alloc(ctx->tb, ctx->stream, n, t.leaf, 1));
         CK(gbh::adj_tree_reserve(t.tbs, ctx->tb));
     }
     const double *src[] = {px, py, pz, vx, vy, vz, mass};
@@ -1440,7 +1440,7 @@ int gbh_bwd(gbh_ctx *ctx, const double *gx, const double *gy, const double *gz, 
     size_t b = sizeof(double) * size_t(n);
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
     if (t.tree) {  // other calls since the forward may have resized the context's tree buffers
-        CK(gbh::tree_alloc(ctx->tb, n, t.leaf, 1));
+        CK(gbh::tree_alloc(ctx->tb, ctx->stream, n, t.leaf, 1));
         CK(gbh::adj_tree_reserve(t.tbs, ctx->tb));
     }
     const double *gin[6] = {gx, gy, gz, gvx, gvy, gvz};

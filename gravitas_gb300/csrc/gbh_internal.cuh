@@ -212,7 +212,9 @@ inline cudaError_t launch_after(const Launch &L, void (*kernel)(Par...), dim3 gr
     } while (0)
 
 // ---- tree.cu (FP64 parts compiled without FMA contraction) ----
-cudaError_t tree_alloc(TreeBufs &b, int64_t n, int leaf_size, int32_t nsys = 1);
+// The first values (launch order, arrival counters) are written on `stream`, that of the builds: one
+// without blocking is not ordered after work on the default stream.
+cudaError_t tree_alloc(TreeBufs &b, cudaStream_t stream, int64_t n, int leaf_size, int32_t nsys = 1);
 void tree_free(TreeBufs &b);
 // Builds the tree of the alive non-hole bodies; zeroes alive holes' accelerations. exact:
 // FP64 moments bit identical to the reference (the FP64 walk); otherwise the FP32 upsweep of

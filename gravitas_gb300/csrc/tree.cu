@@ -1022,7 +1022,7 @@ void tree_free(TreeBufs &b) {
 // cells hold more than leaf stars (only those have children).
 static int64_t node_capacity(int64_t n, int leaf) { return n + 22 * (n / (leaf + 1) + 1) + 1; }
 
-cudaError_t tree_alloc(TreeBufs &b, int64_t n, int leaf, int32_t nsys) {
+cudaError_t tree_alloc(TreeBufs &b, cudaStream_t stream, int64_t n, int leaf, int32_t nsys) {
     int64_t need_nodes = node_capacity(n, leaf);
     if (nsys < 1) nsys = 1;
     if (n <= b.cap_n && need_nodes <= b.cap_nodes && nsys <= b.cap_sys && n / 32 + nsys + 1 <= b.cap_groups) {
@@ -1102,9 +1102,10 @@ cudaError_t tree_alloc(TreeBufs &b, int64_t n, int leaf, int32_t nsys) {
     b.cap_sys = csys;
     b.cap_groups = cgroups;
     b.nsys = nsys;
-    // no launch order yet: gperm[cap_groups] = -1 matches no group count
-    if ((e = cudaMemset(b.gperm, 0xff, sizeof(int32_t) * size_t(cgroups + 1))) != cudaSuccess) return e;
-    if ((e = cudaMemset(b.info, 0, sizeof(DevInfo))) != cudaSuccess) return e;
+    // no launch order yet: gperm[cap_groups] = -1 matches no group count; bbox_done and next_done wrap
+    // to 0 by themselves and must start there
+    if ((e = cudaMemsetAsync(b.gperm, 0xff, sizeof(int32_t) * size_t(cgroups + 1), stream)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(b.info, 0, sizeof(DevInfo), stream)) != cudaSuccess) return e;
     return split_reserve(b, n);
 }
 
