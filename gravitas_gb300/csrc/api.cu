@@ -1225,7 +1225,8 @@ int gbh_state_diagnostics(gbh_ctx *ctx, const gbh_params *p, double c, gbh_diagn
     // potential: the tree at min(theta, 0.9) with the FP64 walk (potential.go:12-42)
     const std::vector<int32_t> &holes = ctx->hole_list;  // alive holes of the state, from its upload
     CK(grow(ctx->holes, ctx->holes_cap, int64_t(holes.size()) + 1));
-    if (!holes.empty()) CK(cudaMemcpy(ctx->holes, holes.data(), holes.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+    if (!holes.empty())  // on the stream of the kernels that read it
+        CK(cudaMemcpyAsync(ctx->holes, holes.data(), holes.size() * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
     int leaf = leaf_of(p);
     double theta = std::min(theta_of(p), 0.9);
     const bool forest = ctx->nsys > 1;
@@ -1306,8 +1307,8 @@ int gbh_forest_upload(gbh_ctx *ctx, int32_t nsys, const int64_t *offsets, const 
     CK(grow(ctx->sys_tiles, ctx->sys_tiles_cap, int64_t(tiles.size()) + 1));
     CK(grow(ctx->sys_off, ctx->sys_off_cap, int64_t(nsys) + 1));
     if (!tiles.empty())
-        CK(cudaMemcpy(ctx->sys_tiles, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(ctx->sys_off, offsets, sizeof(int64_t) * size_t(nsys + 1), cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(ctx->sys_tiles, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->sys_off, offsets, sizeof(int64_t) * size_t(nsys + 1), cudaMemcpyHostToDevice, ctx->stream));
     ctx->h2d += int64_t(sizeof(int4) * tiles.size() + sizeof(int64_t) * size_t(nsys + 1));
     ctx->tiles = gbh::ForestTiles{ctx->sys_tiles, int32_t(tiles.size()), most, ctx->sys_off};
     ctx->nsys = nsys;

@@ -45,3 +45,20 @@ def test_first_block_step_in_fresh_contexts():
         first = first or got
         for a, b in zip(got, first):
             assert np.array_equal(a, b)
+
+
+def test_forest_layouts_one_after_another():
+    """Every upload's layout reaches the build that follows it at once."""
+    sizes = ((900, 1500, 40), (40, 2300, 100), (1200, 1200, 40), (2439, 0, 1))
+    with abi.Context(0) as ctx:
+        for k in range(12):
+            parts = [ics.plummer(n, seed=10 * k + n) for n in sizes[k % 4] if n]
+            s = {f: np.concatenate([p[f] for p in parts]) for f in parts[0]}
+            off = np.concatenate([[0], np.cumsum(sizes[k % 4])]).astype(np.int64)
+            ctx.forest_upload(off, *[s[f] for f in F9[:6]], s["mass"])
+            ctx.call("gbh_state_accelerations", abi.make_params(0.7, 0.02, 16, walk="plain"))
+            g, at = ctx.tree_export(), 0
+            for p in parts:
+                e = O.Tree(p["px"], p["py"], p["pz"], p["mass"], theta=0.7, leaf=16).export()
+                assert np.array_equal(g["keys"][at:at + len(e["keys"])], e["keys"])
+                at += len(e["keys"])
