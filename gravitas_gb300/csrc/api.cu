@@ -2,6 +2,8 @@
 // of the force and step path (bh.Solver.Accelerations, Simulation.Step) over the kernels of
 // tree.cu and walk.cu.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 #include <nvtx3/nvToolsExt.h>
 
 #include <algorithm>
@@ -367,12 +369,50 @@ __global__ __launch_bounds__(kCopyThreads) void k_copy_arrays(int64_t n, Arrays 
 // elements 12 / 19 us in and 10 / 74 out, 16,384 16 / 86 and 16 / 80, 60,000 33 / 105 and 36 / 102,
 // 262,144 108 / 190 and 129 / 177, 1,048,576 391 / 512 and 506 / 472.
 constexpr int64_t kCopyKernelMax = int64_t(1) << 18;
-int copy_arrays(gbh_ctx *ctx, cudaStream_t stream, int64_t n, const Arrays &a, bool to_host) {
+
+// Whether `count` arrays of n doubles that the GPU is to write (null ones are skipped) are in memory, but
+// for kNewPages pages each. A page that nothing has written yet costs its first writer a fault, and
+// the GPU's is the dear one: 17 to 25 us for a 64 KB page against some 50 us an array and 6 us a page by
+// the copies. Calls with new arrays, kernel against copies: downloads (9 arrays) of 33,000 elements
+// 0.9 / 1.0 ms, 60,000 1.5 / 1.1, 200,000 5.7 / 1.7; accelerations (3) of 33,000 0.70 / 0.79, 120,000
+// 1.6 / 1.0. An array with an element that is not 0 has been written; of the others the system tells
+// (1.3 us an array, too much for every call). One array is looked at after the other, since the look
+// itself maps a new array's page.
+constexpr int kNewPages = 5;
+bool in_memory(int64_t n, const double *const *arrays, int count) {
+    static const uintptr_t page = uintptr_t(std::max(4096L, sysconf(_SC_PAGESIZE)));
+    constexpr size_t kMost = 2 + sizeof(double) * size_t(kCopyKernelMax) / 4096;
+    if (n <= 0 || n > kCopyKernelMax || sizeof(double) * size_t(n) <= kNewPages * page) return true;
+    for (int k = 0; k < count; ++k) {
+        if (!arrays[k]) continue;
+        // not the last, which may be a hole at rest; byte by byte: the array may be misaligned
+        const volatile uint8_t *element = reinterpret_cast<const volatile uint8_t *>(arrays[k] + (n - 1 - n / 8));
+        uint8_t any = 0;
+        for (size_t b = 0; b < sizeof(double); ++b) any |= element[b];
+        if (any) continue;
+        unsigned char there[kMost];
+        const uintptr_t begin = reinterpret_cast<uintptr_t>(arrays[k]) / page * page;
+        const size_t bytes = reinterpret_cast<uintptr_t>(arrays[k]) + sizeof(double) * size_t(n) - begin;
+        if (mincore(reinterpret_cast<void *>(begin), bytes, there) != 0) return false;
+        int missing = 0;
+        for (size_t q = 0; q < (bytes + page - 1) / page; ++q) missing += !(there[q] & 1);
+        if (missing > kNewPages) return false;
+    }
+    return true;
+}
+
+// How a call's arrays are copied: by the kernel where it can be, or a copy each; kLook: by the kernel
+// if what it is to write is in memory. An array that is read and then written is looked at before
+// the call reads it (a read maps the pages, but not for writing).
+enum class Way { kKernel, kCopies, kLook };
+int copy_arrays(gbh_ctx *ctx, cudaStream_t stream, int64_t n, const Arrays &a, bool to_host, Way way) {
     (to_host ? ctx->d2h : ctx->h2d) += n * (int64_t(sizeof(double)) * a.nd + a.nb);
     if (n <= 0 || a.nd + a.nb == 0) return GBH_OK;
     uintptr_t bits = 0;
     for (int k = 0; k < a.nd; ++k) bits |= reinterpret_cast<uintptr_t>(a.src[k]) | reinterpret_cast<uintptr_t>(a.dst[k]);
-    if (ctx->host_access && n <= kCopyKernelMax && bits % sizeof(double) == 0) {
+    bool kernel = way != Way::kCopies && ctx->host_access && n <= kCopyKernelMax && bits % sizeof(double) == 0;
+    if (kernel && way == Way::kLook) kernel = in_memory(n, a.dst, a.nd);
+    if (kernel) {
         ctx->touching = true;
         Launch L{stream, &ctx->launches, ctx->num_sms};
         CK(gbh::launch_after(L, k_copy_arrays, unsigned((n + kCopyThreads - 1) / kCopyThreads), kCopyThreads, n, a));
@@ -382,6 +422,11 @@ int copy_arrays(gbh_ctx *ctx, cudaStream_t stream, int64_t n, const Arrays &a, b
     for (int k = 0; k < a.nd; ++k) CK(cudaMemcpyAsync(a.dst[k], a.src[k], sizeof(double) * size_t(n), dir, stream));
     for (int k = 0; k < a.nb; ++k) CK(cudaMemcpyAsync(a.bdst[k], a.bsrc[k], size_t(n), dir, stream));
     return GBH_OK;
+}
+
+// The way for arrays that the call reads and then writes.
+Way look(const gbh_ctx *ctx, int64_t n, const double *const *arrays, int count) {
+    return ctx->host_access && !in_memory(n, arrays, count) ? Way::kCopies : Way::kKernel;
 }
 
 // Whichever way an entry point returns, no kernel touches the caller's arrays afterwards (finish has
@@ -792,7 +837,7 @@ int run_block_steps(gbh_ctx *ctx, const gbh_params *p, double T, double eta, int
 
 int upload_state(gbh_ctx *ctx, int64_t n, const double *px, const double *py, const double *pz, const double *vx,
                  const double *vy, const double *vz, const double *ax, const double *ay, const double *az,
-                 const double *mass, const uint8_t *kind, const uint8_t *alive) {
+                 const double *mass, const uint8_t *kind, const uint8_t *alive, Way way = Way::kKernel) {
     if (n < 0 || n > (int64_t(1) << 30)) return fail(ctx, GBH_ERR_ARG, "n = %lld out of range", (long long)n);
     if (n > 0 && (!px || !py || !pz || !vx || !vy || !vz || !mass))
         return fail(ctx, GBH_ERR_ARG, "state arrays must not be NULL");
@@ -804,7 +849,7 @@ int upload_state(gbh_ctx *ctx, int64_t n, const double *px, const double *py, co
     for (int k = 0; k < 10; ++k) in.add(dst[k], src[k]);
     in.add(ctx->kind, kind);
     in.add(ctx->alive, alive);
-    int rc = copy_arrays(ctx, ctx->stream, n, in, false);
+    int rc = copy_arrays(ctx, ctx->stream, n, in, false, way);
     if (rc) return rc;
     if (!acc && n > 0) {
         const size_t b = sizeof(double) * size_t(n);
@@ -831,12 +876,12 @@ int upload_state(gbh_ctx *ctx, int64_t n, const double *px, const double *py, co
 }
 
 int download_state(gbh_ctx *ctx, double *px, double *py, double *pz, double *vx, double *vy, double *vz, double *ax,
-                   double *ay, double *az) {
+                   double *ay, double *az, Way way = Way::kLook) {
     double *dst[] = {px, py, pz, vx, vy, vz, ax, ay, az};
     const double *src[] = {ctx->px, ctx->py, ctx->pz, ctx->vx, ctx->vy, ctx->vz, ctx->ax, ctx->ay, ctx->az};
     Arrays out;
     for (int k = 0; k < 9; ++k) out.add(dst[k], src[k]);
-    return copy_arrays(ctx, ctx->stream, ctx->n, out, true);
+    return copy_arrays(ctx, ctx->stream, ctx->n, out, true, way);
 }
 
 }  // namespace
@@ -979,14 +1024,15 @@ int gbh_accelerations(gbh_ctx *ctx, const gbh_params *p, int64_t n, const double
     for (int k = 0; k < 7; ++k) in.add(dst[k], src[k]);
     in.add(ctx->kind, kind);
     in.add(ctx->alive, alive);
-    if ((rc = copy_arrays(ctx, ctx->stream, n, in, false))) return rc;
+    const Way way = look(ctx, n, src + 4, 3);
+    if ((rc = copy_arrays(ctx, ctx->stream, n, in, false, way))) return rc;
     rc = forces(ctx, p, n, ctx->px, ctx->py, ctx->pz, ctx->mass, kind ? ctx->kind : nullptr,
                 alive ? ctx->alive : nullptr, ctx->ax, ctx->ay, ctx->az, theta_of(p));
     if (rc) return rc;
     out.add(ax, ctx->ax);
     out.add(ay, ctx->ay);
     out.add(az, ctx->az);
-    if ((rc = copy_arrays(ctx, ctx->stream, n, out, true))) return rc;
+    if ((rc = copy_arrays(ctx, ctx->stream, n, out, true, way))) return rc;
     return finish(ctx, true);
 }
 
@@ -1012,7 +1058,7 @@ int gbh_potential_energy(gbh_ctx *ctx, const gbh_params *p, int64_t n, const dou
     in.add(ctx->mass, mass);
     in.add(ctx->kind, kind);
     in.add(ctx->alive, alive);
-    if ((rc = copy_arrays(ctx, ctx->stream, n, in, false))) return rc;
+    if ((rc = copy_arrays(ctx, ctx->stream, n, in, false, Way::kKernel))) return rc;
     // Holes in state order (collect, build.go:65-69).
     std::vector<int32_t> holes;
     if (kind)
@@ -1073,7 +1119,7 @@ int gbh_direct_accelerations(gbh_ctx *ctx, const gbh_params *p, int64_t n, const
     in.add(ctx->pz, pz);
     in.add(ctx->mass, mass);
     in.add(ctx->kind, kind);
-    if ((rc = copy_arrays(ctx, ctx->stream, n, in, false))) return rc;
+    if ((rc = copy_arrays(ctx, ctx->stream, n, in, false, Way::kKernel))) return rc;
     CK(grow_targets(ctx, ntargets));
     if (targets && (rc = h2d(ctx, ctx->targets, targets, sizeof(int64_t) * size_t(ntargets)))) return rc;
     double *tx = ctx->tout, *ty = tx + ctx->targets_cap, *tz = ty + ctx->targets_cap;
@@ -1084,7 +1130,7 @@ int gbh_direct_accelerations(gbh_ctx *ctx, const gbh_params *p, int64_t n, const
     out.add(ax, tx);
     out.add(ay, ty);
     out.add(az, tz);
-    if ((rc = copy_arrays(ctx, ctx->stream, ntargets, out, true))) return rc;
+    if ((rc = copy_arrays(ctx, ctx->stream, ntargets, out, true, Way::kLook))) return rc;
     return finish(ctx, false);
 }
 
@@ -1098,8 +1144,9 @@ int gbh_step_kdk(gbh_ctx *ctx, const gbh_params *p, double dt, int64_t nsteps, i
     if (nsteps < 0) return fail(ctx, GBH_ERR_ARG, "nsteps < 0");
     if (!ax || !ay || !az) return fail(ctx, GBH_ERR_ARG, "acceleration arrays must not be NULL");
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-    rc = upload_state(ctx, n, px, py, pz, vx, vy, vz, acc_valid ? ax : nullptr, acc_valid ? ay : nullptr,
-                      acc_valid ? az : nullptr, mass, kind, alive);
+    const double *in[] = {px, py, pz, vx, vy, vz, acc_valid ? ax : nullptr, acc_valid ? ay : nullptr, acc_valid ? az : nullptr};
+    const Way way = look(ctx, n, in, 9), back = way == Way::kCopies || acc_valid ? way : Way::kLook;
+    rc = upload_state(ctx, n, px, py, pz, vx, vy, vz, in[6], in[7], in[8], mass, kind, alive, way);
     if (rc) return rc;
     ctx->last_substeps = 1;
     if (n > 0 && (rc = ctx->state_holes ? run_split_steps(ctx, p, dt, nsteps) : run_steps(ctx, p, dt, nsteps)))
@@ -1112,18 +1159,18 @@ int gbh_step_kdk(gbh_ctx *ctx, const gbh_params *p, double dt, int64_t nsteps, i
         pos.add(px, ctx->px);
         pos.add(py, ctx->py);
         pos.add(pz, ctx->pz);
-        if ((rc = copy_arrays(ctx, ctx->copy_stream, n, pos, true))) {
+        if ((rc = copy_arrays(ctx, ctx->copy_stream, n, pos, true, way))) {
             cudaStreamSynchronize(ctx->copy_stream);  // no copy into the caller's arrays after return
             return rc;
         }
         cudaError_t e = cudaEventRecord(ctx->copy_done, ctx->copy_stream);
-        if (e == cudaSuccess) rc = download_state(ctx, nullptr, nullptr, nullptr, vx, vy, vz, ax, ay, az);
+        if (e == cudaSuccess) rc = download_state(ctx, nullptr, nullptr, nullptr, vx, vy, vz, ax, ay, az, back);
         if (e == cudaSuccess && rc == GBH_OK) e = cudaStreamWaitEvent(ctx->stream, ctx->copy_done, 0);
         if (e != cudaSuccess || rc != GBH_OK) {
             cudaStreamSynchronize(ctx->copy_stream);  // no copy into the caller's arrays after return
             return rc != GBH_OK ? rc : fail(ctx, GBH_ERR_CUDA, "position copy: %s", cudaGetErrorString(e));
         }
-    } else if ((rc = download_state(ctx, px, py, pz, vx, vy, vz, ax, ay, az))) {
+    } else if ((rc = download_state(ctx, px, py, pz, vx, vy, vz, ax, ay, az, back))) {
         return rc;
     }
     return finish(ctx, n > 0);
@@ -1416,13 +1463,13 @@ int gbh_fwd_save(gbh_ctx *ctx, const gbh_adjoint_params *ap, int64_t n, const do
     double *dst[] = {t.x, t.x + n, t.x + 2 * n, t.v, t.v + n, t.v + 2 * n, t.m};
     Arrays in, out;
     for (int k = 0; k < 7; ++k) in.add(dst[k], src[k]);
-    if ((rc = copy_arrays(ctx, ctx->stream, n, in, false))) return rc;
+    if ((rc = copy_arrays(ctx, ctx->stream, n, in, false, Way::kKernel))) return rc;
     t.mark = [](void *c) { return stage_event(static_cast<gbh_ctx *>(c)); };
     t.mark_arg = ctx;
     CK(gbh::adj_forward(launch_of(ctx), t));
     double *outs[6] = {out_px, out_py, out_pz, out_vx, out_vy, out_vz};
     for (int k = 0; k < 6; ++k) out.add(outs[k], (k < 3 ? t.x : t.v) + (k % 3) * n);
-    if ((rc = copy_arrays(ctx, ctx->stream, n, out, true))) return rc;
+    if ((rc = copy_arrays(ctx, ctx->stream, n, out, true, Way::kLook))) return rc;
     t.valid = false;
     if ((rc = finish(ctx, false))) return rc;
     t.valid = true;
@@ -1450,12 +1497,12 @@ int gbh_bwd(gbh_ctx *ctx, const double *gx, const double *gy, const double *gz, 
         in.add(t.lam + k * n, gin[k]);
         if (!gin[k]) CK(cudaMemsetAsync(t.lam + k * n, 0, b, ctx->stream));
     }
-    if ((rc = copy_arrays(ctx, ctx->stream, n, in, false))) return rc;
+    if ((rc = copy_arrays(ctx, ctx->stream, n, in, false, Way::kKernel))) return rc;
     CK(cudaMemsetAsync(t.lam + 6 * n, 0, b, ctx->stream));
     CK(gbh::adj_backward(launch_of(ctx), t));
     double *outs[7] = {dx, dy, dz, dvx, dvy, dvz, dm};
     for (int k = 0; k < 7; ++k) out.add(outs[k], t.lam + k * n);
-    if ((rc = copy_arrays(ctx, ctx->stream, n, out, true))) return rc;
+    if ((rc = copy_arrays(ctx, ctx->stream, n, out, true, Way::kLook))) return rc;
     return finish(ctx, false);
 }
 
