@@ -408,13 +408,19 @@ __device__ __forceinline__ void bitonic_sort(uint64_t (&e)[kPer], uint64_t *s_e)
 // the slot in the tile, which settles equal keys by state index; dead bodies, holes and slots beyond
 // the tile have the top bit set, above every star (a star in the root cube's highest corner has a key
 // of all ones). Where neighbours agree in all 53 bits (levels 18 to 21 tell them apart, if
-// anything) each such run is then put in order by the whole key. Against (key, index) pairs
-// of three registers: 16,384 bodies 16.6 -> 11.6 us, the 1.1M-body forest 57 -> 40 (ncu, cold caches).
+// anything) each such run is then put in order by the whole key: short runs by counting, a tile with a
+// longer one (a cluster far tighter than the rest, coincident stars) by the network once more. Against
+// (key, index) pairs of three registers: 16,384 bodies 16.6 -> 11.6 us, the 1.1M-body forest 57 -> 40
+// (ncu, cold caches).
 // 1,024 bodies a tile spread a small state over more SMs than 2,048 would, and a million
 // bodies are 6.7 tiles a SM. pos4 (may be null): each star's position and mass in one record, for
 // the last merge's reads through the order.
 constexpr int kSlotBits = 10;
 constexpr uint64_t kNoStar = uint64_t(1) << 63;
+// Runs of more stars than this take the network. 16,384 stars in clusters of 8: 80.5 us a build either
+// way, of 16 85 by counting and 80.6 by the network, of 128 213 and 146, of 512 387 and 198 (clusters 1e-7
+// of the whole wide; by radix passes, without tiles, 163, 163, 221 and 288).
+constexpr int kRankRun = 8;
 static_assert(kSortTile == 1 << kSlotBits, "a word holds the slot");
 template <bool kForest>
 __global__ __launch_bounds__(kThreads) void k_tile_sort(int64_t n, const int4 *__restrict__ tiles, int32_t ntiles,
@@ -455,18 +461,44 @@ __global__ __launch_bounds__(kThreads) void k_tile_sort(int64_t n, const int4 *_
         e[j] = (star ? k >> kSlotBits << kSlotBits : kNoStar) | uint64_t(slot);
         cnt += __syncthreads_count(star);
     }
-    bitonic_sort(e, s_e);
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) s_e[4 * t + j] = e[j];
-    if (t == 0) s_e[kSortTile] = ~0ull;
-    __syncthreads();
     bool tie = false;
+    for (int pass = 0;; ++pass) {
+        bitonic_sort(e, s_e);
 #pragma unroll
-    for (int j = 0; j < kPer; ++j)
-        tie |= 4 * t + j + 1 < cnt && (s_e[4 * t + j] >> kSlotBits) == (s_e[4 * t + j + 1] >> kSlotBits);
-    if (__syncthreads_or(tie)) {
+        for (int j = 0; j < kPer; ++j) s_e[4 * t + j] = e[j];
+        if (t == 0) s_e[kSortTile] = ~0ull;
+        __syncthreads();
+        if (pass == 1) break;
+        // whether the places p and p + d hold stars of equal words
+        auto equal = [&](int p, int d) { return p + d < cnt && s_e[p] >> kSlotBits == s_e[p + d] >> kSlotBits; };
+        bool many = false;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            tie |= equal(4 * t + j, 1);
+            many |= equal(4 * t + j, kRankRun);
+        }
+        tie = __syncthreads_or(tie);
+        if (!tie || !__syncthreads_or(many)) break;
+        // long runs: the network again, by (the run's first place, the key's lower bits, slot)
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const int p = 4 * t + j;
+            if (p >= cnt) continue;  // behind the stars already
+            int lo = 0, hi = p;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (s_e[mid] >> kSlotBits < e[j] >> kSlotBits) lo = mid + 1;
+                else hi = mid;
+            }
+            const int slot = int(e[j] & (kSortTile - 1));
+            e[j] = uint64_t(lo) << 2 * kSlotBits | (s_key[slot] & (kSortTile - 1)) << kSlotBits | uint64_t(slot);
+        }
+        tie = false;
+        __syncthreads();
+    }
+    if (tie) {
         // rank every element of a run of equal words by its whole key and slot (a run of m takes m
-        // steps a thread; only coincident or nearly coincident stars share 53 bits)
+        // steps a thread, at most kRankRun)
         int rank[kPer];
 #pragma unroll
         for (int j = 0; j < kPer; ++j) {
