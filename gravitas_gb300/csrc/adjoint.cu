@@ -155,9 +155,10 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
-// 1 / sqrt(v) to FP32 rounding. rsqrtf guards against a denormal argument with two multiplications
-// and a test; kNormal leaves them out (v is at least the softening squared, a normal number): the
-// same bits, k_force32 0.758 -> 0.669 ms and k_vjp32 1.31 -> 1.23 ms at 32,768 bodies.
+// 1 / sqrt(v), an approximation within 2^-22.9 of it. kNormal: rsqrt.approx.ftz.f32, which takes a
+// subnormal argument for 0; none occurs (v is at least the softening squared, a normal number), and the
+// outputs are the bits that rsqrtf gives. k_force32 0.758 -> 0.669 ms and k_vjp32 1.31 -> 1.23 ms at
+// 32,768 bodies.
 template <bool kNormal>
 __device__ __forceinline__ float2 rsqrt2(float2 v) {
     if constexpr (kNormal) {

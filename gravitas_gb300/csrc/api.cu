@@ -691,7 +691,7 @@ int run_steps(gbh_ctx *ctx, const gbh_params *p, double dt, int64_t nsteps) {
         ctx->acc_valid = true;
     }
     if (ctx->use_graphs && nsteps > 0) {
-        // One captured step per replay: the ~50 kernels of a step launch as one graph.
+        // One captured step per replay: the 12 to 40 kernels of a step launch as one graph.
         CK(gbh::tree_alloc(ctx->tb, ctx->stream, n, leaf_of(p), ctx->nsys));  // any growth happens outside the capture
         StepGraph &g = ctx->step_graph;
         if (!(g.exec && g.n == n && same_params(g.p, *p) && g.dt == dt && g.tree_gen == ctx->tb.generation &&

@@ -771,6 +771,9 @@ cudaError_t run_sort(const Launch &L, int64_t n, const double *px, const double 
 // Whole build, CUDA events, merges against radix passes: Plummer spheres of 131,072 bodies 0.131 /
 // 0.209 ms, 262,144 0.181 / 0.237, 393,216 0.237 / 0.287, 524,288 0.275 / 0.308, 786,432 0.400 /
 // 0.397, 1,048,576 0.58 / 0.467 (each element searches more and longer runs, the passes stream).
+// Forests take merges at any size; against passes over keys and system ids (as they were sorted before):
+// one system of 1,048,576 among 63 of 100 0.49 / 0.91 ms, two of 1,048,576 0.89 / 1.35, 5,000 of 100
+// 0.28 / 0.90, 20,000 of 50 0.85 / 2.56.
 constexpr int64_t kMergeTiles = 768;
 constexpr int kRsThreads = 256, kRsItems = 8, kRsTile = kRsThreads * kRsItems, kRsWarps = kRsThreads / 32,
               kRsBins = 256, kRsPasses = 8;

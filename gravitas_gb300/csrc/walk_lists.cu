@@ -725,12 +725,13 @@ __device__ __forceinline__ void store_acc(const GroupStars<kS> &G, const Acc (&a
 }
 
 // The part that a split walk's item of rank r walks, for a group whose first star is at sorted place
-// k: the part that holds the star first, then its neighbours on both sides, farther and farther. A
-// part's work falls with its distance from the group (the near one opens leaves, the far ones
-// accept a few nodes), so taking all groups' near parts first is longest first, and the items left
-// for the end are short. Walks against taking each group's parts one after the other: Plummer spheres
-// (theta 0.5) of 16,384 stars 0.122 -> 0.111 ms, 60,000 0.341 -> 0.296; theta 0.9 0.075 -> 0.060 and
-// 0.144 -> 0.126.
+// k: the part that holds the star first, then the next, the one before, the next but one, ... modulo
+// the number of parts (so for a group in the first or last part one of ranks 1 and 2 is the farthest).
+// A part's work falls with its distance from the group (the near one opens leaves, the far ones accept
+// a few nodes), so taking all groups' own parts first, then most near ones, is about longest first, and
+// the items left for the end are short. Walks against taking each group's parts one after the other:
+// Plummer spheres (theta 0.5) of 16,384 stars 0.122 -> 0.111 ms, 60,000 0.341 -> 0.296; theta 0.9 0.075
+// -> 0.060 and 0.144 -> 0.126.
 __device__ __forceinline__ int split_part(int r, int32_t k, int32_t ns, int nparts) {
     const int own = min(int(int64_t(k) * nparts / ns), nparts - 1);
     const int d = (r & 1) ? (r + 1) / 2 : nparts - r / 2;  // 0, +1, -1, +2, ... modulo nparts

@@ -395,8 +395,9 @@ int gbh_probe_fp32_peak(gbh_ctx *ctx, double ms, double *tflops);
  * and the stable sort of the tree build). All pointers except nstars, err and stream
  * are device pointers owned by the caller: px/py/pz hold n doubles, kind/alive n bytes (each
  * may be NULL: all stars, all alive), keys and order room for n entries; *nstars (host)
- * receives the number of sorted bodies. stream is a cudaStream_t (NULL: the legacy default
- * stream); the call returns after the work on it has finished.
+ * receives the number of sorted bodies, and what keys and order hold beyond it is undefined.
+ * stream is a cudaStream_t (NULL: the legacy default stream); the call returns after the work
+ * on it has finished.
  *
  * It allocates nothing: its temporaries live in one static device array of 4.5 MiB that
  * every GPU which loads the library holds until the process exits, enough for at most
