@@ -78,8 +78,8 @@ __device__ __forceinline__ double source_mass(int64_t i, const double *mass, con
 // classify (split.go:39-85): near flags, the near stars' list in index order, and the minimum
 // timescale over near stars and hole pairs (a positive double orders like its bits; their complement
 // is kept, so that the scalars start at 0). Blocks take tiles of 256 bodies in counter order and rank
-// their near stars by look-back. 20,002-body step with the list scanned and written by four more
-// launches 434 us, 420 so.
+// their near stars by look-back. 20,002-body step of 4 substeps with the list scanned and written by
+// four more launches 434 us, 420 so.
 __global__ __launch_bounds__(kEw) void k_classify(int64_t n, const double *__restrict__ px,
                                                   const double *__restrict__ py, const double *__restrict__ pz,
                                                   const double *__restrict__ mass, const uint8_t *__restrict__ kind,
