@@ -364,8 +364,8 @@ __global__ __launch_bounds__(kCopyThreads) void k_copy_arrays(int64_t n, Arrays 
 }
 
 // One kernel copies a call's arrays of up to kCopyKernelMax elements where the GPU reads and writes
-// pageable memory through the host's page tables (Grace over C2C); otherwise, for misaligned arrays
-// and for larger ones, a copy each. Measured with 9 pageable arrays, kernel against copies: 1,013
+// pageable memory through the host's page tables (Grace over C2C); otherwise, for misaligned arrays,
+// for larger ones and where much of what comes back is new (in_memory), a copy each. Measured with 9 pageable arrays, kernel against copies: 1,013
 // elements 12 / 19 us in and 10 / 74 out, 16,384 16 / 86 and 16 / 80, 60,000 33 / 105 and 36 / 102,
 // 262,144 108 / 190 and 129 / 177, 1,048,576 391 / 512 and 506 / 472.
 constexpr int64_t kCopyKernelMax = int64_t(1) << 18;
